@@ -1,233 +1,388 @@
 // The true 32-bit matrix product: C[M, N] (+)= A[M, K] * W[N, K]^T (+ bias[N]), float32 in, float32 out,
 // plain FMA on the CUDA cores. No tensor-core mode of any kind is involved, so nothing is rounded below float32.
 //
-// Every output element is accumulated by one thread with k ascending from 0 to K-1 (one fmaf per k), whatever the
-// tile shape and whatever M is. A row's result therefore does not depend on how many rows run together, which is
-// what lets the 32-bit path give the same logits for a whole prompt, for single tokens and for any batch.
+// The order of every sum depends on K alone. K is cut into at most eight segments (segment_length); a segment is one
+// chain acc = fmaf(a[k], w[k], acc) with k ascending, and the segments' sums are added in ascending order. Both kernels
+// below do exactly this, whatever tile they take and whatever M is. A row's result therefore does not depend on how many
+// rows run together, which is what lets the 32-bit path give the same logits for a whole prompt, for single tokens and
+// for any batch. With few rows the segments are the only parallelism a narrow matrix has; shorter chains also round less.
 // (The reference has no such path on the GPU: its float32 models run under bfloat16 autocast there,
 // sleuth/forge/infer/generate.py:76-77.)
-#include "common.cuh"
+#include "packed_f32.cuh"
 
 namespace slb {
 
-constexpr int kBK = 16;
-
-template <int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc, int accumulate) {
-  pdl_enter();
-  constexpr int THREADS = (BM / TM) * (BN / TN);
-  __shared__ float As[kBK][BM + 1];
-  __shared__ float Ws[kBK][BN + 1];
-  const int tid = threadIdx.x;
-  const int tx = tid % (BN / TN), ty = tid / (BN / TN);
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-
-  float acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
-
-  for (int k0 = 0; k0 < K; k0 += kBK) {
-    for (int e = tid; e < BM * kBK; e += THREADS) {
-      const int m = e / kBK, k = e % kBK;
-      const int gm = m0 + m, gk = k0 + k;
-      As[k][m] = (gm < M && gk < K) ? A[(size_t)gm * lda + gk] : 0.0f;
-    }
-    for (int e = tid; e < BN * kBK; e += THREADS) {
-      const int n = e / kBK, k = e % kBK;
-      const int gn = n0 + n, gk = k0 + k;
-      Ws[k][n] = (gn < N && gk < K) ? W[(size_t)gn * ldw + gk] : 0.0f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kBK; ++kk) {
-      float a[TM], b[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = Ws[kk][tx * TN + j];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int gm = m0 + ty * TM + i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int gn = n0 + tx * TN + j;
-      if (gn >= N) continue;
-      float v = acc[i][j];
-      if (bias) v += bias[gn];
-      float* c = C + (size_t)gm * ldc + gn;
-      *c = accumulate ? *c + v : v;
-    }
-  }
+constexpr int kMaxSegments = 8;
+// k values in a segment: an eighth of K in whole 64s, at least 128.
+__host__ __device__ inline int segment_length(int K) {
+  const int len = ((K + kMaxSegments * 64 - 1) / (kMaxSegments * 64)) * 64;
+  return len < 128 ? 128 : len;
 }
 
-// The same product for up to 16 rows (single-token steps): a block takes 32 output features and all rows, a thread one
-// row and two features, k in slices of 32. What bounds it is not arithmetic but the wait for each slice, so the next
-// slice is fetched into registers (16-byte loads) while the current one is multiplied. Same chain per output as above.
-constexpr int kRowsBK = 32;
+struct GemmF32Args {
+  const float* A;
+  const float* W;
+  const float* bias;
+  float* C;
+  int M, N, K, lda, ldw, ldc, accumulate;
+};
 
-__global__ void __launch_bounds__(256)
-gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                     float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc, int accumulate) {
-  pdl_enter();
-  __shared__ float As[kRowsBK][16 + 1];
-  __shared__ float Ws[kRowsBK][32 + 1];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;       // row ty, features 2 * tx and 2 * tx + 1
-  const int n0 = blockIdx.x * 32;
-  // this thread's share of a slice: four k values of one weight row; threads 0..127 also four of one token row
-  const int wr = tid >> 3, wk = (tid & 7) * 4;
-  float4 pw, pa;
-  auto fetch = [&](int k0) {
-    pw = make_float4(0.f, 0.f, 0.f, 0.f);
-    pa = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int gk = k0 + wk;
-    if (n0 + wr < N && gk < K) pw = *reinterpret_cast<const float4*>(W + (size_t)(n0 + wr) * ldw + gk);      // K is a multiple of 4 here
-    if (tid < 128 && wr < M && gk < K) pa = *reinterpret_cast<const float4*>(A + (size_t)wr * lda + gk);
-  };
-  float acc0 = 0.0f, acc1 = 0.0f;
-  fetch(0);
-  for (int k0 = 0; k0 < K; k0 += kRowsBK) {
-    Ws[wk][wr] = pw.x; Ws[wk + 1][wr] = pw.y; Ws[wk + 2][wr] = pw.z; Ws[wk + 3][wr] = pw.w;
-    if (tid < 128) { As[wk][wr] = pa.x; As[wk + 1][wr] = pa.y; As[wk + 2][wr] = pa.z; As[wk + 3][wr] = pa.w; }
-    __syncthreads();
-    if (k0 + kRowsBK < K) fetch(k0 + kRowsBK);
-    const int kn = min(kRowsBK, K - k0);
-    if (kn == kRowsBK) {
+// ---- few rows -------------------------------------------------------------------------------------------------
+// Up to MP rows (and tiles of MP rows beyond). What bounds it is the weight stream and, from some 8 rows on, what shared memory
+// can deliver (a lane's 16-byte read costs its full 16 bytes of 128 a cycle, broadcast or not). So warp w of a block owns segment
+// w of K, and streams its part of the block's weight rows (NT features), with the token rows' values for the same k, through a
+// ring of its own: CH k values a stage, D stages, 16-byte asynchronous copies, no barrier between warps until a tile's sums are
+// joined. A block goes from tile to tile (tile + gridDim.x) with the ring running on, so its copies never drain. The first
+// stages' weights are asked for before the wait for the kernel in front. LM lanes along the rows and 32 / LM along the features
+// make each lane's block R x CN as square as the tile allows. 0.6B sizes, 8 rows, us before (one chain per output over all of K, slices of
+// 32 k values behind barriers) / now: q/k/v 25.1 / 5.9, o 50.2 / 7.6, gate and up 34.9 / 9.1, down 74.5 / 10.8, head 479 / 145; 64 rows:
+// q/k/v 238 / 22.9, o 456 / 17.8.
+template <int MP, int NT, int CH, int D, bool VEC>
+struct RowsShape {
+  static constexpr int LM = MP >= 64 ? 8 : (MP < 4 ? MP : 4);       // lanes along the rows
+  static constexpr int LN = NT < 32 / LM ? NT : 32 / LM;           // lanes along the features
+  static constexpr int R = MP / LM, CN = NT / LN;
+  static constexpr int kRow = CH + 4;                              // floats: 16-byte reads of 8 rows hit 8 different bank groups
+  static constexpr int kStage = (NT + MP) * kRow;
+  static constexpr int kJoinBuffers = MP * NT >= 512 ? 1 : 2;
+  static constexpr int kSmem = (kMaxSegments * D * kStage + kJoinBuffers * kMaxSegments * MP * NT) * 4;
+  static constexpr int kBlocksPerSm = kSmem <= 113 * 1024 ? 2 : 1;
+};
+
+template <int MP, int NT, int CH, int D, bool VEC>
+__global__ void __launch_bounds__(256, (RowsShape<MP, NT, CH, D, VEC>::kBlocksPerSm))
+gemm_f32_rows_kernel(GemmF32Args a, int seg, int tiles) {
+  using S = RowsShape<MP, NT, CH, D, VEC>;
+  extern __shared__ __align__(16) float smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int lm = lane % S::LM, ln = (lane / S::LM) % S::LN;
+  float* ring = smem + warp * (D * S::kStage);
+  float* join = smem + kMaxSegments * D * S::kStage;
+  const int m0 = blockIdx.y * MP, rows = min(MP, a.M - m0);
+  const int k_begin = warp * seg, k_len = max(0, min(seg, a.K - k_begin));
+  const int chunks = (k_len + CH - 1) / CH, segments = (a.K + seg - 1) / seg;
+
+  // A copy brings kCopy k values of one row; a warp's copy instruction kRowsPer rows (or 1 / kTurns of one). Lane: row lr, k value lk.
+  constexpr int kCopy = VEC ? 4 : 1, kPerRow = CH / kCopy;
+  constexpr int kRowsPer = kPerRow < 32 ? 32 / kPerRow : 1, kTurns = kPerRow < 32 ? 1 : kPerRow / 32;
+  const int lr = kPerRow < 32 ? lane / kPerRow : 0, lk = (lane % kPerRow) * kCopy;
+  const float* a_lane = a.A + (size_t)(m0 + min(lr, rows - 1)) * a.lda + k_begin + lk;
+  auto copy_rows = [&](float* dst, const float* src, size_t ld, int count, int most, int k0) {      // src: this lane's row lr, chunk 0
+    float* d = dst + lr * S::kRow + lk;
 #pragma unroll
-      for (int kk = 0; kk < kRowsBK; ++kk) {
-        const float av = As[kk][ty];
-        acc0 = fmaf(av, Ws[kk][2 * tx], acc0);
-        acc1 = fmaf(av, Ws[kk][2 * tx + 1], acc1);
-      }
-    } else {
-      for (int kk = 0; kk < kn; ++kk) {
-        const float av = As[kk][ty];
-        acc0 = fmaf(av, Ws[kk][2 * tx], acc0);
-        acc1 = fmaf(av, Ws[kk][2 * tx + 1], acc1);
+    for (int turn = 0; turn < kTurns; ++turn) {
+      const int k = k0 + lk + 32 * turn;
+      const int bytes = k < k_len ? 4 * kCopy : 0;
+      const float* p = bytes ? src + k0 + 32 * turn : src - lk;      // (nothing is read there)
+#pragma unroll
+      for (int r = 0; r < most; r += kRowsPer) {
+        if (r + lr < count) copy_async<VEC>(d + r * S::kRow + 32 * turn, p, bytes);
+        p += kRowsPer * ld;
       }
     }
-    __syncthreads();
+  };
+  // the stage after the last one asked for: its tile and its chunk
+  int ask_tile = blockIdx.x, ask_chunk = 0, ask_slot = 0;
+  auto ask_weights = [&]() {
+    const int n0 = ask_tile * NT;
+    copy_rows(ring + ask_slot * S::kStage, a.W + (size_t)(n0 + lr) * a.ldw + k_begin + lk, a.ldw, a.N - n0, NT, ask_chunk * CH);
+  };
+  auto ask_tokens = [&](int chunk, int slot) {
+    copy_rows(ring + slot * S::kStage + NT * S::kRow, a_lane, a.lda, rows, MP, chunk * CH);
+  };
+  auto advance = [&]() {
+    if (++ask_chunk == chunks) { ask_chunk = 0; ask_tile += gridDim.x; }
+    if (++ask_slot == D) ask_slot = 0;
+  };
+
+  pdl_launch_dependents();
+  if (chunks) {
+    for (int s = 0; s < D - 1; ++s) {
+      if (ask_tile < tiles) ask_weights();
+      advance();
+    }
   }
-  if (ty < M) {
+  pdl_wait();
+  if (chunks) {
+    for (int s = 0, c = 0; s < D - 1; ++s) {
+      ask_tokens(c, s);       // (beyond the last tile: copied and not used)
+      if (++c == chunks) c = 0;
+      copies_commit();
+    }
+  }
+
+  constexpr int kOut = (MP * NT + 255) / 256;
+  int slot = 0, buffer = 0;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int n0 = tile * NT;
+    float old[kOut];
+#pragma unroll
+    for (int i = 0; i < kOut; ++i) {
+      const int idx = tid + 256 * i, r = idx / NT, n = n0 + idx % NT;
+      old[i] = (a.accumulate && idx < MP * NT && r < rows && n < a.N) ? a.C[(size_t)(m0 + r) * a.ldc + n] : 0.0f;
+    }
+    float acc[S::R][S::CN];
+#pragma unroll
+    for (int i = 0; i < S::R; ++i)
+#pragma unroll
+      for (int j = 0; j < S::CN; ++j) acc[i][j] = 0.0f;
+    for (int c = 0; c < chunks; ++c) {
+      copies_wait<D - 2>();
+      __syncwarp();
+      const float* ws = ring + slot * S::kStage + ln * S::kRow;
+      const float* as = ring + slot * S::kStage + (NT + lm) * S::kRow;
+      if (++slot == D) slot = 0;
+      if (ask_tile < tiles) {
+        ask_weights();
+        ask_tokens(ask_chunk, ask_slot);
+      }
+      advance();
+      copies_commit();
+      auto quad = [&](int k) {
+        float4 av[S::R];
+#pragma unroll
+        for (int i = 0; i < S::R; ++i) av[i] = *reinterpret_cast<const float4*>(as + i * S::LM * S::kRow + k);
+#pragma unroll
+        for (int j = 0; j < S::CN; ++j) {
+          const float4 wv = *reinterpret_cast<const float4*>(ws + j * S::LN * S::kRow + k);
+#pragma unroll
+          for (int i = 0; i < S::R; ++i) acc[i][j] = fmaf(av[i].x, wv.x, acc[i][j]);
+#pragma unroll
+          for (int i = 0; i < S::R; ++i) acc[i][j] = fmaf(av[i].y, wv.y, acc[i][j]);
+#pragma unroll
+          for (int i = 0; i < S::R; ++i) acc[i][j] = fmaf(av[i].z, wv.z, acc[i][j]);
+#pragma unroll
+          for (int i = 0; i < S::R; ++i) acc[i][j] = fmaf(av[i].w, wv.w, acc[i][j]);
+        }
+      };
+      const int kn = k_len - c * CH;
+      if (kn >= CH) {
+#pragma unroll
+        for (int k = 0; k < CH; k += 4) quad(k);
+      } else {
+        for (int k = 0; k < kn; k += 4) quad(k);
+      }
+    }
+    // the segments' sums, joined in ascending order
+    float* mine = join + (buffer * kMaxSegments + warp) * (MP * NT);
+    if (lane < S::LM * S::LN) {
+#pragma unroll
+      for (int i = 0; i < S::R; ++i)
+#pragma unroll
+        for (int j = 0; j < S::CN; ++j) mine[(lm + i * S::LM) * NT + ln + j * S::LN] = acc[i][j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kOut; ++i) {
+      const int idx = tid + 256 * i, r = idx / NT, n = n0 + idx % NT;
+      if (idx >= MP * NT || r >= rows || n >= a.N) continue;
+      const float* p = join + buffer * kMaxSegments * (MP * NT) + idx;
+      float v = p[0];
+#pragma unroll
+      for (int s = 1; s < kMaxSegments; ++s)
+        if (s < segments) v += p[s * (MP * NT)];
+      if (a.bias) v += a.bias[n];
+      a.C[(size_t)(m0 + r) * a.ldc + n] = a.accumulate ? old[i] + v : v;
+    }
+    if (S::kJoinBuffers == 2) buffer ^= 1;      // two buffers: the next tile's barrier stands between these reads and the next writes
+    else __syncthreads();
+  }
+  copies_wait<0>();
+}
+
+// ---- many rows ------------------------------------------------------------------------------------------------
+// A tile of 16 * RT rows by 128 features per block of 256 threads, RT x 8 outputs per thread, two blocks an SM where there are tiles
+// enough. What bounds it is the FMA pipe and, level with it, what shared memory delivers (a k value is RT + 8 floats read per thread
+// for 8 * RT FMAs). Operands go through registers into shared memory k-major, kTileK k values at a time, two buffers: a warp's
+// reads are then float4 of four rows or features; the FMAs go in packed pairs of neighbouring features. The sums of finished
+// segments wait in shared memory, each thread its own. 3,000 rows x 6,144 x 1,024: 784 us, 48 TFLOP/s, as without packing and
+// segments before; measured and left: tiles of 64 x 128 with 8 x 16 outputs a thread and transposing 4-byte copies (856 us: a
+// quarter less to read from shared memory, but two warps a scheduler do not cover its latency), row-major operands with pairs
+// along k (910 us).
+constexpr int kTileK = 16, kTileN = 128, kTileWRow = kTileN + 4;
+constexpr int tile_smem(int rt) { return (2 * kTileK * (16 * rt + 4 + kTileWRow) + 256 * rt * 8) * 4; }
+
+template <int RT, bool VEC>
+__global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(GemmF32Args a, int seg) {
+  extern __shared__ __align__(16) float smem[];
+  constexpr int BM = 16 * RT, kARow = BM + 4, kBuffer = kTileK * (kARow + kTileWRow);
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * kTileN;
+  // this thread's rows: 4 * ty + 0..3, then 64 + (RT - 4) * ty + 0..RT - 5; its features: 4 * tx + 0..3 and 64 + 4 * tx + 0..3
+  float4* totals = reinterpret_cast<float4*>(smem + 2 * kBuffer) + tid;       // [2 * RT][256]
+  // its share of a slice: k values lk .. lk + 3 of rows and features lr, lr + 64
+  const int lr = tid >> 2, lk = (tid & 3) * 4;
+  const float* ap[2];
+  const float* wp[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    ap[h] = a.A + (size_t)min(m0 + lr + 64 * h, a.M - 1) * a.lda + lk;       // beyond the matrix: its last row, whose results are not stored
+    wp[h] = a.W + (size_t)min(n0 + lr + 64 * h, a.N - 1) * a.ldw + lk;
+  }
+  float4 pa[2], pw[2];
+  auto four = [&](const float* src, int k0) {
+    if (VEC) return k0 + lk < a.K ? *reinterpret_cast<const float4*>(src + k0) : make_float4(0.f, 0.f, 0.f, 0.f);      // K is a multiple of 4
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (k0 + lk < a.K) v.x = src[k0];
+    if (k0 + lk + 1 < a.K) v.y = src[k0 + 1];
+    if (k0 + lk + 2 < a.K) v.z = src[k0 + 2];
+    if (k0 + lk + 3 < a.K) v.w = src[k0 + 3];
+    return v;
+  };
+  constexpr bool kTwo = RT > 4;
+  const bool second = RT == 8 || lr < BM - 64;
+  auto fetch_weights = [&](int k0) { pw[0] = four(wp[0], k0); pw[1] = four(wp[1], k0); };
+  auto fetch_tokens = [&](int k0) { pa[0] = four(ap[0], k0); if (kTwo && second) pa[1] = four(ap[1], k0); };
+  auto put = [&](int buffer) {
+    float* as = smem + buffer * kBuffer + lk * kARow + lr;
+    float* ws = smem + buffer * kBuffer + kTileK * kARow + lk * kTileWRow + lr;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h == 0 || (kTwo && second)) {
+        as[64 * h] = pa[h].x; as[kARow + 64 * h] = pa[h].y; as[2 * kARow + 64 * h] = pa[h].z; as[3 * kARow + 64 * h] = pa[h].w;
+      }
+      ws[64 * h] = pw[h].x; ws[kTileWRow + 64 * h] = pw[h].y; ws[2 * kTileWRow + 64 * h] = pw[h].z; ws[3 * kTileWRow + 64 * h] = pw[h].w;
+    }
+  };
+  pdl_launch_dependents();
+  fetch_weights(0);
+  pdl_wait();
+  fetch_tokens(0);
+
+  f32x2 acc[RT][4];
+#pragma unroll
+  for (int i = 0; i < RT; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+#pragma unroll
+  for (int e = 0; e < 2 * RT; ++e) totals[e * 256] = make_float4(0.f, 0.f, 0.f, 0.f);
+  put(0);
+  __syncthreads();
+
+  int buffer = 0, left = seg;
+  for (int k0 = 0; k0 < a.K; k0 += kTileK) {
+    const bool more = k0 + kTileK < a.K;
+    if (more) { fetch_weights(k0 + kTileK); fetch_tokens(k0 + kTileK); }
+    const float* as = smem + buffer * kBuffer + 4 * ty;
+    const float* as2 = smem + buffer * kBuffer + 64 + (RT - 4) * ty;
+    const float* ws = smem + buffer * kBuffer + kTileK * kARow + 4 * tx;
+    auto one = [&](int k) {
+      float av[RT];
+      *reinterpret_cast<float4*>(av) = *reinterpret_cast<const float4*>(as + k * kARow);
+      if (RT == 8) *reinterpret_cast<float4*>(av + 4) = *reinterpret_cast<const float4*>(as2 + k * kARow);
+      if (RT == 6) *reinterpret_cast<float2*>(av + 4) = *reinterpret_cast<const float2*>(as2 + k * kARow);
+      ulonglong2 wv[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) wv[j] = *reinterpret_cast<const ulonglong2*>(ws + k * kTileWRow + 64 * j);
+#pragma unroll
+      for (int i = 0; i < RT; ++i) {
+        const f32x2 v = both(av[i]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          acc[i][2 * j] = fma2(v, wv[j].x, acc[i][2 * j]);
+          acc[i][2 * j + 1] = fma2(v, wv[j].y, acc[i][2 * j + 1]);
+        }
+      }
+    };
+    const int kn = a.K - k0;
+    if (kn >= kTileK) {
+#pragma unroll
+      for (int k = 0; k < kTileK; ++k) one(k);
+    } else {
+      for (int k = 0; k < kn; ++k) one(k);
+    }
+    left -= kTileK;
+    if (left == 0 || !more) {      // a segment is done (segments are whole multiples of 64)
+      left = seg;
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float4 t = totals[(2 * i + j) * 256];
+          t.x += low_half(acc[i][2 * j]);
+          t.y += high_half(acc[i][2 * j]);
+          t.z += low_half(acc[i][2 * j + 1]);
+          t.w += high_half(acc[i][2 * j + 1]);
+          totals[(2 * i + j) * 256] = t;
+          acc[i][2 * j] = acc[i][2 * j + 1] = 0;
+        }
+    }
+    if (more) {
+      buffer ^= 1;
+      put(buffer);
+      __syncthreads();
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < RT; ++i) {
+    const int gm = m0 + (i < 4 ? 4 * ty + i : 64 + (RT - 4) * ty + i - 4);
+    if (gm >= a.M) continue;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const int gn = n0 + 2 * tx + j;
-      if (gn >= N) continue;
-      float v = j ? acc1 : acc0;
-      if (bias) v += bias[gn];
-      float* c = C + (size_t)ty * ldc + gn;
-      *c = accumulate ? *c + v : v;
+      const float4 t = totals[(2 * i + j) * 256];
+      const float tv[4] = {t.x, t.y, t.z, t.w};
+      float* c = a.C + (size_t)gm * a.ldc + n0 + 4 * tx + 64 * j;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int gn = n0 + 4 * tx + 64 * j + e;
+        if (gn >= a.N) continue;
+        float v = tv[e];
+        if (a.bias) v += a.bias[gn];
+        c[e] = a.accumulate ? c[e] + v : v;
+      }
     }
   }
 }
 
-// The same product for many rows: a 128 x 128 tile per block, 8 x 8 outputs per thread (two 4-wide groups of rows
-// by two of columns, so that a warp's shared-memory reads are one or two broadcasts and one contiguous run), operands
-// brought in 16 k values at a time with 16-byte global loads where the matrices allow it (the next slice is already in
-// registers while the current one is multiplied), read back from shared memory as float4. Every output is still one
-// thread's own chain acc = fmaf(a[k], w[k], acc) for k = 0, 1, ..., K - 1: bit for bit what the kernel above computes.
-constexpr int kBigTile = 128;
-constexpr int kBigPad = 4;       // floats between the k-rows of a tile in shared memory: keeps float4 alignment, spreads banks
+template <int MP, int NT, int CH, int D, bool VEC>
+static int launch_rows(const GemmF32Args& a, cudaStream_t s) {
+  using S = RowsShape<MP, NT, CH, D, VEC>;
+  static_assert(S::kSmem <= 227 * 1024, "the ring must fit shared memory");
+  const auto kernel = gemm_f32_rows_kernel<MP, NT, CH, D, VEC>;
+  static const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem);
+  if (e != cudaSuccess) return fail(2, "gemm_f32: cannot reserve %d bytes of shared memory: %s", S::kSmem, cudaGetErrorString(e));
+  const int tiles = (a.N + NT - 1) / NT, row_tiles = (a.M + MP - 1) / MP;
+  SLB_REQUIRE(row_tiles < 65536, "gemm_f32: M=%d needs more than 65535 row tiles", a.M);
+  const int room = S::kBlocksPerSm * sm_count() / row_tiles > 1 ? S::kBlocksPerSm * sm_count() / row_tiles : 1;
+  launch_prefetching(kernel, dim3(tiles < room ? tiles : room, row_tiles), dim3(256), S::kSmem, s, a, segment_length(a.K), tiles);
+  return check_launch("gemm_f32 (few rows)");
+}
 
-__global__ void __launch_bounds__(256)
-gemm_f32_big_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                    float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc, int accumulate, int vector_loads) {
-  pdl_enter();
-  __shared__ __align__(16) float As[kBK][kBigTile + kBigPad];
-  __shared__ __align__(16) float Ws[kBK][kBigTile + kBigPad];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * kBigTile, n0 = blockIdx.x * kBigTile;
-  // this thread's share of a slice: rows lr and lr + 64 of each operand, k values lk .. lk + 3
-  const int lr = tid >> 2, lk = (tid & 3) * 4;
+// Which kernel and tile a product takes, from what a round over the SMs costs (nanoseconds per k value, B200, products of 1,024 to
+// 6,144 features): a round of tiles with one block an SM, a round with two, and a round of the streaming kernel's 64 x 32 tiles.
+// The sums of rounds meet the measured times within 5 % (us at 1,500 rows x 6,144 x 1,024: 8 / 6 / 4 rows a thread
+// 399 / 479 / 494; 1,500 x 1,024 x 2,048: 219 / 176 / 251; 300 x 1,024 x 2,048: 218 / 176 / 137, streaming 81).
+constexpr int kRoundAlone[3] = {107, 86, 67}, kRoundTwo[3] = {191, 155, 120}, kRoundRows = 21;      // 8, 6, 4 rows a thread
 
-  float acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+static int round_of(int rt) { return rt == 8 ? 0 : (rt == 6 ? 1 : 2); }
+static long long tiles_of(const GemmF32Args& a, int rt) {
+  return (long long)((a.N + kTileN - 1) / kTileN) * ((a.M + 16 * rt - 1) / (16 * rt));
+}
+static long long tile_cost(const GemmF32Args& a, int rt) {
+  const long long sms = sm_count(), tiles = tiles_of(a, rt), rest = tiles % (2 * sms);
+  return tiles / (2 * sms) * kRoundTwo[round_of(rt)] + (rest == 0 ? 0 : (rest <= sms ? kRoundAlone : kRoundTwo)[round_of(rt)]);
+}
 
-  float4 pa[2], pw[2];
-  auto fetch = [&](int k0) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int gm = m0 + lr + 64 * h, gn = n0 + lr + 64 * h, gk = k0 + lk;
-      float4 va = make_float4(0.f, 0.f, 0.f, 0.f), vw = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (gm < M) {
-        const float* src = A + (size_t)gm * lda + gk;
-        if (vector_loads && gk + 3 < K) va = *reinterpret_cast<const float4*>(src);
-        else {
-          if (gk < K) va.x = src[0];
-          if (gk + 1 < K) va.y = src[1];
-          if (gk + 2 < K) va.z = src[2];
-          if (gk + 3 < K) va.w = src[3];
-        }
-      }
-      if (gn < N) {
-        const float* src = W + (size_t)gn * ldw + gk;
-        if (vector_loads && gk + 3 < K) vw = *reinterpret_cast<const float4*>(src);
-        else {
-          if (gk < K) vw.x = src[0];
-          if (gk + 1 < K) vw.y = src[1];
-          if (gk + 2 < K) vw.z = src[2];
-          if (gk + 3 < K) vw.w = src[3];
-        }
-      }
-      pa[h] = va;
-      pw[h] = vw;
-    }
-  };
-  fetch(0);
-  for (int k0 = 0; k0 < K; k0 += kBK) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = lr + 64 * h;
-      As[lk][r] = pa[h].x; As[lk + 1][r] = pa[h].y; As[lk + 2][r] = pa[h].z; As[lk + 3][r] = pa[h].w;
-      Ws[lk][r] = pw[h].x; Ws[lk + 1][r] = pw[h].y; Ws[lk + 2][r] = pw[h].z; Ws[lk + 3][r] = pw[h].w;
-    }
-    __syncthreads();
-    if (k0 + kBK < K) fetch(k0 + kBK);
-#pragma unroll
-    for (int kk = 0; kk < kBK; ++kk) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[kk][64 + ty * 4]);
-      const float4 b0 = *reinterpret_cast<const float4*>(&Ws[kk][tx * 4]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&Ws[kk][64 + tx * 4]);
-      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
+// Rounds of the streaming kernel with its largest tile (one block an SM; a block keeps to its 64 rows), times their cost.
+static long long rows_cost(const GemmF32Args& a) {
+  const long long sms = sm_count(), down = (a.M + 63) / 64, across = (a.N + 31) / 32;
+  const long long blocks = down < sms ? (sms / down < across ? sms / down : across) : 1;
+  return (across + blocks - 1) / blocks * ((blocks * down + sms - 1) / sms) * kRoundRows;
+}
 
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int gm = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int gn = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
-      if (gn >= N) continue;
-      float v = acc[i][j];
-      if (bias) v += bias[gn];
-      float* c = C + (size_t)gm * ldc + gn;
-      *c = accumulate ? *c + v : v;
-    }
-  }
+template <int RT, bool VEC>
+static int launch_tile(const GemmF32Args& a, cudaStream_t s) {
+  const auto kernel = gemm_f32_tile_kernel<RT, VEC>;
+  // One block an SM is asked for (by its shared memory) where every tile gets an SM of its own: left to itself a kernel that
+  // starts while the one before still runs finds half-empty SMs and doubles up there (1,500 x 1,024 x 2,048: 276 instead of 176 us).
+  constexpr int kAlone = 116 * 1024;
+  static const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAlone);
+  if (e != cudaSuccess) return fail(2, "gemm_f32: cannot reserve %d bytes of shared memory: %s", kAlone, cudaGetErrorString(e));
+  const dim3 grid((a.N + kTileN - 1) / kTileN, (a.M + 16 * RT - 1) / (16 * RT));
+  SLB_REQUIRE(grid.y < 65536, "gemm_f32: M=%d needs more than 65535 row tiles", a.M);
+  const int smem = tiles_of(a, RT) <= sm_count() ? kAlone : tile_smem(RT);
+  launch_prefetching(kernel, grid, dim3(256), smem, s, a, segment_length(a.K));
+  return check_launch("gemm_f32 (tiles)");
 }
 
 }  // namespace slb
@@ -241,22 +396,29 @@ extern "C" int slb_gemm_f32(const float* A, const float* W, const float* bias, f
               ldw, ldc, K, N);
   if (M == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
-  const bool aligned = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
-  if (M <= 16 && aligned) {
-    launch(gemm_f32_rows_kernel, dim3((N + 31) / 32), dim3(256), 0, s, A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate);
-  } else if (M <= 16) {
-    constexpr int BM = 16, BN = 32;
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    launch(gemm_f32_kernel<BM, BN, 1, 2>, dim3(grid), dim3(256), 0, s, A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate);
-  } else if (M < 96) {
-    constexpr int BM = 64, BN = 64;
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    launch(gemm_f32_kernel<BM, BN, 4, 4>, dim3(grid), dim3(256), 0, s, A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate);
-  } else {
-    dim3 grid((N + kBigTile - 1) / kBigTile, (M + kBigTile - 1) / kBigTile);
-    SLB_REQUIRE(grid.y < 65536, "gemm_f32: M=%d needs more than 65535 row tiles", M);
-    const int vector_loads = (lda % 4 == 0) && (ldw % 4 == 0) && ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
-    launch(gemm_f32_big_kernel, dim3(grid), dim3(256), 0, s, A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, vector_loads);
+  const GemmF32Args a{A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate};
+  const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
+  int rt = 8;
+  if (tile_cost(a, 6) < tile_cost(a, rt)) rt = 6;
+  if (tile_cost(a, 4) < tile_cost(a, rt)) rt = 4;
+  const bool few = M <= 64 || rows_cost(a) < tile_cost(a, rt);
+  if (!vec) {      // no 16-byte reads: copies of four bytes
+    if (M <= 16) return launch_rows<16, 8, 32, 2, false>(a, s);
+    if (few) return launch_rows<64, 8, 32, 2, false>(a, s);
+  } else if (few) {
+    // 32 features a tile where that still gives every SM one, else 16 or 8
+    const int nt = N >= 4096 ? 32 : (N >= 2048 ? 16 : 8);
+    if (M <= 1) return nt >= 16 ? launch_rows<1, 16, 64, 4, true>(a, s) : launch_rows<1, 8, 64, 4, true>(a, s);
+    if (M <= 2) return nt >= 16 ? launch_rows<2, 16, 64, 3, true>(a, s) : launch_rows<2, 8, 64, 4, true>(a, s);
+    if (M <= 4) return nt == 32 ? launch_rows<4, 32, 32, 4, true>(a, s) : nt == 16 ? launch_rows<4, 16, 64, 2, true>(a, s) : launch_rows<4, 8, 64, 3, true>(a, s);
+    if (M <= 8) return nt == 32 ? launch_rows<8, 32, 32, 4, true>(a, s) : nt == 16 ? launch_rows<8, 16, 64, 2, true>(a, s) : launch_rows<8, 8, 64, 3, true>(a, s);
+    if (M <= 16) return nt == 32 ? launch_rows<16, 32, 32, 3, true>(a, s) : nt == 16 ? launch_rows<16, 16, 32, 2, true>(a, s) : launch_rows<16, 8, 32, 3, true>(a, s);
+    if (M <= 32) return nt == 32 ? launch_rows<32, 32, 32, 2, true>(a, s) : nt == 16 ? launch_rows<32, 16, 32, 3, true>(a, s) : launch_rows<32, 8, 32, 2, true>(a, s);
+    if (M <= 64 && nt == 8) return launch_rows<64, 8, 32, 2, true>(a, s);
+    return launch_rows<64, 32, 16, 2, true>(a, s);
   }
-  return check_launch("gemm_f32");
+  if (!vec) return launch_tile<8, false>(a, s);
+  if (rt == 8) return launch_tile<8, true>(a, s);
+  if (rt == 6) return launch_tile<6, true>(a, s);
+  return launch_tile<4, true>(a, s);
 }
