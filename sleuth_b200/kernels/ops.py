@@ -313,6 +313,34 @@ def attention(q, k_pool, v_pool, out, tok_seq, tok_pos, block_table, heads: int,
                _p(sinks), vd, DT[q.dtype], stream if stream is not None else current_stream())
 
 
+def attention_f32_supported(heads: int, kv_heads: int, head_dim: int, value_dim: int, dtype: torch.dtype) -> bool:
+    """Whether the float32 attention kernels take these heads (all steps of a layer go the same way)."""
+    return dtype == torch.float32 and head_dim in (64, 128) and value_dim == head_dim and heads // kv_heads <= 16
+
+
+def attention_f32_scratch_floats(n_seqs: int, heads: int, head_dim: int, table_stride: int) -> int:
+    """Scratch of a step of single tokens: a chunk (two pages) leaves its weighted values, maximum and sum there."""
+    return n_seqs * heads * ((table_stride + 1) // 2) * (head_dim + 2)
+
+
+def attention_f32(q, k_pool, v_pool, out, seq_start, past, counts, block_table, max_count: int, heads: int, kv_heads: int,
+                  head_dim: int, window: int, scale: float, scratch, stream=None, sinks=None) -> None:
+    """Causal attention in true float32. Results do not depend on how a sequence was cut into steps. ``scratch`` (for
+    ``max_count`` 1): ``attention_f32_scratch_floats`` floats."""
+    _cuda(q, k_pool, v_pool, out, seq_start, past, counts, block_table, sinks, scratch)
+    T, n = q.shape[0], block_table.shape[0]
+    _need(q.shape == (T, heads, head_dim) and out.shape == (T, heads * head_dim), "attention_f32: shapes disagree")
+    _need(q.dtype == out.dtype == k_pool.dtype == v_pool.dtype == torch.float32, "attention_f32: float32 only")
+    _need(tuple(k_pool.shape[1:]) == tuple(v_pool.shape[1:]) == (kv_heads, 64, head_dim) and k_pool.shape[0] == v_pool.shape[0],
+          "attention_f32: pool shape")
+    _need(block_table.dtype == torch.int32 and block_table.dim() == 2, "attention_f32: block table")
+    _need(sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == heads), "attention_f32: sinks are float32, one per head")
+    _need(seq_start.numel() >= n and past.numel() >= n and counts.numel() >= n, "attention_f32: per-sequence tables")
+    lib().call("slb_attention_f32", _p(q), _p(k_pool), _p(v_pool), _p(out), _p(seq_start), _p(past), _p(counts), _p(block_table),
+               block_table.shape[1], n, int(max_count), heads, kv_heads, head_dim, int(window), float(scale), _p(sinks),
+               _p(scratch), scratch.numel() if scratch is not None else 0, stream if stream is not None else current_stream())
+
+
 def flash_supported(head_dim: int, dtype: torch.dtype) -> bool:
     """Whether the tensor-core attention kernels take this head size and dtype."""
     return dtype == torch.bfloat16 and head_dim in (64, 128)

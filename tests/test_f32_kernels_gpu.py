@@ -1,0 +1,112 @@
+"""The true 32-bit kernels (csrc/gemm_f32.cu, csrc/attention_f32.cu) at the edges of their tiles, against float64, and their
+promise that a row's bits depend neither on the rows beside it nor on how a sequence was cut into steps."""
+
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from test_kernels_gpu import DEV, make_cache, ops, plain_attention
+
+pytestmark = pytest.mark.gpu
+
+
+# Few rows: every row tile (1, 2, 4, 8, 16, 32, 64 rows), both feature tiles (8; 16 from 8,192 features on), segments of 128 and more,
+# a last segment that is short or missing, inner dimensions that no 16-byte copy takes. Many rows: tiles of 128, 96 and 64 rows.
+@pytest.mark.parametrize("M,N,K", [(1, 8, 4), (1, 9, 132), (2, 8200, 96), (3, 17, 1028), (7, 8192, 260), (8, 1000, 1024), (9, 8195, 644),
+                                   (16, 40, 3072), (20, 8200, 132), (33, 100, 1100), (64, 8197, 200), (65, 8, 2052), (100, 24, 77),
+                                   (129, 1024, 1024), (700, 1000, 388), (1500, 1030, 64), (1500, 2304, 100), (1100, 6150, 36)])
+def test_gemm_f32_error_and_rows(M, N, K):
+    g = torch.Generator().manual_seed(M * 7 + N)
+    a, w, bias = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV), torch.randn(N, generator=g).to(DEV)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    ops().gemm_f32(a, w, out, bias)
+    ref = a.double() @ w.double().T + bias.double()
+    # chains of half a segment, then the halves, at most eight segments and the bias: each step rounds by 2^-24 at most
+    seg = max(128, -(-K // 512) * 64)
+    steps = min(K, seg) / 2 + 10
+    bound = 2.0 ** -24 * steps * 1.01 * (a.double().abs() @ w.double().abs().T + bias.double().abs())
+    assert ((out.double() - ref).abs() <= bound).all()
+    for rows in (1, 2, 5, 12, 30, 60):
+        if rows < M:
+            some = torch.empty(rows, N, device=DEV)
+            ops().gemm_f32(a[M - rows:].contiguous(), w, some, bias)
+            assert torch.equal(some, out[M - rows:])
+    acc = torch.full((M, N), 2.0, device=DEV)
+    ops().gemm_f32(a, w, acc, accumulate=True)
+    plain = torch.empty(M, N, device=DEV)
+    ops().gemm_f32(a, w, plain)
+    assert torch.equal(acc, plain + 2.0)
+
+
+def run_f32(q, k_pool, v_pool, table, pasts, counts, heads, kv_heads, hd, window, sinks=None):
+    o = ops()
+    d = lambda a: torch.as_tensor(np.asarray(a, dtype=np.int32)).to(DEV)
+    out = torch.full((q.shape[0], heads * hd), float("nan"), device=DEV)
+    starts = np.concatenate([[0], np.cumsum(counts)])
+    floats = o.attention_f32_scratch_floats(len(counts), heads, hd, table.shape[1])
+    scratch = torch.full((floats,), float("nan"), device=DEV) if max(counts) == 1 else None
+    o.attention_f32(q, k_pool, v_pool, out, d(starts), d(pasts), d(counts), table, max(counts), heads, kv_heads, hd, window,
+                    1.0 / math.sqrt(hd), scratch, sinks=sinks)
+    return out
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd", [(4, 2, 128), (5, 1, 64), (8, 8, 64), (16, 1, 128), (3, 3, 128), (12, 2, 64)])
+@pytest.mark.parametrize("window,sink", [(0, False), (0, True), (50, False), (200, True), (-96, False)])
+def test_attention_f32(heads, kv_heads, hd, window, sink):
+    pasts, counts = [0, 70, 0, 129, 300], [1, 1, 200, 64, 130]
+    gen = torch.Generator().manual_seed(heads + hd + window)
+    lens = [p + c for p, c in zip(pasts, counts)]
+    k_pool, v_pool, table, ks, vs = make_cache(lens, kv_heads, hd, torch.float32, gen)
+    k_pool, v_pool, table = k_pool.to(DEV), v_pool.to(DEV), table.to(DEV)
+    q = torch.randn(sum(counts), heads, hd, generator=gen)
+    sinks = torch.randn(heads, generator=gen) if sink else None
+    dev_sinks = sinks.to(DEV) if sink else None
+    got = run_f32(q.to(DEV), k_pool, v_pool, table, pasts, counts, heads, kv_heads, hd, window, dev_sinks)
+    at = 0
+    for i, (p, c) in enumerate(zip(pasts, counts)):
+        for t in range(c):
+            pos = p + t
+            lo = max(0, pos - window + 1) if window > 0 else (pos // -window * -window if window < 0 else 0)
+            if t % 37 and t not in (0, c - 1):
+                continue
+            kk = ks[i][lo:pos + 1].double().repeat_interleave(heads // kv_heads, 1)
+            vv = vs[i][lo:pos + 1].double().repeat_interleave(heads // kv_heads, 1)
+            s = torch.einsum("hd,jhd->hj", q[at + t].double(), kk) / math.sqrt(hd)
+            if sink:
+                s = torch.cat([s, sinks.double()[:, None]], 1)
+            ref = torch.einsum("hj,jhd->hd", torch.softmax(s, 1)[:, :kk.shape[0]], vv)
+            # scores to about 1e-6 (chains of 64 at most, values of a few units), weights and sums to a few 1e-6
+            torch.testing.assert_close(got[at + t].cpu().double().view(heads, hd), ref, rtol=1e-5, atol=5e-6)
+        at += c
+    # one sequence at a time, in portions, and its last tokens one by one (all sequences in one step): the same bits
+    at = 0
+    for i, (p, c) in enumerate(zip(pasts, counts)):
+        cuts = [0] + [x for x in (1, 40, 104) if x < c] + [c]
+        for x, y in zip(cuts[:-1], cuts[1:]):
+            part = run_f32(q[at + x:at + y].to(DEV), k_pool, v_pool, table[i:i + 1], [p + x], [y - x], heads, kv_heads, hd, window, dev_sinks)
+            assert torch.equal(part, got[at + x:at + y])
+        at += c
+    starts = np.concatenate([[0], np.cumsum(counts)])
+    for back in (1, 2):
+        which = [max(starts[i + 1] - back, starts[i]) for i in range(len(counts))]
+        alone = run_f32(q[which].contiguous().to(DEV), k_pool, v_pool, table, [p + int(w - s) for p, w, s in zip(pasts, which, starts)],
+                        [1] * len(counts), heads, kv_heads, hd, window, dev_sinks)
+        assert torch.equal(alone, got[which])
+
+
+def test_attention_f32_leaves_later_tokens_out():
+    """Infinite values of tokens that a query does not see do not reach it; a NaN key that it sees does."""
+    heads, kv_heads, hd, n = 4, 2, 128, 150
+    gen = torch.Generator().manual_seed(3)
+    k_pool, v_pool, table, ks, vs = make_cache([n], kv_heads, hd, torch.float32, gen)
+    q = torch.randn(n, heads, hd, generator=gen).to(DEV)
+    clean = run_f32(q, k_pool.to(DEV), v_pool.to(DEV), table.to(DEV), [0], [n], heads, kv_heads, hd, 0)
+    v_pool[int(table[0, 1]), :, 36] = float("inf")          # position 100
+    k_pool[int(table[0, 1]), :, 46, 0] = float("nan")       # position 110
+    got = run_f32(q, k_pool.to(DEV), v_pool.to(DEV), table.to(DEV), [0], [n], heads, kv_heads, hd, 0)
+    assert torch.equal(got[:100], clean[:100])
+    assert not torch.isfinite(got[100:]).any() and torch.isnan(got[110:]).all()
+    one = run_f32(q[120:121], k_pool.to(DEV), v_pool.to(DEV), table.to(DEV), [120], [1], heads, kv_heads, hd, 0)
+    assert torch.isnan(one).all()
