@@ -15,9 +15,11 @@
 // are built with atomics. Tokens tied with the top-p threshold value are kept together (the reference keeps those
 // that its unstable sort happens to place first).
 //
-// Cost at a 152k vocabulary: a pass over the row with exp and division is compute-bound on one SM (~50 us), hence
-// the eight blocks; top-k works on the stored values (order is all it needs) and usually leaves few enough tokens
-// to finish on a short list in one block.
+// Cost: a row's eighth is read once into shared memory, and one histogram over values between a lower bound and the row's
+// maximum finds the short list that holds the answer (see quick_list below). 64 rows of 151,936, top-k 50, top-p 0.9: 247 us
+// before (six passes over the row, four of them with 64 KB of histograms to clear and add up), 55 us now. Rows for which
+// that cannot work (longer than the blocks hold, NaN or infinite maxima, more candidates than fit) take the general path:
+// a radix descent over the sort keys, eight bits a pass.
 #include <math.h>
 
 #include <cooperative_groups.h>
@@ -31,7 +33,7 @@ namespace cg = cooperative_groups;
 
 namespace slb {
 
-constexpr int kSampleThreads = 1024;
+constexpr int kSampleThreads = 512;
 constexpr double kMassScale = 1099511627776.0;  // 2^40
 
 __device__ __forceinline__ unsigned int sort_key(float v) {
@@ -150,6 +152,10 @@ struct SampleExchange {
   float max[2];
   int count[2];
   unsigned long long seg[kSampleWarps];
+  float low;                               // quick path: the block's share of the lower bound, and whether it must not be taken
+  int bad;
+  int total;                               // quick path: candidates
+  unsigned int key;                        // quick path: what block 0 found
 };
 
 struct SampleShared {
@@ -386,14 +392,157 @@ __device__ int warp_walk(int n, G get, float mx, unsigned int floor_key, float m
   return -1;
 }
 
-__global__ void __cluster_dims__(kSampleTeam, 1, 1) __launch_bounds__(kSampleThreads)
+// ---- the quick path ----
+// Block `rank` of a row keeps its eighth of it in shared memory, warp by warp in token order: thread i's float4 c holds the tokens
+// base + 128 * c + 4 * lane .. + 3 of its warp's stretch. One histogram of kBins equal steps of value, from a lower bound to the
+// maximum, is added up over the team; the step in which the weight from above reaches the target is known then, and the few
+// tokens at or above it (for top-k), or in it (for top-p without top-k), are all that the exact decision needs.
+constexpr int kHeld = 10;              // float4 per thread
+constexpr int kHeldTokens = kHeld * 4 * kSampleThreads;
+constexpr int kBins = 1024;
+constexpr int kQuickList = 1024;       // candidates of a row at most
+constexpr int kSmallList = 512;        // up to this many entries are compared each with each
+
+struct Held {
+  float4* mine;            // this thread's first float4; the next ones kSampleThreads apart
+  int begin, end;          // its warp's stretch of tokens (row numbers), whole chunks of 128 but for the row's last
+  int lane;
+  template <typename F> __device__ __forceinline__ void each(F f) const {
+#pragma unroll 2
+    for (int c = 0; begin + 128 * c < end; ++c) {
+      const int t = begin + 128 * c + 4 * lane;
+      const float4 v = mine[c * kSampleThreads];
+      if (t < end) f(t, v.x);
+      if (t + 1 < end) f(t + 1, v.y);
+      if (t + 2 < end) f(t + 2, v.z);
+      if (t + 3 < end) f(t + 3, v.w);
+    }
+  }
+};
+
+// Which step a value lies in; never decreasing as the value falls.
+__device__ __forceinline__ int bin_of(float v, float mx, float per) { return min(kBins - 1, (int)((mx - v) * per)); }
+
+// The step at which the weight of the team's histogram, added up from step 0, first reaches `target`, or -1; `above` = the
+// weight of the steps before it. LIMBS 1: counts; 3: masses in parts of 16, 16 and 9 bits (shared memory adds 32-bit words).
+template <int LIMBS>
+__device__ int find_bin(Team& team, const unsigned int* hist, unsigned long long target, unsigned long long& above) {
+  SampleShared& sh = *team.sh;
+  constexpr int kPer = kBins / kSampleThreads;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long h[kPer], mine = 0ull;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    unsigned long long t = 0ull;
+#pragma unroll
+    for (int l = 0; l < LIMBS; ++l) {
+      unsigned long long part = 0ull;
+      for (int c = 0; c < kSampleTeam; ++c) part += team.cluster.map_shared_rank(hist, c)[l * kBins + threadIdx.x * kPer + j];
+      t += part << (16 * l);
+    }
+    h[j] = t;
+    mine += t;
+  }
+  unsigned long long incl = mine;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (threadIdx.x == 0) sh.chosen = -1;
+  if (lane == 31) sh.hist[warp] = incl;
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) incl += sh.hist[w];
+  unsigned long long acc = incl - mine;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    if (acc < target && acc + h[j] >= target) {      // one thread and step at most
+      sh.chosen = threadIdx.x * kPer + j;
+      sh.above = acc;
+    }
+    acc += h[j];
+  }
+  __syncthreads();
+  const int found = sh.chosen;
+  above = sh.above;
+  __syncthreads();
+  return found;
+}
+
+// Among the n entries: the key of the one whose inclusion, in descending key order, makes the weight (starting from `above`) reach
+// `target`. COUNT: each weighs 1, otherwise its mass. The block is on its own. Entries below floor_key weigh nothing.
+template <bool COUNT>
+__device__ unsigned int list_threshold(Team& team, const int* token, const float* value, int n, float mx, unsigned int floor_key,
+                                       unsigned long long above, unsigned long long target, unsigned long long* scratch) {
+  SampleShared& sh = *team.sh;
+  if (n > kSmallList) return radix_threshold<COUNT>(team, ListSource{token, value, n}, mx, floor_key, target - above, scratch);
+  unsigned int* keys = reinterpret_cast<unsigned int*>(scratch + kSmallList);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const unsigned int key = sort_key(value[i]);
+    keys[i] = key;
+    scratch[i] = key >= floor_key ? (COUNT ? 1ull : mass_of(value[i], mx)) : 0ull;
+  }
+  if (threadIdx.x == 0) sh.prefix = 0u;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const unsigned int key = keys[i];
+    unsigned long long more = above, same = 0ull;
+    for (int j = 0; j < n; ++j) {
+      const unsigned int k = keys[j];
+      const unsigned long long w = scratch[j];
+      more += k > key ? w : 0ull;
+      same += k == key ? w : 0ull;
+    }
+    if (more < target && more + same >= target) sh.prefix = key;      // (equal entries write the same)
+  }
+  __syncthreads();
+  const unsigned int found = sh.prefix;
+  __syncthreads();
+  return found;
+}
+
+// Appends (token, value) to this block's list.
+__device__ __forceinline__ void keep_candidate(SampleShared& sh, int* tokens, float* values, int t, float v) {
+  const int at = atomicAdd(&sh.count, 1);
+  if (at < kQuickList) { tokens[at] = t; values[at] = v; }
+}
+
+// The blocks' lists together in block 0 (at all_token / all_value), if they fit: returns their length, or -1. After it the other
+// blocks' lists are free. Once per launch.
+__device__ int gather_lists(Team& team, int* tokens, float* values, int* all_token, float* all_value, int rank, int most) {
+  SampleShared& sh = *team.sh;
+  __syncthreads();
+  if (threadIdx.x == 0) sh.x.total = sh.count;
+  team.cluster.sync();
+  int n = 0;
+  for (int c = 0; c < kSampleTeam; ++c) n += team.cluster.map_shared_rank(&sh.x, c)->total;
+  if (n > most) return -1;
+  if (rank == 0) {
+    int at = 0;
+    for (int c = 0; c < kSampleTeam; ++c) {
+      const int k = team.cluster.map_shared_rank(&sh.x, c)->total;
+      const int* their_token = team.cluster.map_shared_rank(tokens, c);
+      const float* their_value = team.cluster.map_shared_rank(values, c);
+      for (int i = threadIdx.x; i < k; i += blockDim.x) { all_token[at + i] = their_token[i]; all_value[at + i] = their_value[i]; }
+      at += k;
+    }
+  }
+  team.cluster.sync();
+  return n;
+}
+
+__global__ void __cluster_dims__(kSampleTeam, 1, 1) __launch_bounds__(kSampleThreads, 2)
 sample_kernel(const float* __restrict__ logits, long long ld, int limit, float temperature, int top_k, float top_p,
               float min_p, const float* __restrict__ uniform, int* __restrict__ out) {
   pdl_enter();
   __shared__ SampleShared sh;
-  __shared__ int cand_token[kCandidates];
-  __shared__ float cand_value[kCandidates];
-  extern __shared__ __align__(16) unsigned long long warp_hist[];      // [warps][256]
+  __shared__ int quick_token[kQuickList];
+  __shared__ float quick_value[kQuickList];
+  int* cand_token = quick_token;
+  float* cand_value = quick_value;
+  extern __shared__ __align__(16) unsigned long long dynamic[];
+  unsigned long long* warp_hist = dynamic;         // general path: [warps][256]
+  float4* held = reinterpret_cast<float4*>(dynamic);                                        // quick path: [kHeld][threads]
+  unsigned int* bins = reinterpret_cast<unsigned int*>(dynamic + kHeldTokens / 2);          // quick path: [3][kBins]
   Team team{cg::this_cluster(), &sh, false, kSampleTeam};
   const int r = blockIdx.x / kSampleTeam, rank = (int)team.cluster.block_rank();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -406,16 +555,169 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
   const RowSource whole{raw, temperature};
   __syncthreads();
 
-  // division by a positive temperature keeps the order, so the largest quotient is the quotient of the largest value
   float mx = -INFINITY;
+  unsigned int floor_key = 0u;
+  bool listed = false, cut = false;      // cut: floor_key says already what top-p leaves
+  int n_listed = 0;
+
+  const bool count_first = top_k > 0 && top_k < limit;
+  const int chunks = (raw.n + 128 * kSampleWarps - 1) / (128 * kSampleWarps);
+  Held mine{held + threadIdx.x, part_begin + warp * chunks * 128, min(part_end, part_begin + (warp + 1) * chunks * 128), lane};
+  bool quick = per_block <= kHeldTokens && (count_first || top_p < 1.0f);      // the same for all blocks of a row
+  if (quick) {
+    // the one read of the row; the largest value, a lower bound, and whether anything is no number
+    const bool aligned = (reinterpret_cast<uintptr_t>(row + part_begin) & 15) == 0;
+    float most = -INFINITY;
+    bool bad = false;
+#pragma unroll 5
+    for (int c = 0; mine.begin + 128 * c < mine.end; ++c) {
+      const int t = mine.begin + 128 * c + 4 * lane;
+      float4 v = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+      if (t + 3 < mine.end && aligned) {
+        v = *reinterpret_cast<const float4*>(row + t);
+      } else {
+        if (t < mine.end) v.x = row[t];
+        if (t + 1 < mine.end) v.y = row[t + 1];
+        if (t + 2 < mine.end) v.z = row[t + 2];
+        if (t + 3 < mine.end) v.w = row[t + 3];
+      }
+      bad = bad || v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w;
+      most = fmaxf(most, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+      mine.mine[c * kSampleThreads] = v;
+    }
+    // At least as many values as there are warps (threads) with a maximum of their own reach the smallest of those maxima.
+    const float warp_most = warp_max(most);
+    const int warps_with = (limit + chunks * 128 - 1) / max(1, chunks * 128);      // warps of the row that hold tokens, about
+    float low = top_k <= warps_with / 2 ? warp_most : most;
+    if (mine.begin + 4 * lane >= mine.end) low = INFINITY;
+    const float low_block = -block_max(-low, sh.red);
+    const float most_block = block_max(most, sh.red);
+    const int any_bad = __syncthreads_or(bad ? 1 : 0);
+    const int f = team.flip();
+    if (threadIdx.x == 0) { sh.x.max[f] = most_block; sh.x.low = low_block; sh.x.bad = any_bad; sh.count = 0; }
+    for (int i = threadIdx.x; i < 3 * kBins; i += blockDim.x) bins[i] = 0u;
+    team.cluster.sync();
+    float row_most = -INFINITY, row_low = INFINITY;
+    for (int c = 0; c < kSampleTeam; ++c) {
+      const SampleExchange* x = team.cluster.map_shared_rank(&sh.x, c);
+      row_most = fmaxf(row_most, x->max[f]);
+      row_low = fminf(row_low, x->low);
+      quick = quick && x->bad == 0;
+    }
+    const float size = fmaxf(fabsf(row_most), fabsf(row_low));
+    const float width = (row_most - row_low) / kBins;
+    quick = quick && size < 1e30f;      // (not for infinities)
+    if (count_first) {
+      // Candidates are taken one step below the k-th value's: a step must be wider than what rounds to the same quotient.
+      quick = quick && width > 1e-5f * size && width > 1e-30f * temperature && temperature > 1e-30f;
+      if (quick) {
+        const float per = (kBins - 0.5f) / (row_most - row_low);
+        mine.each([&](int, float x) { if (x >= row_low) atomicAdd(&bins[bin_of(x, row_most, per)], 1u); });
+        team.cluster.sync();
+        unsigned long long above;
+        const int bin = find_bin<1>(team, bins, (unsigned long long)top_k, above);
+        quick = bin >= 0 && bin < kBins - 2;
+        if (quick) {
+          mine.each([&](int t, float x) {
+            if (x >= row_low && bin_of(x, row_most, per) <= bin + 1) keep_candidate(sh, cand_token, cand_value, t, x);
+          });
+          int* all_token = reinterpret_cast<int*>(bins);
+          float* all_value = reinterpret_cast<float*>(dynamic);      // the held row is not needed any more where the list fits
+          const int n = gather_lists(team, cand_token, cand_value, all_token, all_value, rank, kQuickList);
+          quick = n >= 0;
+          if (quick) {
+            if (rank != 0) return;
+            team.solo = true;
+            mx = row_most / temperature;
+            unsigned long long* scratch = dynamic + kQuickList / 2;
+            const unsigned int kth = list_threshold<true>(team, all_token, all_value, n, 0.0f, 0u, 0ull, (unsigned long long)top_k, scratch);
+            const unsigned int b = (kth & 0x80000000u) ? (kth & 0x7fffffffu) : ~kth;     // back to the float
+            floor_key = sort_key(__uint_as_float(b) / temperature);
+            // in token order (the draw walks it), divided by the temperature
+            for (int i = threadIdx.x; i < n; i += blockDim.x) {
+              const int t = all_token[i];
+              int pos = 0;
+              for (int j = 0; j < n; ++j) pos += all_token[j] < t ? 1 : 0;
+              cand_token[pos] = t;
+              cand_value[pos] = all_value[i] / temperature;
+            }
+            __syncthreads();
+            listed = true;
+            n_listed = n;
+            if (top_p < 1.0f) {
+              const unsigned long long total = kept_mass(team, ListSource{cand_token, cand_value, n}, mx, floor_key);
+              unsigned long long target = (unsigned long long)ceil((double)top_p * (double)total);
+              if (target < 1ull) target = 1ull;
+              if (target > total) target = total;
+              floor_key = list_threshold<false>(team, cand_token, cand_value, n, mx, floor_key, 0ull, target, scratch);
+            }
+            cut = true;
+          }
+        }
+      }
+    } else if (quick) {
+      // top-p over the whole row: quotients, of which those more than 16 below the largest weigh next to nothing
+      mx = row_most / temperature;
+      const float per = (kBins - 0.5f) / 16.0f, lowest = mx - 16.0f;
+      quick = size / temperature < 1e4f;      // (a step must be wider than a quotient's last place)
+      if (quick) {
+        unsigned long long part = 0ull;
+        mine.each([&](int, float x) {
+          const float v = x / temperature;
+          const unsigned long long m = mass_of(v, mx);
+          part += m;
+          if (v >= lowest) {
+            unsigned int* at = bins + bin_of(v, mx, per);
+            atomicAdd(at, (unsigned int)(m & 0xffffull));
+            atomicAdd(at + kBins, (unsigned int)((m >> 16) & 0xffffull));
+            atomicAdd(at + 2 * kBins, (unsigned int)(m >> 32));
+          }
+        });
+        const unsigned long long total = team.sum(part);       // (its cluster barrier also ends the histograms)
+        unsigned long long target = (unsigned long long)ceil((double)top_p * (double)total), above;
+        if (target < 1ull) target = 1ull;
+        if (target > total) target = total;
+        const int bin = find_bin<3>(team, bins, target, above);
+        quick = bin >= 0 && bin < kBins - 1;
+        if (quick) {
+          mine.each([&](int t, float x) {
+            const float v = x / temperature;
+            if (v >= lowest && bin_of(v, mx, per) == bin) keep_candidate(sh, cand_token, cand_value, t, v);
+          });
+          // block 0 has the histogram's place for the list and what is worked out on it (it still holds its part of the row)
+          int* all_token = reinterpret_cast<int*>(bins);
+          float* all_value = reinterpret_cast<float*>(bins) + kSmallList;
+          const int n = gather_lists(team, cand_token, cand_value, all_token, all_value, rank, kSmallList);
+          quick = n >= 0;
+          if (quick && rank == 0) {
+            team.solo = true;
+            const unsigned int key = list_threshold<false>(team, all_token, all_value, n, mx, 0u, above, target,
+                                                             reinterpret_cast<unsigned long long*>(bins + 2 * kSmallList));
+            team.solo = false;
+            if (threadIdx.x == 0) sh.x.key = key;
+          }
+          if (quick) {
+            team.cluster.sync();
+            floor_key = team.cluster.map_shared_rank(&sh.x, 0)->key;
+            cut = true;
+          }
+        }
+      }
+    }
+    if (!quick) team.cluster.sync();        // nobody clears its shared memory while another block still reads it
+  }
+
+  if (!quick) {
+    floor_key = 0u;
+    cand_token = reinterpret_cast<int*>(warp_hist + kSampleWarps * 256);
+    cand_value = reinterpret_cast<float*>(cand_token + kCandidates);
+  // division by a positive temperature keeps the order, so the largest quotient is the quotient of the largest value
+  mx = -INFINITY;
   raw.each([&](int, float x) { mx = fmaxf(mx, x); });
   mx = team.max(mx) / temperature;
 
   // ---- top-k: the key of the k-th largest value; what it leaves usually fits in shared memory, and everything
   // after works on that short list in one block (sorted by token, since the draw walks in token order) ----
-  unsigned int floor_key = 0u;
-  bool listed = false;
-  int n_listed = 0;
   if (top_k > 0 && top_k < limit) {
     // The k-th largest quotient is the quotient of the k-th largest stored value, so the descent runs on the stored
     // values (no division). Values a little below the k-th one can still round to the same quotient and then stay
@@ -497,10 +799,11 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
       __syncthreads();
     }
   }
+  }
   const ListSource list{cand_token, cand_value, n_listed};
 
   // ---- top-p: the key at which the descending running mass of what top-k left reaches p * total ----
-  if (top_p < 1.0f) {
+  if (top_p < 1.0f && !cut) {
     const unsigned long long total = listed ? kept_mass(team, list, mx, floor_key) : kept_mass(team, whole, mx, floor_key);
     unsigned long long target = (unsigned long long)ceil((double)top_p * (double)total);
     if (target < 1ull) target = 1ull;
@@ -661,7 +964,9 @@ extern "C" int slb_sample(const float* logits, long long ld, int rows, int limit
   SLB_REQUIRE(top_k >= 0 && top_p > 0.0f && min_p >= 0.0f && min_p <= 1.0f, "sample: top_k=%d top_p=%g min_p=%g", top_k,
               (double)top_p, (double)min_p);
   if (rows == 0) return 0;
-  const size_t hist_bytes = (size_t)(kSampleThreads / 32) * 256 * sizeof(unsigned long long);
+  // the quick path's row and histogram; the general path's warp histograms and candidates lie in the same place
+  constexpr size_t hist_bytes = kHeldTokens * sizeof(float) + 3 * kBins * sizeof(unsigned int);
+  static_assert(kSampleWarps * 256 * sizeof(unsigned long long) + 2 * kCandidates * sizeof(int) <= kHeldTokens * sizeof(float), "the general path's place");
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_bytes);
