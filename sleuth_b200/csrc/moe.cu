@@ -16,6 +16,7 @@
 // The last experts of the router may be identity experts: they have no matrices and return the token's own input row. They
 // come last in the expert order too, so the product kernels, which are given the number of experts that have matrices, never
 // meet their pairs; the kernels that sum a token's choices add weight * h for them.
+// Steps of few pairs (single tokens) take kernels of their own, moe_few_*.
 // In bfloat16 with inner sizes that are multiples of 8 the two products run on the tensor cores (moe_mma_kernel);
 // the kernels above then serve float32 and odd sizes.
 #include "mma_sync.cuh"
@@ -537,6 +538,7 @@ __global__ void __launch_bounds__(128) moe_mma_kernel(const __nv_bfloat16* __res
 
 // ---- few pairs (single-token steps): a warp per output, every weight row streamed once per pair that uses it ----
 // (act rows lie in the order of the pairs here: nothing needs the expert order, so a step of few pairs skips the layout.)
+// These two serve float32 and widths that are no multiples of 32; the kernels behind them the rest.
 // grid (pairs, column groups of 8): act[pair, j] = f(gate_e[j] . h[token]) * (up_e[j] . h[token]).
 template <typename T>
 __global__ void __launch_bounds__(256) moe_few_gate_up_kernel(const T* __restrict__ h, const T* __restrict__ w_gu,
@@ -628,6 +630,197 @@ __global__ void __launch_bounds__(256) moe_few_down_kernel(const T* __restrict__
     if (extra) total += extra[(size_t)t * dim + n];
     float* dst = x + (size_t)t * dim + n;
     *dst = store ? total : *dst + total;
+  }
+}
+
+// The same two products on the warp-level tensor cores (bfloat16, widths that are multiples of 32), every expert's matrices read
+// once for all the pairs that chose it. What bounds a step of few pairs is that read, so it is laid out as in gemm_skinny.cu: a lane
+// fetches 16 neighbouring bytes of a weight row straight into the layout the instruction wants, eight such loads in flight; the
+// rows of the instruction are the pairs with the expert (sixteen at a time), its columns eight weight rows. Both products, us with
+// every pair for itself (the kernels above) / now: width 2,048, 64 experts of 1,408, 6 a token: 8 tokens 174 / 116 (about 35 experts, 5.2 TB/s),
+// 4 tokens 91 / 74, 1 token 42 / 29; width 1,024, 16 experts of 768, 4 a token: 16 tokens 69 / 30, 8 tokens 39 / 26, 1 token 14 / 11.
+struct MoeFewArgs {
+  const __nv_bfloat16* h;
+  const __nv_bfloat16* w_gu;
+  const __nv_bfloat16* w_down;
+  const int* choice;
+  const float* weight;
+  __nv_bfloat16* act;
+  float* x;
+  const float* extra;
+  int pairs, top, dim, ff, E, store;
+  GateAct gate;
+};
+
+__device__ __forceinline__ uint4 load_weights16(const void* p) {      // read once: not kept in L1
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+// Pairs 0 .. 63 as bits; a lane holds the choices of pairs `lane` and `lane + 32` (-1 for none).
+__device__ __forceinline__ unsigned long long pairs_with(int c0, int c1, int e) {
+  const unsigned lo = __ballot_sync(0xffffffffu, c0 == e), hi = __ballot_sync(0xffffffffu, c1 == e);
+  return (unsigned long long)hi << 32 | lo;
+}
+
+// Takes up to sixteen pairs out of `with`; this lane's rows of the instruction are numbers g and g + 8 of them (-1 beyond).
+// Returns how many there are.
+__device__ __forceinline__ int take_rows(unsigned long long& with, int g, int& p0, int& p1) {
+  p0 = p1 = -1;
+  int n = 0;
+  for (; n < 16 && with; ++n) {
+    const int p = __ffsll(with) - 1;
+    with &= with - 1;
+    if (n == g) p0 = p;
+    if (n == g + 8) p1 = p;
+  }
+  return n;
+}
+
+// grid (pairs, groups of 8 columns): act[pair, j] = f(gate_e[j] . h[token]) * (up_e[j] . h[token]), for the pairs that share the expert of
+// pair blockIdx.x, if it is the first of them. The block's warps take an eighth of the width each.
+__global__ void __launch_bounds__(256, 3) moe_few_gate_up_mma_kernel(MoeFewArgs a) {
+  pdl_enter();
+  __shared__ float red[8][2][16][8 + 1];
+  __shared__ int row_pair[16];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int c0 = lane < a.pairs ? a.choice[lane] : -1, c1 = lane + 32 < a.pairs ? a.choice[lane + 32] : -1;
+  const int e = __shfl_sync(0xffffffffu, blockIdx.x < 32 ? c0 : c1, blockIdx.x & 31);
+  unsigned long long with = pairs_with(c0, c1, e);
+  if (e >= a.E || __ffsll(with) - 1 != (int)blockIdx.x) return;      // an identity expert; another pair leads (the whole block agrees)
+  const int feat = blockIdx.y * 8 + g;
+  const __nv_bfloat16* wrow[2];
+#pragma unroll
+  for (int f = 0; f < 2; ++f)
+    wrow[f] = feat < a.ff ? a.w_gu + ((size_t)e * 2 * a.ff + (size_t)f * a.ff + feat) * a.dim + 8 * t : nullptr;
+  const int kb_total = a.dim / 32, per = (kb_total + 7) / 8;
+  const int kb_begin = warp * per, kb_end = min(kb_total, kb_begin + per);
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  constexpr int U = 4;
+  while (with) {
+    int p0, p1;
+    const int n = take_rows(with, g, p0, p1);
+    const __nv_bfloat16* x0 = p0 >= 0 ? a.h + (size_t)(p0 / a.top) * a.dim + 8 * t : nullptr;
+    const __nv_bfloat16* x1 = p1 >= 0 ? a.h + (size_t)(p1 / a.top) * a.dim + 8 * t : nullptr;
+    float acc[2][4] = {};
+    for (int kb = kb_begin; kb < kb_end; kb += U) {
+      uint4 w[U][2], xa[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int f = 0; f < 2; ++f) w[u][f] = (kb + u < kb_end && wrow[f]) ? load_weights16(wrow[f] + (kb + u) * 32) : zero;
+#pragma unroll
+      for (int u = 0; u < U; ++u) xa[u] = (kb + u < kb_end && x0) ? *reinterpret_cast<const uint4*>(x0 + (kb + u) * 32) : zero;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint4 xb = (n > 8 && kb + u < kb_end && x1) ? *reinterpret_cast<const uint4*>(x1 + (kb + u) * 32) : zero;
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+          mma_bf16(acc[f], (const uint32_t[4]){xa[u].x, xb.x, xa[u].y, xb.y}, w[u][f].x, w[u][f].y);
+          mma_bf16(acc[f], (const uint32_t[4]){xa[u].z, xb.z, xa[u].w, xb.w}, w[u][f].z, w[u][f].w);
+        }
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+      red[warp][f][g][2 * t] = acc[f][0];
+      red[warp][f][g][2 * t + 1] = acc[f][1];
+      red[warp][f][g + 8][2 * t] = acc[f][2];
+      red[warp][f][g + 8][2 * t + 1] = acc[f][3];
+    }
+    if (warp == 0 && t == 0) { row_pair[g] = p0; row_pair[g + 8] = p1; }
+    __syncthreads();
+    const int r = threadIdx.x >> 3, c = threadIdx.x & 7, j = blockIdx.y * 8 + c;
+    if (r < n && j < a.ff) {
+      float gv = 0.f, uv = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) { gv += red[k][0][r][c]; uv += red[k][1][r][c]; }
+      a.act[(size_t)row_pair[r] * a.ff + j] = __float2bfloat16_rn(gated(a.gate, gv, uv));
+    }
+    if (with) __syncthreads();
+  }
+}
+
+// grid (groups of 8 columns): x[t, n] += (store: =) sum over the token's choices, in their order, of weight[pair] * (down_e[n] . act[pair]),
+// or weight[pair] * h[t, n] for an identity expert. A warp takes one of PIECES parts of the experts' width of one expert at a time.
+template <int PIECES>
+__global__ void __launch_bounds__(256, 2) moe_few_down_mma_kernel(MoeFewArgs a) {
+  pdl_enter();
+  __shared__ float product[PIECES][kMoeFewPairs][8];
+  __shared__ int leads[kMoeFewPairs];
+  __shared__ int n_leads;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n0 = blockIdx.x * 8;
+  const int c0 = lane < a.pairs ? a.choice[lane] : -1, c1 = lane + 32 < a.pairs ? a.choice[lane + 32] : -1;
+  if (warp == 0) {
+    // the first pair of every expert that has a matrix (the whole warp matches and shuffles, whatever its lanes hold)
+    const bool lowest0 = __ffs(__match_any_sync(0xffffffffu, c0)) - 1 == lane;
+    const bool lowest1 = __ffs(__match_any_sync(0xffffffffu, c1)) - 1 == lane;
+    bool seen = false;
+    for (int i = 0; i < 32; ++i) {
+      const int other = __shfl_sync(0xffffffffu, c0, i);
+      seen = seen || other == c1;
+    }
+    const bool first0 = lowest0 && c0 >= 0 && c0 < a.E, first1 = lowest1 && !seen && c1 >= 0 && c1 < a.E;
+    const unsigned lo = __ballot_sync(0xffffffffu, first0), hi = __ballot_sync(0xffffffffu, first1);
+    const unsigned below = (1u << lane) - 1u;
+    if (first0) leads[__popc(lo & below)] = lane;
+    if (first1) leads[__popc(lo) + __popc(hi & below)] = lane + 32;
+    if (lane == 0) n_leads = __popc(lo) + __popc(hi);
+  }
+  __syncthreads();
+  const int kb_total = a.ff / 32, per = (kb_total + PIECES - 1) / PIECES;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  constexpr int U = 8;
+  for (int unit = warp; unit < n_leads * PIECES; unit += 8) {
+    const int lead = leads[unit / PIECES], piece = unit % PIECES;
+    const int e = __shfl_sync(0xffffffffu, lead < 32 ? c0 : c1, lead & 31);
+    unsigned long long with = pairs_with(c0, c1, e);
+    const int kb_begin = piece * per, kb_end = min(kb_total, kb_begin + per);
+    const __nv_bfloat16* wrow = n0 + g < a.dim ? a.w_down + ((size_t)e * a.dim + n0 + g) * a.ff + 8 * t : nullptr;
+    while (with) {
+      int p0, p1;
+      const int n = take_rows(with, g, p0, p1);
+      const __nv_bfloat16* x0 = p0 >= 0 ? a.act + (size_t)p0 * a.ff + 8 * t : nullptr;
+      const __nv_bfloat16* x1 = p1 >= 0 ? a.act + (size_t)p1 * a.ff + 8 * t : nullptr;
+      float acc[4] = {};
+      for (int kb = kb_begin; kb < kb_end; kb += U) {
+        uint4 w[U], xa[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) w[u] = (kb + u < kb_end && wrow) ? load_weights16(wrow + (kb + u) * 32) : zero;
+#pragma unroll
+        for (int u = 0; u < U; ++u) xa[u] = (kb + u < kb_end && x0) ? *reinterpret_cast<const uint4*>(x0 + (kb + u) * 32) : zero;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const uint4 xb = (n > 8 && kb + u < kb_end && x1) ? *reinterpret_cast<const uint4*>(x1 + (kb + u) * 32) : zero;
+          mma_bf16(acc, (const uint32_t[4]){xa[u].x, xb.x, xa[u].y, xb.y}, w[u].x, w[u].y);
+          mma_bf16(acc, (const uint32_t[4]){xa[u].z, xb.z, xa[u].w, xb.w}, w[u].z, w[u].w);
+        }
+      }
+      if (p0 >= 0) { product[piece][p0][2 * t] = acc[0]; product[piece][p0][2 * t + 1] = acc[1]; }
+      if (p1 >= 0) { product[piece][p1][2 * t] = acc[2]; product[piece][p1][2 * t + 1] = acc[3]; }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < a.pairs / a.top * 8; i += 256) {
+    const int tok = i >> 3, c = i & 7, n = n0 + c;
+    if (n >= a.dim) continue;
+    float total = 0.f;
+    for (int k = 0; k < a.top; ++k) {
+      const int pair = tok * a.top + k;
+      float v = 0.f;
+      if (a.choice[pair] >= a.E) {
+        v = __bfloat162float(a.h[(size_t)tok * a.dim + n]);
+      } else {
+#pragma unroll
+        for (int piece = 0; piece < PIECES; ++piece) v += product[piece][pair][c];
+      }
+      total = fmaf(a.weight[pair], v, total);
+    }
+    if (a.extra) total += a.extra[(size_t)tok * a.dim + n];
+    float* dst = a.x + (size_t)tok * a.dim + n;
+    *dst = a.store ? total : *dst + total;
   }
 }
 
@@ -857,6 +1050,13 @@ extern "C" int slb_moe_experts(const void* h, const void* w_gu, const void* w_do
     if (dtype == kF32) {
       launch(moe_few_gate_up_kernel<float>, f1, block, 0, s, (const float*)h, (const float*)w_gu, choice, (float*)act, top, dim, ff, E, gate);
       launch(moe_few_down_kernel<float>, f2, block, 0, s, (const float*)h, (const float*)act, (const float*)w_down, choice, weight, x, extra, top, dim, ff, E, store);
+    } else if (dim % 32 == 0 && ff % 32 == 0) {
+      const MoeFewArgs a{(const __nv_bfloat16*)h, (const __nv_bfloat16*)w_gu, (const __nv_bfloat16*)w_down, choice, weight, (__nv_bfloat16*)act, x, extra,
+                         (int)pairs, top, dim, ff, E, store, gate};
+      launch(moe_few_gate_up_mma_kernel, f1, block, 0, s, a);
+      // parts of the experts' width: enough units for the eight warps where few experts are met
+      if (pairs <= 8) launch(moe_few_down_mma_kernel<4>, dim3((dim + 7) / 8), block, 0, s, a);
+      else launch(moe_few_down_mma_kernel<2>, dim3((dim + 7) / 8), block, 0, s, a);
     } else {
       launch(moe_few_gate_up_kernel<__nv_bfloat16>, f1, block, 0, s, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w_gu, choice,
              (__nv_bfloat16*)act, top, dim, ff, E, gate);
