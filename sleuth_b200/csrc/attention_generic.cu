@@ -52,6 +52,7 @@ template <> struct RowDot<float> {
     float d = 0.0f;
     if ((hd & 3) == 0) {
       const float4* k4 = reinterpret_cast<const float4*>(k);
+#pragma unroll 8
       for (int i = 0; i < hd / 4; ++i) {
         const float4 kv = k4[i];
         d = fmaf(q[4 * i + 0], kv.x, d);
@@ -72,6 +73,7 @@ template <> struct RowDot<__nv_bfloat16> {
     float d = 0.0f;
     if ((hd & 7) == 0) {
       const Bf16x8* k8 = reinterpret_cast<const Bf16x8*>(k);
+#pragma unroll 4
       for (int i = 0; i < hd / 8; ++i) {
         float f[8];
         unpack8(k8[i], f);
@@ -86,6 +88,7 @@ template <> struct RowDot<__nv_bfloat16> {
 };
 
 constexpr int kAttnWarps = 8;
+constexpr int kValueBatch = 8;      // value rows asked for together: one after the other, a warp waited for memory once per key (heads of 24, 60 keys: 11.1 -> 6.4 us)
 
 template <typename T, int PER_LANE>
 __global__ void __launch_bounds__(kAttnWarps * 32) attn_generic_kernel(AttnArgs a) {
@@ -137,14 +140,24 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_generic_kernel(AttnArgs 
 #pragma unroll
     for (int i = 0; i < PER_LANE; ++i) acc[i] *= alpha;
     const int first = max(lo - base, 0), last = min(31, pos - base);
-    for (int jj = first; jj <= last; ++jj) {
-      const float pj = __shfl_sync(0xffffffffu, p, jj);
-      const int rj = __shfl_sync(0xffffffffu, row, jj);
-      const T* vrow = vpool + (size_t)rj * vd;
+    // values in batches whose loads are all out before the first is used; the sums still take key after key
+    for (int j0 = first; j0 <= last; j0 += kValueBatch) {
+      T v[kValueBatch][PER_LANE];
 #pragma unroll
-      for (int i = 0; i < PER_LANE; ++i) {
-        const int c = lane + 32 * i;
-        if (c < vd) acc[i] = fmaf(pj, to_f32(vrow[c]), acc[i]);
+      for (int u = 0; u < kValueBatch; ++u) {
+        const int rj = __shfl_sync(0xffffffffu, row, min(j0 + u, 31));
+#pragma unroll
+        for (int i = 0; i < PER_LANE; ++i) {
+          const int c = lane + 32 * i;
+          if (j0 + u <= last && c < vd) v[u][i] = vpool[(size_t)rj * vd + c];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kValueBatch; ++u) {
+        const float pj = __shfl_sync(0xffffffffu, p, min(j0 + u, 31));
+#pragma unroll
+        for (int i = 0; i < PER_LANE; ++i)
+          if (j0 + u <= last && lane + 32 * i < vd) acc[i] = fmaf(pj, to_f32(v[u][i]), acc[i]);
       }
     }
     m = m_new;
