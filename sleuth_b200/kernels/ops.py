@@ -1175,7 +1175,7 @@ def moe_tile_words(tokens: int, top: int, experts: int) -> int:
     return 1 + 3 * (pairs // 128 + min(pairs, experts))
 
 
-MOE_FEW_PAIRS = 64      # up to this many (token, choice) pairs ``moe_experts`` runs a warp per output (csrc/moe.cu: kMoeFewPairs)
+MOE_FEW_PAIRS = 64      # up to this many (token, choice) pairs ``moe_experts`` takes its kernels for few pairs (csrc/moe.cu: kMoeFewPairs)
 
 
 def moe_route(h, w_router, bias, choice, weight, rank, counts, place, order, top: int, stream=None, logits=None,
@@ -1219,7 +1219,7 @@ def moe_experts(h, w_gate_up, w_down, counts, order, weight, act, y, x, top: int
                 store: bool = False) -> None:
     """x[t] += sum over the token's choices of weight * down_e(f(gate_e h) * (up_e h)). w_gate_up [experts, 2 * ff, d]
     (gate rows, then up rows), w_down [experts, d, ff]; act [T * top, ff] and y [T * top, d] float32 are scratch.
-    With ``choice`` and ``place`` (from ``moe_route``) a step of few pairs runs a warp per output instead of tiles, and then
+    With ``choice`` and ``place`` (from ``moe_route``) a step of few pairs takes kernels of its own instead of tiles, and then
     adds the rows of ``extra`` (float32, the stream's shape) as well, if given. ``identity``: so many experts behind the ones
     with matrices may be among the choices; they return h. ``store``: x = the sum instead of x += the sum."""
     _cuda(h, w_gate_up, w_down, counts, order, weight, act, y, x, choice, place, extra)

@@ -160,8 +160,13 @@ class ParallelLayer(Part):
         b.next_read = None
         with torch.cuda.stream(side):
             b.stream = side.cuda_stream
-            x2.zero_()
+            if getattr(self.ffn, "stores_result", False):
+                b.store_first = True            # it overwrites its target: nothing to clear
+            else:
+                x2.zero_()
             self.ffn.forward(h2, x2, b, ws)
+            if getattr(b, "store_first", False):
+                raise RuntimeError(f"{type(self.ffn).__name__} says it stores its result and did not")
         b.stream = main.cuda_stream
         ws.top = max(ws.top, ws.high)
         ws.high = max(seen, ws.high)
