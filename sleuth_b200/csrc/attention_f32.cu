@@ -469,7 +469,8 @@ __global__ void __launch_bounds__(HD) attn_f32_join_kernel(AttnF32Args a) {
 template <int HD, int GP>
 static int launch_token(const AttnF32Args& a, cudaStream_t s) {
   constexpr int smem = token_smem<HD, GP>();
-  static const cudaError_t e = cudaFuncSetAttribute(attn_f32_token_kernel<HD, GP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  static std::atomic<unsigned long long> allowed;
+  const cudaError_t e = allow_shared((const void*)attn_f32_token_kernel<HD, GP>, smem, allowed);
   if (e != cudaSuccess) return fail(2, "attention_f32: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
   // about four blocks an SM; a block with several chunks takes them in turn
   const int pairs = a.n_seqs * a.kv_heads;
@@ -490,7 +491,8 @@ static int launch_f32(const AttnF32Args& a, int max_count, cudaStream_t s) {
     return launch_token<HD, 16>(a, s);
   }
   constexpr int smem = prompt_smem<HD>();
-  static const cudaError_t e = cudaFuncSetAttribute(attn_f32_prompt_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  static std::atomic<unsigned long long> allowed;
+  const cudaError_t e = allow_shared((const void*)attn_f32_prompt_kernel<HD>, smem, allowed);
   if (e != cudaSuccess) return fail(2, "attention_f32: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
   const int tile_tokens = kRows / G, tiles = (max_count + tile_tokens - 1) / tile_tokens;
   SLB_REQUIRE(tiles < 65536 && a.n_seqs < 65536, "attention_f32: %d tiles, %d sequences", tiles, a.n_seqs);

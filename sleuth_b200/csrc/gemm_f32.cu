@@ -339,7 +339,8 @@ static int launch_rows(const GemmF32Args& a, cudaStream_t s) {
   using S = RowsShape<MP, NT, CH, D, VEC>;
   static_assert(S::kSmem <= 227 * 1024, "the ring must fit shared memory");
   const auto kernel = gemm_f32_rows_kernel<MP, NT, CH, D, VEC>;
-  static const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem);
+  static std::atomic<unsigned long long> allowed;
+  const cudaError_t e = allow_shared((const void*)kernel, S::kSmem, allowed);
   if (e != cudaSuccess) return fail(2, "gemm_f32: cannot reserve %d bytes of shared memory: %s", S::kSmem, cudaGetErrorString(e));
   const int tiles = (a.N + NT - 1) / NT, row_tiles = (a.M + MP - 1) / MP;
   SLB_REQUIRE(row_tiles < 65536, "gemm_f32: M=%d needs more than 65535 row tiles", a.M);
@@ -376,7 +377,8 @@ static int launch_tile(const GemmF32Args& a, cudaStream_t s) {
   // One block an SM is asked for (by its shared memory) where every tile gets an SM of its own: left to itself a kernel that
   // starts while the one before still runs finds half-empty SMs and doubles up there (1,500 x 1,024 x 2,048: 276 instead of 176 us).
   constexpr int kAlone = 116 * 1024;
-  static const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAlone);
+  static std::atomic<unsigned long long> allowed;
+  const cudaError_t e = allow_shared((const void*)kernel, kAlone, allowed);
   if (e != cudaSuccess) return fail(2, "gemm_f32: cannot reserve %d bytes of shared memory: %s", kAlone, cudaGetErrorString(e));
   const dim3 grid((a.N + kTileN - 1) / kTileN, (a.M + 16 * RT - 1) / (16 * RT));
   SLB_REQUIRE(grid.y < 65536, "gemm_f32: M=%d needs more than 65535 row tiles", a.M);
