@@ -679,12 +679,9 @@ static int launch_prefill(const FlashArgs& a, int n_seqs, int max_count, cudaStr
   const int G = a.heads / a.kv_heads;
   const int tiles = (max_count * G + 63) / 64;
   const int smem = 5 * 64 * HD * 2;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return fail(2, "attention (prefill): cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    configured = true;
-  }
+  static std::atomic<unsigned long long> allowed;
+  const cudaError_t e = allow_shared((const void*)attn_prefill_kernel<HD>, smem, allowed);
+  if (e != cudaSuccess) return fail(2, "attention (prefill): cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
   dim3 grid(tiles, a.kv_heads, n_seqs);
   launch(attn_prefill_kernel<HD>, dim3(grid), dim3(kFlashThreads), smem, s, a);
   return check_launch("attention (prefill)");
@@ -704,12 +701,9 @@ static int launch_decode_staged(const FlashArgs& a, int n_seqs, cudaStream_t s) 
   const int tiles_bytes = 2 * S * 16 * W * HD * 2 + 16 * HD * 2;
   const int merge_bytes = (W * 16 * HD + 2 * W * 16) * 4;
   const int smem = tiles_bytes > merge_bytes ? tiles_bytes : merge_bytes;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<HD, S, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return fail(2, "attention (decode): cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    configured = true;
-  }
+  static std::atomic<unsigned long long> allowed;
+  const cudaError_t e = allow_shared((const void*)attn_decode_kernel<HD, S, W>, smem, allowed);
+  if (e != cudaSuccess) return fail(2, "attention (decode): cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
   dim3 grid(a.splits * row_tiles, a.kv_heads, n_seqs);
   if (a.qkv != nullptr)      // the fused form asks for its pages before it waits for the kernel in front of it
     launch_prefetching(attn_decode_kernel<HD, S, W>, dim3(grid), dim3(W * 32), smem, s, a);

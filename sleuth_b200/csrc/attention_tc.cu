@@ -773,13 +773,9 @@ template <int HD>
 static int launch_attn_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnTcArgs& a,
                           int n_seqs, int max_count, bool wide, cudaStream_t s) {
   const int total = wide ? AttnWideLayout<HD>::TOTAL : AttnTcLayout<HD>::TOTAL;
-  static bool configured[2] = {false, false};
-  if (!configured[wide]) {
-    cudaError_t e = wide ? cudaFuncSetAttribute(attn_tc_wide_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, total)
-                         : cudaFuncSetAttribute(attn_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, total);
-    if (e != cudaSuccess) return fail(2, "attention (tcgen05): cannot reserve %d bytes of shared memory: %s", total, cudaGetErrorString(e));
-    configured[wide] = true;
-  }
+  static std::atomic<unsigned long long> allowed[2];
+  const cudaError_t e = allow_shared(wide ? (const void*)attn_tc_wide_kernel<HD> : (const void*)attn_tc_kernel<HD>, total, allowed[wide]);
+  if (e != cudaSuccess) return fail(2, "attention (tcgen05): cannot reserve %d bytes of shared memory: %s", total, cudaGetErrorString(e));
   const int G = a.heads / a.kv_heads;
   const int tiles = (max_count * G + kAtRows - 1) / kAtRows;
   dim3 grid(tiles, a.kv_heads, n_seqs);

@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "grants.h"
+
 namespace slb {
 
 constexpr int kPageTokens = 64;   // tokens per cache page

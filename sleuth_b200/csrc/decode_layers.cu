@@ -933,14 +933,18 @@ static int dl_red_bytes(int rows) { return kDlMaxAcc * kDlConsumerWarps * rows *
 
 template <int HD>
 static int launch_decode_layers(const DlHost& h, const CUtensorMap& m0, const CUtensorMap& m1, int smem, cudaStream_t s) {
-  static int configured = 0;
-  if (configured < smem) {
-    cudaError_t e = cudaFuncSetAttribute(decode_layers_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return fail(2, "decode_layers: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    configured = smem;
-  }
+  // all that a block can have: the ring's length differs from call to call
+  int dev = 0, most = 0;
+  cudaFuncAttributes own = {};
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&own, decode_layers_kernel<HD>);
+  most -= (int)own.sharedSizeBytes;
+  static std::atomic<unsigned long long> allowed;
+  if (e == cudaSuccess) e = smem > most ? cudaErrorInvalidValue : allow_shared((const void*)decode_layers_kernel<HD>, most, allowed);
+  if (e != cudaSuccess) return fail(2, "decode_layers: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
   int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_layers_kernel<HD>, kDlThreads, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_layers_kernel<HD>, kDlThreads, smem);
   if (e != cudaSuccess || per_sm < 1) return fail(2, "decode_layers: a block does not fit an SM (%s)", cudaGetErrorString(e));
   e = cudaMemsetAsync(h.args.barrier, 0, 2 * sizeof(unsigned int), s);
   if (e != cudaSuccess) return fail(2, "decode_layers: clearing the barrier failed: %s", cudaGetErrorString(e));

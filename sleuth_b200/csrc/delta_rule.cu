@@ -808,7 +808,8 @@ extern "C" int slb_delta_prep(float* rows, long long stride, int groups, int dim
 
 // Portions of more than kWalkTokens tokens run in chunks (states of up to 128 key channels).
 constexpr int kWalkTokens = 24;
-static bool runs_in_chunks(int max_count, int N) { return max_count > kWalkTokens && N <= 128; }
+constexpr int kChunkRows = 128;      // state rows the chunked form takes at most
+static bool runs_in_chunks(int max_count, int N) { return max_count > kWalkTokens && N <= kChunkRows; }
 
 // Floats of scratch memory that a step whose longest portion has max_count tokens needs (0: token by token).
 extern "C" long long slb_state_scan_scratch_floats(int n_seqs, int max_count, int H, int N, int P, int delta) {
@@ -824,13 +825,10 @@ static int launch_chunk_state(const ScanArgs& a, cudaStream_t s) {
   const bool delta = a.beta != nullptr;
   constexpr int NP = 16 * RN, KS = TH / (8 * PS);
   const int smem = (NP * PS + kChunk * PS + KS * (NP > kChunk ? NP : kChunk) * PS + 2 * (kChunk + 4) + (delta ? 4 : 2) * kChunk * NP) * 4;
-  static bool configured[2] = {false, false};
-  if (!configured[delta]) {
-    const cudaError_t e = delta ? cudaFuncSetAttribute(chunk_state_kernel<RN, PS, TH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
-                                : cudaFuncSetAttribute(chunk_state_kernel<RN, PS, TH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return fail(2, "state_scan: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    configured[delta] = true;
-  }
+  static std::atomic<unsigned long long> allowed[2];
+  const cudaError_t e = allow_shared(delta ? (const void*)chunk_state_kernel<RN, PS, TH, true> : (const void*)chunk_state_kernel<RN, PS, TH, false>, smem,
+                                     allowed[delta]);
+  if (e != cudaSuccess) return fail(2, "state_scan: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
   if (delta) launch(chunk_state_kernel<RN, PS, TH, true>, grid, block, (size_t)smem, s, a);
   else launch(chunk_state_kernel<RN, PS, TH, false>, grid, block, (size_t)smem, s, a);
   return check_launch("state_scan (states)");
@@ -870,12 +868,10 @@ extern "C" int slb_state_scan(const float* q, long long q_stride, const float* k
   SLB_REQUIRE(H < 65536 && (long long)H * ((P + kOutCols - 1) / kOutCols) < 65536, "state_scan: too many heads (%d)", H);
   if (delta) {
     const int smem = (N * kPad + kChunk * kPad) * 4;
-    static int most = 0;
-    if (smem > most) {
-      const cudaError_t e = cudaFuncSetAttribute(chunk_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return fail(2, "state_scan: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-      most = smem;
-    }
+    constexpr int most = (kChunkRows + kChunk) * kPad * 4;
+    static std::atomic<unsigned long long> allowed;
+    const cudaError_t e = allow_shared((const void*)chunk_solve_kernel, most, allowed);
+    if (e != cudaSuccess) return fail(2, "state_scan: cannot reserve %d bytes of shared memory: %s", most, cudaGetErrorString(e));
     launch(chunk_solve_kernel, dim3(a.chunks, H, n_seqs), dim3(128), (size_t)smem, s, a);
     const int rc = check_launch("state_scan (triangular systems)");
     if (rc) return rc;
@@ -890,12 +886,10 @@ extern "C" int slb_state_scan(const float* q, long long q_stride, const float* k
     if (rc) return rc;
   }
   const int smem = (kChunk * out_row(N) + out_keys_floats(N) + kChunk * kPad + kChunk * kOutCols) * 4;
-  static int most_out = 0;
-  if (smem > most_out) {
-    const cudaError_t e = cudaFuncSetAttribute(chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return fail(2, "state_scan: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    most_out = smem;
-  }
+  const int most = (kChunk * out_row(kChunkRows) + out_keys_floats(kChunkRows) + kChunk * kPad + kChunk * kOutCols) * 4;
+  static std::atomic<unsigned long long> allowed;
+  const cudaError_t e = allow_shared((const void*)chunk_out_kernel, most, allowed);
+  if (e != cudaSuccess) return fail(2, "state_scan: cannot reserve %d bytes of shared memory: %s", most, cudaGetErrorString(e));
   launch(chunk_out_kernel, dim3(a.chunks, H * ((P + kOutCols - 1) / kOutCols), n_seqs), dim3(256), (size_t)smem, s, a);
   return check_launch("state_scan (outputs)");
 }

@@ -259,13 +259,10 @@ static int launch_skinny_mode(const SkinnyArgs& a, cudaStream_t s) {
   const int blocks = (a.N + NF * 8 - 1) / (NF * 8);
   const size_t smem = NORM ? (size_t)a.M * (a.K * 2 + kNormPad) : 0;     // rows that do not exist multiply as zeros
   if (NORM) {
-    static bool configured = false;
-    if (!configured) {
-      const int most = 16 * (kNormMaxK * 2 + kNormPad);
-      cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<NF, MODE, NORM, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-      if (e != cudaSuccess) return fail(2, "gemm_skinny: cannot reserve %d bytes of shared memory: %s", most, cudaGetErrorString(e));
-      configured = true;
-    }
+    constexpr int most = 16 * (kNormMaxK * 2 + kNormPad);
+    static std::atomic<unsigned long long> allowed;
+    const cudaError_t e = allow_shared((const void*)gemm_skinny_kernel<NF, MODE, NORM, MT>, most, allowed);
+    if (e != cudaSuccess) return fail(2, "gemm_skinny: cannot reserve %d bytes of shared memory: %s", most, cudaGetErrorString(e));
   }
   launch_prefetching(gemm_skinny_kernel<NF, MODE, NORM, MT>, dim3(blocks), dim3(kSkinnyWarps * 32), smem, s, a);
   return check_launch("gemm_skinny");

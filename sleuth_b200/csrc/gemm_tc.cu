@@ -626,12 +626,9 @@ static int launch_tc(const CUtensorMap& mx, const CUtensorMap& mw, const TcArgs&
   constexpr int kBRows = PAIR ? BN / 2 : BN;
   constexpr int kStages = tc_stages(kBRows);
   const int smem = kStages * (kTcBM * kTcBK * 2 + kBRows * kTcBK * 2) + (2 * kStages + 4) * 8 + 16 + 1024;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, QKV, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return fail(2, "gemm_tc: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    configured = true;
-  }
+  static std::atomic<unsigned long long> allowed;
+  const cudaError_t e = allow_shared((const void*)gemm_tc_kernel<BN, QKV, PAIR>, smem, allowed);
+  if (e != cudaSuccess) return fail(2, "gemm_tc: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
   const int cols_per_tile = a.mode == kTcSwiglu ? BN / 2 : BN;
   const int rows_per_tile = PAIR ? 2 * kTcBM : kTcBM;
   const long long total = (long long)((a.N + cols_per_tile - 1) / cols_per_tile) * ((a.M + rows_per_tile - 1) / rows_per_tile);

@@ -992,11 +992,9 @@ extern "C" int slb_latent_attention(const void* q_lat, const void* q_raw, const 
     const dim3 grid((max_count + a.tq - 1) / a.tq, n_seqs, head_chunks * groups * splits), block(128);
 #define SLB_LATM(V)                                                                                              \
   do {                                                                                                           \
-    static bool raised = false;                                                                                  \
-    if (!raised) {                                                                                               \
-      cudaFuncSetAttribute(latent_attn_mma_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLatMaxSmem);   \
-      raised = true;                                                                                             \
-    }                                                                                                            \
+    static std::atomic<unsigned long long> allowed;                                                              \
+    const cudaError_t e = allow_shared((const void*)latent_attn_mma_kernel<V>, (int)kLatMaxSmem, allowed);       \
+    if (e != cudaSuccess) return fail(2, "latent_attention: cannot reserve shared memory: %s", cudaGetErrorString(e)); \
     launch(latent_attn_mma_kernel<V>, grid, block, smem, s, a, nt16, groups, buffers);                                   \
   } while (0)
     if (nt16 <= 4) SLB_LATM(4); else if (nt16 <= 8) SLB_LATM(8); else SLB_LATM(16);
@@ -1018,11 +1016,9 @@ extern "C" int slb_latent_attention(const void* q_lat, const void* q_raw, const 
   const dim3 grid((max_count + a.tq - 1) / a.tq, n_seqs, head_chunks * splits), block(kLatWarps * 32);
 #define SLB_LAT(TT, V)                                                                                   \
   do {                                                                                                   \
-    static bool raised_##V = false;                                                                      \
-    if (!raised_##V) {                                                                                   \
-      cudaFuncSetAttribute(latent_attn_kernel<TT, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
-      raised_##V = true;                                                                                 \
-    }                                                                                                    \
+    static std::atomic<unsigned long long> allowed;                                                      \
+    const cudaError_t e = allow_shared((const void*)latent_attn_kernel<TT, V>, 200 * 1024, allowed);     \
+    if (e != cudaSuccess) return fail(2, "latent_attention: cannot reserve shared memory: %s", cudaGetErrorString(e)); \
     launch(latent_attn_kernel<TT, V>, grid, block, bytes, s, a);                                         \
   } while (0)
 #define SLB_LAT_RV(TT)                                                                   \
@@ -1079,11 +1075,9 @@ extern "C" int slb_head_prompt_attention(const void* q, const void* kv, const vo
   const int kq = (dn + P) / 16, nv = dv / 16;
 #define SLB_HP(KQ, NV)                                                                                          \
   do {                                                                                                          \
-    static bool raised = false;                                                                                 \
-    if (!raised) {                                                                                              \
-      cudaFuncSetAttribute(head_prompt_mma_kernel<KQ, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLatMaxSmem); \
-      raised = true;                                                                                            \
-    }                                                                                                           \
+    static std::atomic<unsigned long long> allowed;                                                             \
+    const cudaError_t e = allow_shared((const void*)head_prompt_mma_kernel<KQ, NV>, (int)kLatMaxSmem, allowed); \
+    if (e != cudaSuccess) return fail(2, "head_prompt_attention: cannot reserve shared memory: %s", cudaGetErrorString(e)); \
     launch(head_prompt_mma_kernel<KQ, NV>, grid, block, smem, s, a, nbuf);                                         \
   } while (0)
   if (kq <= 8) {

@@ -650,11 +650,9 @@ extern "C" int slb_latent_decode_attention(const void* q_lat, const void* q_raw,
   const bool one = R <= 256;
 #define SLB_LD(MT, NP, KQ)                                                                                                   \
   do {                                                                                                                       \
-    static bool raised = false;                                                                                              \
-    if (!raised) {                                                                                                           \
-      cudaFuncSetAttribute(latent_decode_attn_kernel<MT, NP, KQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLdMaxSmem); \
-      raised = true;                                                                                                         \
-    }                                                                                                                        \
+    static std::atomic<unsigned long long> allowed;                                                                          \
+    const cudaError_t e = allow_shared((const void*)latent_decode_attn_kernel<MT, NP, KQ>, (int)kLdMaxSmem, allowed);        \
+    if (e != cudaSuccess) return fail(2, "latent_decode_attention: cannot reserve shared memory: %s", cudaGetErrorString(e)); \
     launch(latent_decode_attn_kernel<MT, NP, KQ>, grid, block, smem, s, a);                                                      \
   } while (0)
 #define SLB_LD_NP(MT) \
@@ -695,11 +693,9 @@ extern "C" int slb_latent_query(const float* lat, long long lat_stride, const fl
   a.w_uq = (const __nv_bfloat16*)w_uq; a.w_ukt = (const __nv_bfloat16*)w_ukt; a.cos_t = cos_t; a.sin_t = sin_t;
   a.q_lat = (__nv_bfloat16*)q_lat; a.q_raw = (__nv_bfloat16*)q_raw; a.pool = (__nv_bfloat16*)pool; a.pos = pos; a.table = table;
   a.stride = stride; a.n = n; a.H = H; a.K = K; a.q_rank = q_rank; a.R = R; a.P = P; a.dn = dn; a.rot = rot; a.eps = eps;
-  static bool raised = false;
-  if (!raised) {
-    cudaFuncSetAttribute(latent_query_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLdMaxSmem - 8 * 1024);
-    raised = true;
-  }
+  static std::atomic<unsigned long long> allowed;
+  const cudaError_t e = allow_shared((const void*)latent_query_kernel, (int)kLdMaxSmem - 8 * 1024, allowed);
+  if (e != cudaSuccess) return fail(2, "latent_query: cannot reserve shared memory: %s", cudaGetErrorString(e));
   launch_clusters(pdl_mode() != 0, kTeam, latent_query_kernel, dim3(kTeam * H, (n + kGroup - 1) / kGroup), dim3(256), query_smem(K, dn),
                   (cudaStream_t)stream, a);
   return check_launch("latent_query");
@@ -716,11 +712,9 @@ extern "C" int slb_latent_value(const float* parts, const void* o_lat, const flo
   LatentValueArgs a;
   a.parts = parts; a.o_lat = (const __nv_bfloat16*)o_lat; a.sinks = sinks; a.w_uv = (const __nv_bfloat16*)w_uv; a.gate = gate;
   a.y = (__nv_bfloat16*)y; a.gate_stride = gate_stride; a.n = n; a.H = H; a.R = R; a.dv = dv; a.splits = splits; a.gate_per_head = gate_per_head;
-  static bool raised = false;
-  if (!raised) {
-    cudaFuncSetAttribute(latent_value_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLdMaxSmem - 8 * 1024);
-    raised = true;
-  }
+  static std::atomic<unsigned long long> allowed;
+  const cudaError_t e = allow_shared((const void*)latent_value_kernel, (int)kLdMaxSmem - 8 * 1024, allowed);
+  if (e != cudaSuccess) return fail(2, "latent_value: cannot reserve shared memory: %s", cudaGetErrorString(e));
   launch_clusters(pdl_mode() != 0, kTeam, latent_value_kernel, dim3(kTeam * H, (n + kGroup - 1) / kGroup), dim3(256), value_smem(R),
                   (cudaStream_t)stream, a);
   return check_launch("latent_value");

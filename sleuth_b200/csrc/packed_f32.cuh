@@ -4,8 +4,6 @@
 // slot, so that shared-memory reads and address work fit between; operands are pairs as they lie in memory.
 #pragma once
 
-#include <atomic>
-
 #include "common.cuh"
 
 namespace slb {
@@ -43,17 +41,5 @@ __device__ __forceinline__ void copy_async(void* dst, const void* src, int bytes
 }
 __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
-
-// Lets `kernel` have `bytes` of dynamic shared memory on the current device; `done` remembers the devices (by bit) where it may.
-inline cudaError_t allow_shared(const void* kernel, int bytes, std::atomic<unsigned long long>& done) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
-  return e;
-}
 
 }  // namespace slb

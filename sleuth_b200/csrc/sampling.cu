@@ -967,12 +967,9 @@ extern "C" int slb_sample(const float* logits, long long ld, int rows, int limit
   // the quick path's row and histogram; the general path's warp histograms and candidates lie in the same place
   constexpr size_t hist_bytes = kHeldTokens * sizeof(float) + 3 * kBins * sizeof(unsigned int);
   static_assert(kSampleWarps * 256 * sizeof(unsigned long long) + 2 * kCandidates * sizeof(int) <= kHeldTokens * sizeof(float), "the general path's place");
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_bytes);
-    if (e != cudaSuccess) return fail(2, "sample: cannot reserve %d bytes of shared memory: %s", (int)hist_bytes, cudaGetErrorString(e));
-    configured = true;
-  }
+  static std::atomic<unsigned long long> allowed;
+  const cudaError_t e = allow_shared((const void*)sample_kernel, (int)hist_bytes, allowed);
+  if (e != cudaSuccess) return fail(2, "sample: cannot reserve %d bytes of shared memory: %s", (int)hist_bytes, cudaGetErrorString(e));
   launch(sample_kernel, dim3(rows * kSampleTeam), dim3(kSampleThreads), hist_bytes, (cudaStream_t)stream, logits, ld, limit, temperature, top_k, top_p,
          min_p, uniform, out);
   return check_launch("sample");
