@@ -25,6 +25,7 @@ struct GemmF32Args {
   const float* bias;
   float* C;
   int M, N, K, lda, ldw, ldc, accumulate;
+  int early;             // W is fetched before the wait for the kernel in front: only where no kernel writes it
 };
 
 // ---- few rows -------------------------------------------------------------------------------------------------
@@ -32,8 +33,8 @@ struct GemmF32Args {
 // can deliver (a lane's 16-byte read costs its full 16 bytes of 128 a cycle, broadcast or not). So warp w of a block owns segment
 // w of K, and streams its part of the block's weight rows (NT features), with the token rows' values for the same k, through a
 // ring of its own: CH k values a stage, D stages, 16-byte asynchronous copies, no barrier between warps until a tile's sums are
-// joined. A block goes from tile to tile (tile + gridDim.x) with the ring running on, so its copies never drain. The first
-// stages' weights are asked for before the wait for the kernel in front. LM lanes along the rows and 32 / LM along the features
+// joined. A block goes from tile to tile (tile + gridDim.x) with the ring running on, so its copies never drain. Where the
+// caller says that no kernel writes W, the first stages' weights are asked for before the wait for the kernel in front. LM lanes along the rows and 32 / LM along the features
 // make each lane's block R x CN as square as the tile allows. 0.6B sizes, 8 rows, us before (one chain per output over all of K, slices of
 // 32 k values behind barriers) / now: q/k/v 25.1 / 5.9, o 50.2 / 7.6, gate and up 34.9 / 9.1, down 74.5 / 10.8, head 479 / 145; 64 rows:
 // q/k/v 238 / 22.9, o 456 / 17.8.
@@ -96,13 +97,14 @@ gemm_f32_rows_kernel(GemmF32Args a, int seg, int tiles) {
   };
 
   pdl_launch_dependents();
+  if (!a.early) pdl_wait();
   if (chunks) {
     for (int s = 0; s < D - 1; ++s) {
       if (ask_tile < tiles) ask_weights();
       advance();
     }
   }
-  pdl_wait();
+  if (a.early) pdl_wait();
   if (chunks) {
     for (int s = 0, c = 0; s < D - 1; ++s) {
       ask_tokens(c, s);       // (beyond the last tile: copied and not used)
@@ -245,8 +247,9 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(GemmF32Args a, in
     }
   };
   pdl_launch_dependents();
+  if (!a.early) pdl_wait();
   fetch_weights(0);
-  pdl_wait();
+  if (a.early) pdl_wait();
   fetch_tokens(0);
 
   f32x2 acc[RT][4];
@@ -345,7 +348,7 @@ static int launch_rows(const GemmF32Args& a, cudaStream_t s) {
   const int tiles = (a.N + NT - 1) / NT, row_tiles = (a.M + MP - 1) / MP;
   SLB_REQUIRE(row_tiles < 65536, "gemm_f32: M=%d needs more than 65535 row tiles", a.M);
   const int room = S::kBlocksPerSm * sm_count() / row_tiles > 1 ? S::kBlocksPerSm * sm_count() / row_tiles : 1;
-  launch_prefetching(kernel, dim3(tiles < room ? tiles : room, row_tiles), dim3(256), S::kSmem, s, a, segment_length(a.K), tiles);
+  launch_with(a.early ? pdl_mode() != 0 : pdl_mode() == 1, kernel, dim3(tiles < room ? tiles : room, row_tiles), dim3(256), S::kSmem, s, a, segment_length(a.K), tiles);
   return check_launch("gemm_f32 (few rows)");
 }
 
@@ -383,7 +386,7 @@ static int launch_tile(const GemmF32Args& a, cudaStream_t s) {
   const dim3 grid((a.N + kTileN - 1) / kTileN, (a.M + 16 * RT - 1) / (16 * RT));
   SLB_REQUIRE(grid.y < 65536, "gemm_f32: M=%d needs more than 65535 row tiles", a.M);
   const int smem = tiles_of(a, RT) <= sm_count() ? kAlone : tile_smem(RT);
-  launch_prefetching(kernel, grid, dim3(256), smem, s, a, segment_length(a.K));
+  launch_with(a.early ? pdl_mode() != 0 : pdl_mode() == 1, kernel, grid, dim3(256), smem, s, a, segment_length(a.K));
   return check_launch("gemm_f32 (tiles)");
 }
 
@@ -391,14 +394,15 @@ static int launch_tile(const GemmF32Args& a, cudaStream_t s) {
 
 using namespace slb;
 
+// static_weight: no kernel writes W (a loaded matrix), so that it may be read while the kernel in front of this one still runs.
 extern "C" int slb_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda,
-                            int ldw, int ldc, int accumulate, void* stream) {
+                            int ldw, int ldc, int accumulate, int static_weight, void* stream) {
   SLB_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_f32: M=%d N=%d K=%d", M, N, K);
   SLB_REQUIRE(lda >= K && ldw >= K && ldc >= N, "gemm_f32: leading dimensions lda=%d ldw=%d ldc=%d for K=%d N=%d", lda,
               ldw, ldc, K, N);
   if (M == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
-  const GemmF32Args a{A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate};
+  const GemmF32Args a{A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, static_weight};
   const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
   int rt = 8;
   if (tile_cost(a, 6) < tile_cost(a, rt)) rt = 6;

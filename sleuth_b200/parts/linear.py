@@ -164,11 +164,11 @@ class Linear:
             h = h.tensor()
         if self.dtype == torch.float32:
             if into is not None:
-                ops.gemm_f32(h, self.weight, into, accumulate=True, stream=stream)
+                ops.gemm_f32(h, self.weight, into, accumulate=True, stream=stream, static_weight=True)
                 return into
             if out is None:
                 out = ws.take((M, self.out_features), torch.float32)
-            ops.gemm_f32(h, self.weight, out, stream=stream)
+            ops.gemm_f32(h, self.weight, out, stream=stream, static_weight=True)
             return out
         if use_skinny(M, self.out_features, self.in_features):
             if into is not None:

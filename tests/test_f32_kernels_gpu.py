@@ -110,3 +110,24 @@ def test_attention_f32_leaves_later_tokens_out():
     assert not torch.isfinite(got[100:]).any() and torch.isnan(got[110:]).all()
     one = run_f32(q[120:121], k_pool.to(DEV), v_pool.to(DEV), table.to(DEV), [120], [1], heads, kv_heads, hd, 0)
     assert torch.isnan(one).all()
+
+
+@pytest.mark.parametrize("M", [1, 8, 64, 700])
+def test_gemm_f32_second_operand_written_by_the_kernel_in_front(M):
+    """A product may have for its second operand what the launch before it writes: the same bits as with a wait between the two.
+    Only a caller that says that no kernel writes that operand has it read early."""
+    g = torch.Generator().manual_seed(M)
+    N, K = 2100, 1028
+    a, x = torch.randn(N, 512, generator=g).to(DEV), torch.randn(M, K, generator=g).to(DEV)
+    wait, straight = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    for turn in range(4):
+        b = torch.randn(K, 512, generator=g).to(DEV)
+        w = torch.full((N, K), float("nan"), device=DEV)
+        torch.cuda.synchronize()
+        ops().gemm_f32(a, b, w)                      # some hundred microseconds
+        ops().gemm_f32(x, w, straight)
+        torch.cuda.synchronize()
+        ops().gemm_f32(x, w, wait)
+        assert torch.equal(straight, wait)
+        ops().gemm_f32(x, w, straight, static_weight=True)       # (written long ago by now)
+        assert torch.equal(straight, wait)
