@@ -52,7 +52,6 @@ template <> struct RowDot<float> {
     float d = 0.0f;
     if ((hd & 3) == 0) {
       const float4* k4 = reinterpret_cast<const float4*>(k);
-#pragma unroll 8
       for (int i = 0; i < hd / 4; ++i) {
         const float4 kv = k4[i];
         d = fmaf(q[4 * i + 0], kv.x, d);
@@ -73,7 +72,6 @@ template <> struct RowDot<__nv_bfloat16> {
     float d = 0.0f;
     if ((hd & 7) == 0) {
       const Bf16x8* k8 = reinterpret_cast<const Bf16x8*>(k);
-#pragma unroll 4
       for (int i = 0; i < hd / 8; ++i) {
         float f[8];
         unpack8(k8[i], f);
@@ -88,7 +86,13 @@ template <> struct RowDot<__nv_bfloat16> {
 };
 
 constexpr int kAttnWarps = 8;
-constexpr int kValueBatch = 8;      // value rows asked for together: one after the other, a warp waited for memory once per key (heads of 24, 60 keys: 11.1 -> 6.4 us)
+// Value rows asked for together. One after the other a warp waits for memory once a key, but a batch costs registers, and from three
+// channels a lane on the blocks that no longer fit an SM are worth more than the shorter wait. us, one row at a time / in batches:
+//   float32   24 channels (8): 8 prompts of 400 377 / 229, a token at 4,000 260 / 102;  64 (2): 1,448 / 1,198, 295 / 183 (in batches of 8 1,254, 152,
+//             but four tokens on each of 8 pasts of 500 51 instead of 40);  96 (4): 1,772 / 1,828, eight of four tokens 59 / 78;
+//             128 (2): 2,062 / 2,490;  256 (2): 3,697 / 7,134
+//   bfloat16  24 (8): 297 / 231;  64 (8): 1,782 / 1,698, a token at 4,000 300 / 162;  96 (4): 1,686 / 1,782;  128 (4): 3,012 / 3,119;  256 (2): 5,627 / 6,312
+template <typename T> constexpr int value_batch(int per_lane) { return per_lane == 1 ? 8 : per_lane == 2 ? (sizeof(T) == 4 ? 2 : 8) : 1; }
 
 template <typename T, int PER_LANE>
 __global__ void __launch_bounds__(kAttnWarps * 32) attn_generic_kernel(AttnArgs a) {
@@ -140,8 +144,20 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_generic_kernel(AttnArgs 
 #pragma unroll
     for (int i = 0; i < PER_LANE; ++i) acc[i] *= alpha;
     const int first = max(lo - base, 0), last = min(31, pos - base);
-    // values in batches whose loads are all out before the first is used; the sums still take key after key
-    for (int j0 = first; j0 <= last; j0 += kValueBatch) {
+    // the sums take key after key, whether the rows come one by one or in batches whose loads are all out before the first is used
+    constexpr int kValueBatch = value_batch<T>(PER_LANE);
+    if constexpr (kValueBatch == 1) {
+      for (int jj = first; jj <= last; ++jj) {
+        const float pj = __shfl_sync(0xffffffffu, p, jj);
+        const int rj = __shfl_sync(0xffffffffu, row, jj);
+        const T* vrow = vpool + (size_t)rj * vd;
+#pragma unroll
+        for (int i = 0; i < PER_LANE; ++i) {
+          const int c = lane + 32 * i;
+          if (c < vd) acc[i] = fmaf(pj, to_f32(vrow[c]), acc[i]);
+        }
+      }
+    } else for (int j0 = first; j0 <= last; j0 += kValueBatch) {
       T v[kValueBatch][PER_LANE];
 #pragma unroll
       for (int u = 0; u < kValueBatch; ++u) {
@@ -191,25 +207,36 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_generic_kernel(AttnArgs 
 }
 
 template <typename T>
+static auto generic_kernel_for(int value_dim) {
+  switch ((value_dim + 31) / 32) {
+    case 1: return attn_generic_kernel<T, 1>;
+    case 2: return attn_generic_kernel<T, 2>;
+    case 3: return attn_generic_kernel<T, 3>;
+    case 4: return attn_generic_kernel<T, 4>;
+    default: return attn_generic_kernel<T, 8>;
+  }
+}
+
+template <typename T>
 static int launch_attn_generic(const AttnArgs& a, cudaStream_t s) {
   const long long items = (long long)a.tokens * a.heads;
   const long long blocks = items;
   SLB_REQUIRE(blocks < (1ll << 31), "attention: too many rows (%lld)", items);
-  const int per_lane = (a.value_dim + 31) / 32;
-  const int threads = kAttnWarps * 32;
-  switch (per_lane) {
-    case 1: launch(attn_generic_kernel<T, 1>, dim3((int)blocks), dim3(threads), 0, s, a); break;
-    case 2: launch(attn_generic_kernel<T, 2>, dim3((int)blocks), dim3(threads), 0, s, a); break;
-    case 3: launch(attn_generic_kernel<T, 3>, dim3((int)blocks), dim3(threads), 0, s, a); break;
-    case 4: launch(attn_generic_kernel<T, 4>, dim3((int)blocks), dim3(threads), 0, s, a); break;
-    default: launch(attn_generic_kernel<T, 8>, dim3((int)blocks), dim3(threads), 0, s, a); break;
-  }
+  launch(generic_kernel_for<T>(a.value_dim), dim3((int)blocks), dim3(kAttnWarps * 32), 0, s, a);
   return check_launch("attention (general kernel)");
 }
 
 }  // namespace slb
 
 using namespace slb;
+
+// Blocks of the kernel for values of this width that an SM of the current device holds at once (prompts rest on it), or 0.
+extern "C" int slb_attention_generic_blocks_per_sm(int value_dim, int dtype) {
+  int blocks = 0;
+  const cudaError_t e = dtype == kF32 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, generic_kernel_for<float>(value_dim), kAttnWarps * 32, 0)
+                                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, generic_kernel_for<__nv_bfloat16>(value_dim), kAttnWarps * 32, 0);
+  return e == cudaSuccess ? blocks : 0;
+}
 
 extern "C" int slb_attention_generic(const void* q, const void* k_pool, const void* v_pool, void* out,
                                      const int* tok_seq, const int* tok_pos, const int* block_table,
