@@ -16,10 +16,10 @@
 // that its unstable sort happens to place first).
 //
 // Cost: a row's eighth is read once into shared memory, and one histogram over values between a lower bound and the row's
-// maximum finds the short list that holds the answer (see quick_list below). 64 rows of 151,936, top-k 50, top-p 0.9: 247 us
-// before (six passes over the row, four of them with 64 KB of histograms to clear and add up), 55 us now. Rows for which
-// that cannot work (longer than the blocks hold, NaN or infinite maxima, more candidates than fit) take the general path:
-// a radix descent over the sort keys, eight bits a pass.
+// maximum finds the short list that holds the answer (the quick path, below). 64 rows of 151,936, top-k 50, top-p 0.9: 247 us
+// before (six passes over the row, four of them with 64 KB of histograms to clear and add up), 55 us now. Calls and rows for
+// which that cannot work (neither top-k nor top-p, top-k beyond the list, rows longer than the blocks hold, NaN or infinite
+// maxima, more candidates than fit) take the general path: a radix descent over the sort keys, eight bits a pass.
 #include <math.h>
 
 #include <cooperative_groups.h>
@@ -33,7 +33,10 @@ namespace cg = cooperative_groups;
 
 namespace slb {
 
-constexpr int kSampleThreads = 512;
+// Threads of a block. While every block has an SM to itself (18 rows) it takes all that fit; with more rows two blocks of half the
+// size share an SM, so that one works while the other stands at a barrier. 8 rows of 151,936 in us, 512 / 1,024 threads: temperature
+// alone 37 / 25, top-k 3,000 100 / 70; 64 rows: 68 / 84, 255 / 310.
+constexpr int kFewRowsThreads = 1024, kManyRowsThreads = 512;
 constexpr double kMassScale = 1099511627776.0;  // 2^40
 
 __device__ __forceinline__ unsigned int sort_key(float v) {
@@ -139,7 +142,7 @@ __global__ void argmax_final_kernel(const float* __restrict__ part_v, const int*
   if (lane == 0) out[r] = bi == 0x7fffffff ? 0 : bi;   // a row of NaNs picks token 0
 }
 
-constexpr int kSampleWarps = kSampleThreads / 32;
+constexpr int kMostWarps = kFewRowsThreads / 32;
 constexpr int kSampleTeam = 8;        // blocks per row: a thread-block cluster, each block takes an eighth of the row
 constexpr int kCandidates = 2048;     // what top-k leaves is kept in shared memory when it is at most this many tokens
 
@@ -151,7 +154,7 @@ struct SampleExchange {
   unsigned long long sum[2];
   float max[2];
   int count[2];
-  unsigned long long seg[kSampleWarps];
+  unsigned long long seg[kMostWarps];
   float low;                               // quick path: the block's share of the lower bound, and whether it must not be taken
   int bad;
   int total;                               // quick path: candidates
@@ -231,13 +234,13 @@ struct Team {
     for (int c = 0; c < size; ++c) t += cluster.map_shared_rank(&sh->x, c)->sum[f];
     return t;
   }
-  // sh->hist := sum over the team of each block's 32 warp histograms
+  // sh->hist := sum over the team of each block's warp histograms
   __device__ void histogram(const unsigned long long* warp_hist) {
     const int f = solo ? 0 : flip();
     for (int b = threadIdx.x; b < 256; b += blockDim.x) {
       unsigned long long t = 0ull;
 #pragma unroll 8
-      for (int w = 0; w < kSampleWarps; ++w) t += warp_hist[w * 256 + b];
+      for (int w = 0; w < (blockDim.x >> 5); ++w) t += warp_hist[w * 256 + b];
       if (solo) sh->hist[b] = t; else sh->x.hist[f][b] = t;
     }
     if (solo) { __syncthreads(); return; }
@@ -292,7 +295,7 @@ struct ListSource {
 // Radix descent over the 32-bit sort keys, 8 bits a level. COUNT: each element weighs 1 (top-k), otherwise its
 // fixed-point mass (top-p). Among the elements with key >= floor_key it finds the key of the element whose
 // inclusion, in descending key order, first makes the accumulated weight reach `target` (>= 1).
-// Every warp counts into a histogram of its own: most keys share their top byte, and thirty-two warps adding to the
+// Every warp counts into a histogram of its own: most keys share their top byte, and all warps adding to the
 // same two or three words would take turns. The warps' histograms are summed afterwards, over the whole team.
 template <bool COUNT, typename SRC>
 __device__ unsigned int radix_threshold(Team& team, const SRC& src, float mx, unsigned int floor_key,
@@ -302,7 +305,7 @@ __device__ unsigned int radix_threshold(Team& team, const SRC& src, float mx, un
   if (threadIdx.x == 0) { sh.prefix = 0u; sh.above = 0ull; }
   for (int level = 0; level < 4; ++level) {
     const int shift = 24 - 8 * level;
-    for (int i = threadIdx.x; i < 256 * kSampleWarps; i += blockDim.x) warp_hist[i] = 0ull;
+    for (int i = threadIdx.x; i < 8 * blockDim.x; i += blockDim.x) warp_hist[i] = 0ull;      // 256 a warp
     __syncthreads();
     const unsigned int prefix = sh.prefix;
     const unsigned int mask = level == 0 ? 0u : (0xffffffffu << (shift + 8));
@@ -397,21 +400,21 @@ __device__ int warp_walk(int n, G get, float mx, unsigned int floor_key, float m
 // base + 128 * c + 4 * lane .. + 3 of its warp's stretch. One histogram of kBins equal steps of value, from a lower bound to the
 // maximum, is added up over the team; the step in which the weight from above reaches the target is known then, and the few
 // tokens at or above it (for top-k), or in it (for top-p without top-k), are all that the exact decision needs.
-constexpr int kHeld = 10;              // float4 per thread
-constexpr int kHeldTokens = kHeld * 4 * kSampleThreads;
+constexpr int kHeldTokens = 20480;     // tokens a block holds
 constexpr int kBins = 1024;
+constexpr float kBanned = -1e30f;      // logits below are no candidates' (bans set the lowest value or minus infinity)
 constexpr int kQuickList = 1024;       // candidates of a row at most
 constexpr int kSmallList = 512;        // up to this many entries are compared each with each
 
 struct Held {
-  float4* mine;            // this thread's first float4; the next ones kSampleThreads apart
+  float4* mine;            // this thread's first float4; the next ones a block's threads apart
   int begin, end;          // its warp's stretch of tokens (row numbers), whole chunks of 128 but for the row's last
   int lane;
   template <typename F> __device__ __forceinline__ void each(F f) const {
 #pragma unroll 2
     for (int c = 0; begin + 128 * c < end; ++c) {
       const int t = begin + 128 * c + 4 * lane;
-      const float4 v = mine[c * kSampleThreads];
+      const float4 v = mine[c * blockDim.x];
       if (t < end) f(t, v.x);
       if (t + 1 < end) f(t + 1, v.y);
       if (t + 2 < end) f(t + 2, v.z);
@@ -425,10 +428,10 @@ __device__ __forceinline__ int bin_of(float v, float mx, float per) { return min
 
 // The step at which the weight of the team's histogram, added up from step 0, first reaches `target`, or -1; `above` = the
 // weight of the steps before it. LIMBS 1: counts; 3: masses in parts of 16, 16 and 9 bits (shared memory adds 32-bit words).
-template <int LIMBS>
+template <int LIMBS, int THREADS>
 __device__ int find_bin(Team& team, const unsigned int* hist, unsigned long long target, unsigned long long& above) {
   SampleShared& sh = *team.sh;
-  constexpr int kPer = kBins / kSampleThreads;
+  constexpr int kPer = kBins / THREADS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned long long h[kPer], mine = 0ull;
 #pragma unroll
@@ -506,6 +509,17 @@ __device__ __forceinline__ void keep_candidate(SampleShared& sh, int* tokens, fl
   if (at < kQuickList) { tokens[at] = t; values[at] = v; }
 }
 
+// How many of the n tokens (16-byte aligned) lie before t.
+__device__ __forceinline__ int tokens_before(const int* tokens, int n, int t) {
+  int before = 0, j = 0;
+  for (; j + 4 <= n; j += 4) {
+    const int4 v = *reinterpret_cast<const int4*>(tokens + j);
+    before += (v.x < t ? 1 : 0) + (v.y < t ? 1 : 0) + (v.z < t ? 1 : 0) + (v.w < t ? 1 : 0);
+  }
+  for (; j < n; ++j) before += tokens[j] < t ? 1 : 0;
+  return before;
+}
+
 // The blocks' lists together in block 0 (at all_token / all_value), if they fit: returns their length, or -1. After it the other
 // blocks' lists are free. Once per launch.
 __device__ int gather_lists(Team& team, int* tokens, float* values, int* all_token, float* all_value, int rank, int most) {
@@ -530,10 +544,12 @@ __device__ int gather_lists(Team& team, int* tokens, float* values, int* all_tok
   return n;
 }
 
-__global__ void __cluster_dims__(kSampleTeam, 1, 1) __launch_bounds__(kSampleThreads, 2)
+template <int THREADS>
+__global__ void __cluster_dims__(kSampleTeam, 1, 1) __launch_bounds__(THREADS, 1024 / THREADS)
 sample_kernel(const float* __restrict__ logits, long long ld, int limit, float temperature, int top_k, float top_p,
               float min_p, const float* __restrict__ uniform, int* __restrict__ out) {
   pdl_enter();
+  constexpr int kWarps = THREADS / 32;
   __shared__ SampleShared sh;
   __shared__ int quick_token[kQuickList];
   __shared__ float quick_value[kQuickList];
@@ -561,14 +577,16 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
   int n_listed = 0;
 
   const bool count_first = top_k > 0 && top_k < limit;
-  const int chunks = (raw.n + 128 * kSampleWarps - 1) / (128 * kSampleWarps);
+  const int chunks = (raw.n + 128 * kWarps - 1) / (128 * kWarps);
   Held mine{held + threadIdx.x, part_begin + warp * chunks * 128, min(part_end, part_begin + (warp + 1) * chunks * 128), lane};
-  bool quick = per_block <= kHeldTokens && (count_first || top_p < 1.0f);      // the same for all blocks of a row
+  bool quick = per_block <= kHeldTokens && (count_first ? top_k <= kQuickList : top_p < 1.0f);      // the same for all blocks of a row
   if (quick) {
-    // the one read of the row; the largest value, a lower bound, and whether anything is no number
+    // the one read of the row; the largest value, bounds from below, and whether anything is no number. Banned tokens (minus
+    // infinity, or the lowest value) count for no bound.
     const bool aligned = (reinterpret_cast<uintptr_t>(row + part_begin) & 15) == 0;
-    float most = -INFINITY;
+    float most = -INFINITY, least = INFINITY;
     bool bad = false;
+    auto allowed = [](float v) { return v < kBanned ? INFINITY : v; };
 #pragma unroll 5
     for (int c = 0; mine.begin + 128 * c < mine.end; ++c) {
       const int t = mine.begin + 128 * c + 4 * lane;
@@ -583,13 +601,14 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
       }
       bad = bad || v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w;
       most = fmaxf(most, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
-      mine.mine[c * kSampleThreads] = v;
+      if (!count_first) least = fminf(least, fminf(fminf(allowed(v.x), allowed(v.y)), fminf(allowed(v.z), allowed(v.w))));
+      mine.mine[c * THREADS] = v;
     }
     // At least as many values as there are warps (threads) with a maximum of their own reach the smallest of those maxima.
     const float warp_most = warp_max(most);
     const int warps_with = (limit + chunks * 128 - 1) / max(1, chunks * 128);      // warps of the row that hold tokens, about
     float low = top_k <= warps_with / 2 ? warp_most : most;
-    if (mine.begin + 4 * lane >= mine.end) low = INFINITY;
+    low = allowed(count_first ? low : least);      // (threads without tokens have neither)
     const float low_block = -block_max(-low, sh.red);
     const float most_block = block_max(most, sh.red);
     const int any_bad = __syncthreads_or(bad ? 1 : 0);
@@ -615,7 +634,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
         mine.each([&](int, float x) { if (x >= row_low) atomicAdd(&bins[bin_of(x, row_most, per)], 1u); });
         team.cluster.sync();
         unsigned long long above;
-        const int bin = find_bin<1>(team, bins, (unsigned long long)top_k, above);
+        const int bin = find_bin<1, THREADS>(team, bins, (unsigned long long)top_k, above);
         quick = bin >= 0 && bin < kBins - 2;
         if (quick) {
           mine.each([&](int t, float x) {
@@ -635,9 +654,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
             floor_key = sort_key(__uint_as_float(b) / temperature);
             // in token order (the draw walks it), divided by the temperature
             for (int i = threadIdx.x; i < n; i += blockDim.x) {
-              const int t = all_token[i];
-              int pos = 0;
-              for (int j = 0; j < n; ++j) pos += all_token[j] < t ? 1 : 0;
+              const int t = all_token[i], pos = tokens_before(all_token, n, t);
               cand_token[pos] = t;
               cand_value[pos] = all_value[i] / temperature;
             }
@@ -656,10 +673,12 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
         }
       }
     } else if (quick) {
-      // top-p over the whole row: quotients, of which those more than 16 below the largest weigh next to nothing
+      // top-p over the whole row: quotients, of which those more than 16 below the largest weigh next to nothing; where all lie closer
+      // together the steps are narrower (a step must be wider than a quotient's last place)
       mx = row_most / temperature;
-      const float per = (kBins - 0.5f) / 16.0f, lowest = mx - 16.0f;
-      quick = size / temperature < 1e4f;      // (a step must be wider than a quotient's last place)
+      quick = size / temperature < 1e4f;
+      const float span = fminf(16.0f, fmaxf(fmaxf((row_most - row_low) / temperature, 1.1e-3f * (size / temperature)), 1e-6f));
+      const float per = (kBins - 0.5f) / span, lowest = mx - span;
       if (quick) {
         unsigned long long part = 0ull;
         mine.each([&](int, float x) {
@@ -677,7 +696,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
         unsigned long long target = (unsigned long long)ceil((double)top_p * (double)total), above;
         if (target < 1ull) target = 1ull;
         if (target > total) target = total;
-        const int bin = find_bin<3>(team, bins, target, above);
+        const int bin = find_bin<3, THREADS>(team, bins, target, above);
         quick = bin >= 0 && bin < kBins - 1;
         if (quick) {
           mine.each([&](int t, float x) {
@@ -709,7 +728,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
 
   if (!quick) {
     floor_key = 0u;
-    cand_token = reinterpret_cast<int*>(warp_hist + kSampleWarps * 256);
+    cand_token = reinterpret_cast<int*>(warp_hist + kWarps * 256);
     cand_value = reinterpret_cast<float*>(cand_token + kCandidates);
   // division by a positive temperature keeps the order, so the largest quotient is the quotient of the largest value
   mx = -INFINITY;
@@ -790,9 +809,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
       team.solo = true;
       // order by token: each entry counts the entries with a smaller token
       for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int t = all_token[i];
-        int pos = 0;
-        for (int j = 0; j < n; ++j) pos += all_token[j] < t ? 1 : 0;
+        const int t = all_token[i], pos = tokens_before(all_token, n, t);
         cand_token[pos] = t;
         cand_value[pos] = all_value[i];
       }
@@ -834,7 +851,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
   }
   // the whole row: every warp of every block owns a contiguous stretch of tokens and sums it (coalesced loads), each
   // block finds the stretch the draw falls into, and the warp that owns it walks it
-  const int stretch = ((raw.n + kSampleWarps - 1) / kSampleWarps + 31) & ~31;
+  const int stretch = ((raw.n + kWarps - 1) / kWarps + 31) & ~31;
   const int begin = min(raw.n, warp * stretch), end = min(raw.n, begin + stretch);
   {
     unsigned long long mine = 0ull;
@@ -848,7 +865,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
   __syncthreads();
   // the blocks' totals go round; every block then knows the draw's target and which block it falls into
   unsigned long long block_total = 0ull;
-  for (int w = 0; w < kSampleWarps; ++w) block_total += sh.x.seg[w];
+  for (int w = 0; w < kWarps; ++w) block_total += sh.x.seg[w];
   const int f = team.flip();
   if (threadIdx.x == 0) sh.x.sum[f] = block_total;
   team.cluster.sync();
@@ -866,7 +883,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
     // this block's stretch: find the warp, which then walks its tokens
     unsigned long long acc = before;
     int which = -1;
-    for (int w = 0; w < kSampleWarps; ++w) {
+    for (int w = 0; w < kWarps; ++w) {
       const unsigned long long t = sh.x.seg[w];
       if (t > 0ull && target < acc + t) { which = w; break; }
       acc += t;
@@ -956,6 +973,9 @@ extern "C" int slb_argmax_static(const float* logits, long long ld, int rows, in
 
 extern "C" int slb_argmax_static_max_rows() { return kStaticArgmaxRows; }
 
+// Threads of a block for so many rows: all an SM takes while every block of a row's eight has an SM to itself.
+extern "C" int slb_sample_threads(int rows) { return (long long)rows * kSampleTeam <= sm_count() ? kFewRowsThreads : kManyRowsThreads; }
+
 extern "C" int slb_sample(const float* logits, long long ld, int rows, int limit, float temperature, int top_k,
                           float top_p, float min_p, const float* uniform, int* out, void* stream) {
   SLB_REQUIRE(rows >= 0 && limit > 0 && ld >= limit, "sample: rows=%d limit=%d ld=%lld", rows, limit, ld);
@@ -966,11 +986,13 @@ extern "C" int slb_sample(const float* logits, long long ld, int rows, int limit
   if (rows == 0) return 0;
   // the quick path's row and histogram; the general path's warp histograms and candidates lie in the same place
   constexpr size_t hist_bytes = kHeldTokens * sizeof(float) + 3 * kBins * sizeof(unsigned int);
-  static_assert(kSampleWarps * 256 * sizeof(unsigned long long) + 2 * kCandidates * sizeof(int) <= kHeldTokens * sizeof(float), "the general path's place");
-  static std::atomic<unsigned long long> allowed;
-  const cudaError_t e = allow_shared((const void*)sample_kernel, (int)hist_bytes, allowed);
+  static_assert(kMostWarps * 256 * sizeof(unsigned long long) + 2 * kCandidates * sizeof(int) <= kHeldTokens * sizeof(float), "the general path's place");
+  const bool few = slb_sample_threads(rows) == kFewRowsThreads;
+  const auto kernel = few ? sample_kernel<kFewRowsThreads> : sample_kernel<kManyRowsThreads>;
+  static std::atomic<unsigned long long> allowed[2];
+  const cudaError_t e = allow_shared((const void*)kernel, (int)hist_bytes, allowed[few]);
   if (e != cudaSuccess) return fail(2, "sample: cannot reserve %d bytes of shared memory: %s", (int)hist_bytes, cudaGetErrorString(e));
-  launch(sample_kernel, dim3(rows * kSampleTeam), dim3(kSampleThreads), hist_bytes, (cudaStream_t)stream, logits, ld, limit, temperature, top_k, top_p,
+  launch(kernel, dim3(rows * kSampleTeam), dim3(few ? kFewRowsThreads : kManyRowsThreads), hist_bytes, (cudaStream_t)stream, logits, ld, limit, temperature, top_k, top_p,
          min_p, uniform, out);
   return check_launch("sample");
 }

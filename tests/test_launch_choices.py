@@ -62,3 +62,9 @@ def test_timeline_groups_block_records_into_launches():
     assert (first["last_mark2"], first["first_leave"], first["last_leave"]) == (1600, 1700, 1800)
     assert norm["last_mark2"] == 0 and norm["last_leave"] == 2500
     assert (second["first_enter"], second["last_enter"], second["last_leave"]) == (2000, 2600, 3600)
+
+
+def test_sampler_blocks_fill_their_sm():
+    """Few rows: a block an SM, as large as it can be; more rows: two blocks of half the size."""
+    threads = ops.lib().dll.slb_sample_threads
+    assert threads(1) == threads(18) == 1024 and threads(19) == threads(64) == 512
