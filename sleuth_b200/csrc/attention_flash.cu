@@ -344,11 +344,8 @@ __device__ __forceinline__ void put_row(unsigned char* tile, int row, int lane, 
   }
 }
 
-// W: warps per block, 16 keys of a step each; a step is a page (four warps) or half of one (two). Half pages take half of the
-// shared memory, so four blocks fit an SM, and a batch of many sequences (more blocks than 3 an SM) runs in fewer rounds
-// with every block's fixed costs hidden by three others; with fewer blocks a step of four warps is the faster one (48 sequences of
-// 200 to 900 keys: 26 us against 35). 16 / 8 heads of 128, us with pages / half pages: 64 sequences of 32 to 192 keys 14.7 / 11.4,
-// 32 to 512 22.8 / 22.3, 600 to 1,000 43.8 / 40.2, 2,048 90.8 / 80.8; 128 of 32 to 512 41.8 / 39.2; 256 of 10 to 300 57.9 / 46.8.
+// W: warps per block, 16 keys of a step each; a step is a page (four warps) or half of one (two, heads of 128). Half pages take half of
+// the shared memory, so four blocks fit an SM instead of two, every block's fixed costs hidden by three others (decode_warps).
 // S: page buffers per block. Three (two pages on their way while one is worked on) is the default; with two, three
 // blocks fit an SM instead of two, which lets two slices per (sequence, kv head) run at once where one slice each
 // would leave half the GPU idle (see decode_stages).
@@ -694,6 +691,16 @@ static int decode_stages(long long blocks) {
   return (blocks > 2ll * sms && blocks <= 3ll * sms) ? 2 : 3;
 }
 
+// Warps per block. Heads of 64 fit an SM four times with whole pages already (16 / 8 heads, fused, us with pages / half pages: 64
+// sequences of 32 to 512 keys 12.1 / 18.1, 200 to 900 19.6 / 27.3). Heads of 128 take half pages where the blocks are more than 3 an SM
+// and do not just exceed the four that fit: between 4 and 6 an SM the second round of four is nearly empty and three rounds of two
+// are shorter. us: 48 sequences of 200 to 900 keys 26 / 35; 64 of 32 to 192 12.3 / 10.2, of 700 39.3 / 34.0; 80 of 300 to 900 43.8 / 48.8, of
+// 700 53.4 / 62.3; 104 of 700 57.4 / 64.8; 128 of 32 to 192 23.5 / 20.5, of 300 to 900 65.7 / 67.3; 200 of 100 to 600 67.7 / 62.7; 256 46.4 / 37.5
+// (32 to 192), 120.9 / 116.4 (300 to 900).
+static int decode_warps(int head_dim, long long blocks, long long sms) {
+  return head_dim == 128 && blocks > 3 * sms && !(blocks > 4 * sms && blocks <= 6 * sms) ? 2 : 4;
+}
+
 template <int HD, int S, int W>
 static int launch_decode_staged(const FlashArgs& a, int n_seqs, cudaStream_t s) {
   const int G = a.heads / a.kv_heads;
@@ -716,13 +723,17 @@ template <int HD>
 static int launch_decode(const FlashArgs& a, int n_seqs, cudaStream_t s) {
   const int row_tiles = (a.heads / a.kv_heads + 15) / 16;
   const long long blocks = (long long)a.splits * row_tiles * a.kv_heads * n_seqs;
-  if (blocks > 3ll * sm_count()) return launch_decode_staged<HD, 3, 2>(a, n_seqs, s);
+  if constexpr (HD == 128)
+    if (decode_warps(HD, blocks, sm_count()) == 2) return launch_decode_staged<HD, 3, 2>(a, n_seqs, s);
   return decode_stages(blocks) == 2 ? launch_decode_staged<HD, 2, 4>(a, n_seqs, s) : launch_decode_staged<HD, 3, 4>(a, n_seqs, s);
 }
 
 }  // namespace slb
 
 using namespace slb;
+
+// Warps a block of the single-token kernel has (4: whole pages a step, 2: half pages), on a device of `sms` SMs.
+extern "C" int slb_attention_decode_warps(int head_dim, long long blocks, int sms) { return decode_warps(head_dim, blocks, sms); }
 SLB_TIMELINE_SETTER(attention_flash)
 
 // 1 when the tensor-core kernels take this shape, else 0 (the general kernel then serves it).

@@ -1,6 +1,8 @@
 """Host-side choices that the kernels' launches rest on, checked without a GPU: how many slices the single-token
 attention cuts a sequence into, and when a product normalises its own input."""
 
+import ctypes
+
 import pytest
 
 from sleuth_b200.kernels import ops
@@ -62,6 +64,13 @@ def test_timeline_groups_block_records_into_launches():
     assert (first["last_mark2"], first["first_leave"], first["last_leave"]) == (1600, 1700, 1800)
     assert norm["last_mark2"] == 0 and norm["last_leave"] == 2500
     assert (second["first_enter"], second["last_enter"], second["last_leave"]) == (2000, 2600, 3600)
+
+
+def test_single_token_attention_takes_half_pages_where_they_were_faster():
+    """Heads of 128 from three blocks an SM on, but for the loads that just exceed the four blocks that fit; heads of 64 never."""
+    warps = lambda hd, blocks: ops.lib().dll.slb_attention_decode_warps(hd, ctypes.c_longlong(blocks), SMS)
+    assert [warps(128, b) for b in (8, 444, 445, 512, 592, 593, 640, 888, 889, 1024, 2048)] == [4, 4, 2, 2, 2, 4, 4, 4, 2, 2, 2]
+    assert all(warps(64, b) == 4 for b in (8, 512, 640, 1024, 2048))
 
 
 def test_sampler_blocks_fill_their_sm():
