@@ -678,10 +678,13 @@ __device__ __forceinline__ int take_rows(unsigned long long& with, int g, int& p
   return n;
 }
 
-// grid (pairs, groups of 8 columns): act[pair, j] = f(gate_e[j] . h[token]) * (up_e[j] . h[token]), for the pairs that share the expert of
-// pair blockIdx.x, if it is the first of them. The block's warps take an eighth of the width each.
+// grid (pairs, groups of 64 / PARTS columns): act[pair, j] = f(gate_e[j] . h[token]) * (up_e[j] . h[token]), for the pairs that share the
+// expert of pair blockIdx.x, if it is the first of them. A warp takes one of PARTS parts of the width for 8 columns: with narrow matrices
+// fewer parts, so that a warp has eight loads to ask for and the blocks that all wait for the choices first are not many rounds.
+template <int PARTS>
 __global__ void __launch_bounds__(256, 3) moe_few_gate_up_mma_kernel(MoeFewArgs a) {
   pdl_enter();
+  constexpr int kGroups = 8 / PARTS;
   __shared__ float red[8][2][16][8 + 1];
   __shared__ int row_pair[16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -689,13 +692,13 @@ __global__ void __launch_bounds__(256, 3) moe_few_gate_up_mma_kernel(MoeFewArgs 
   const int e = __shfl_sync(0xffffffffu, blockIdx.x < 32 ? c0 : c1, blockIdx.x & 31);
   unsigned long long with = pairs_with(c0, c1, e);
   if (e >= a.E || __ffsll(with) - 1 != (int)blockIdx.x) return;      // an identity expert; another pair leads (the whole block agrees)
-  const int feat = blockIdx.y * 8 + g;
+  const int part = warp % PARTS, feat = (blockIdx.y * kGroups + warp / PARTS) * 8 + g;
   const __nv_bfloat16* wrow[2];
 #pragma unroll
   for (int f = 0; f < 2; ++f)
     wrow[f] = feat < a.ff ? a.w_gu + ((size_t)e * 2 * a.ff + (size_t)f * a.ff + feat) * a.dim + 8 * t : nullptr;
-  const int kb_total = a.dim / 32, per = (kb_total + 7) / 8;
-  const int kb_begin = warp * per, kb_end = min(kb_total, kb_begin + per);
+  const int kb_total = a.dim / 32, per = (kb_total + PARTS - 1) / PARTS;
+  const int kb_begin = part * per, kb_end = min(kb_total, kb_begin + per);
   const uint4 zero = make_uint4(0, 0, 0, 0);
   constexpr int U = 4;
   while (with) {
@@ -731,11 +734,12 @@ __global__ void __launch_bounds__(256, 3) moe_few_gate_up_mma_kernel(MoeFewArgs 
     }
     if (warp == 0 && t == 0) { row_pair[g] = p0; row_pair[g + 8] = p1; }
     __syncthreads();
-    const int r = threadIdx.x >> 3, c = threadIdx.x & 7, j = blockIdx.y * 8 + c;
-    if (r < n && j < a.ff) {
+    for (int i = threadIdx.x; i < 128 * kGroups; i += 256) {
+      const int r = i >> 3 & 15, c = i & 7, w0 = (i >> 7) * PARTS, j = (blockIdx.y * kGroups + (i >> 7)) * 8 + c;
+      if (r >= n || j >= a.ff) continue;
       float gv = 0.f, uv = 0.f;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) { gv += red[k][0][r][c]; uv += red[k][1][r][c]; }
+      for (int k = 0; k < PARTS; ++k) { gv += red[w0 + k][0][r][c]; uv += red[w0 + k][1][r][c]; }
       a.act[(size_t)row_pair[r] * a.ff + j] = __float2bfloat16_rn(gated(a.gate, gv, uv));
     }
     if (with) __syncthreads();
@@ -823,6 +827,9 @@ __global__ void __launch_bounds__(256, 2) moe_few_down_mma_kernel(MoeFewArgs a) 
     *dst = a.store ? total : *dst + total;
   }
 }
+
+// Matrices below 512 x 512 are read faster than the pairs of an expert are found (256 x 512: 11 us either product for itself, 15 together).
+static bool few_pairs_on_tensor_cores(int dim, int ff) { return dim % 32 == 0 && ff % 32 == 0 && (long long)dim * ff >= 1ll << 18; }
 
 // What the kernels that sum a token's choices need to know of identity experts: the choices, the number of experts that
 // have matrices and the tokens' input rows (all unused when `choice` is null).
@@ -1050,13 +1057,18 @@ extern "C" int slb_moe_experts(const void* h, const void* w_gu, const void* w_do
     if (dtype == kF32) {
       launch(moe_few_gate_up_kernel<float>, f1, block, 0, s, (const float*)h, (const float*)w_gu, choice, (float*)act, top, dim, ff, E, gate);
       launch(moe_few_down_kernel<float>, f2, block, 0, s, (const float*)h, (const float*)act, (const float*)w_down, choice, weight, x, extra, top, dim, ff, E, store);
-    } else if (dim % 32 == 0 && ff % 32 == 0) {
+    } else if (few_pairs_on_tensor_cores(dim, ff)) {
       const MoeFewArgs a{(const __nv_bfloat16*)h, (const __nv_bfloat16*)w_gu, (const __nv_bfloat16*)w_down, choice, weight, (__nv_bfloat16*)act, x, extra,
                          (int)pairs, top, dim, ff, E, store, gate};
-      launch(moe_few_gate_up_mma_kernel, f1, block, 0, s, a);
-      // parts of the experts' width: enough units for the eight warps where few experts are met
-      if (pairs <= 8) launch(moe_few_down_mma_kernel<4>, dim3((dim + 7) / 8), block, 0, s, a);
-      else launch(moe_few_down_mma_kernel<2>, dim3((dim + 7) / 8), block, 0, s, a);
+      // The parts depend on the matrices alone, so that a token's bits do not depend on the tokens beside it.
+      const auto gate_up = [&](auto kernel, int parts) { launch(kernel, dim3((unsigned)pairs, (ff + 64 / parts - 1) / (64 / parts)), block, 0, s, a); };
+      if (dim >= 2048) gate_up(moe_few_gate_up_mma_kernel<8>, 8);
+      else if (dim >= 1024) gate_up(moe_few_gate_up_mma_kernel<4>, 4);
+      else gate_up(moe_few_gate_up_mma_kernel<2>, 2);
+      const dim3 f3((dim + 7) / 8);
+      if (ff <= 1024) launch(moe_few_down_mma_kernel<1>, f3, block, 0, s, a);
+      else if (ff <= 2048) launch(moe_few_down_mma_kernel<2>, f3, block, 0, s, a);
+      else launch(moe_few_down_mma_kernel<4>, f3, block, 0, s, a);
     } else {
       launch(moe_few_gate_up_kernel<__nv_bfloat16>, f1, block, 0, s, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w_gu, choice,
              (__nv_bfloat16*)act, top, dim, ff, E, gate);

@@ -44,3 +44,33 @@ def test_few_pairs(tokens, top, E, dim, ff, identity, store, further):
     got = x.cpu().double()
     assert ((got - want).abs() <= 2.0 ** -8 * size + 1e-5 * (1 + want.abs())).all()
     assert float((got - want).norm() / want.norm()) < 1e-3
+
+
+# The same where the tensor-core kernels run (matrices of 512 x 512 values and more): two, four and eight parts of the width with an
+# uneven last one, one, two and four parts of the experts' width, column groups that are not full, more than 16 and 32 rows an expert.
+@pytest.mark.parametrize("tokens,top,E,dim,ff", [(32, 2, 3, 544, 512), (64, 1, 2, 512, 544), (21, 3, 7, 1056, 288), (5, 2, 6, 2080, 160), (8, 8, 40, 512, 1056),
+                                                 (4, 3, 5, 160, 2080), (16, 4, 20, 1024, 2112), (1, 8, 64, 4096, 512), (40, 1, 1, 992, 1088)])
+@pytest.mark.parametrize("identity,store,further", [(0, False, False), (2, False, True), (1, True, False)])
+def test_few_pairs_on_the_tensor_cores(tokens, top, E, dim, ff, identity, store, further):
+    test_few_pairs(tokens, top, E, dim, ff, identity, store, further)
+
+
+@pytest.mark.parametrize("top,E,dim,ff", [(6, 64, 2048, 1408), (4, 16, 1024, 768), (2, 8, 512, 3584), (2, 4, 256, 128)])
+def test_a_tokens_bits_do_not_depend_on_the_tokens_beside_it(top, E, dim, ff):
+    g = torch.Generator().manual_seed(dim + ff)
+    n = 64 // top
+    d = lambda a: a.to(DEV).contiguous()
+    h = d(torch.randn(n, dim, generator=g).bfloat16())
+    w_gu, w_down = d(torch.randn(E, 2 * ff, dim, generator=g).div(dim ** 0.5).bfloat16()), d(torch.randn(E, dim, ff, generator=g).div(ff ** 0.5).bfloat16())
+    choice, weight = d(torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(n)]).int()), d(torch.rand(n, top, generator=g))
+
+    def run(a, b):
+        x, pairs = torch.zeros(b - a, dim, device=DEV), (b - a) * top
+        act, y = torch.empty(pairs, ff, device=DEV, dtype=torch.bfloat16), torch.empty(pairs, dim, device=DEV)
+        ints = torch.zeros(max(pairs, E), dtype=torch.int32, device=DEV)
+        ops.moe_experts(h[a:b], w_gu, w_down, ints[:E], ints[:pairs], weight[a:b].reshape(-1), act, y, x, top, "silu", None, choice[a:b].reshape(-1), ints[:pairs])
+        return x
+
+    together = run(0, n)
+    for a, b in ((0, 1), (1, 3), (n - 1, n), (n // 2, n)):
+        assert torch.equal(run(a, b), together[a:b])
