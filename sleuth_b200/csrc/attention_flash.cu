@@ -72,13 +72,13 @@ template <int HD> __device__ __forceinline__ uint32_t swz(int row, int col) {
   return (uint32_t)(row * (HD * 2) + ((((col >> 3) ^ (row & 7))) << 4));
 }
 
-// Cooperative load of ROWS rows of a page (contiguous in global memory) into a swizzled tile. Rows from
+// Cooperative load of one 64-row page tile (contiguous in global memory) into a swizzled tile. Rows from
 // `valid_rows` on lie beyond the sequence's length: a reused page holds another sequence's leftovers there, and
 // although their weights are exactly zero, 0 * inf would still poison the sum, so they are filled with zeros.
-template <int HD, int THREADS, int ROWS = 64>
+template <int HD, int THREADS>
 __device__ __forceinline__ void load_page(unsigned char* smem_base, uint32_t dst_off, const __nv_bfloat16* src,
                                           int valid_rows, int tid) {
-  constexpr int CHUNKS = ROWS * HD / 8;
+  constexpr int CHUNKS = 64 * HD / 8;
   const uint32_t dst = smem_u32(smem_base) + dst_off;
 #pragma unroll
   for (int i = tid; i < CHUNKS; i += THREADS) {
@@ -344,13 +344,11 @@ __device__ __forceinline__ void put_row(unsigned char* tile, int row, int lane, 
   }
 }
 
-// W: warps per block, 16 keys of a step each; a step is a page (four warps) or half of one (two, heads of 128). Half pages take half of
-// the shared memory, so four blocks fit an SM instead of two, every block's fixed costs hidden by three others (decode_warps).
 // S: page buffers per block. Three (two pages on their way while one is worked on) is the default; with two, three
 // blocks fit an SM instead of two, which lets two slices per (sequence, kv head) run at once where one slice each
 // would leave half the GPU idle (see decode_stages).
-template <int HD, int S, int W>
-__global__ void __launch_bounds__(W * 32) attn_decode_kernel(FlashArgs a) {
+template <int HD, int S>
+__global__ void __launch_bounds__(kFlashThreads) attn_decode_kernel(FlashArgs a) {
   // Fused form: the keys and values of earlier tokens, the block table and the lengths were all written before the
   // kernel that precedes this one began, so pages are requested before the wait for that kernel (which produces
   // only the raw projection of the new token). That holds when this kernel itself appends the token's key and value,
@@ -363,8 +361,7 @@ __global__ void __launch_bounds__(W * 32) attn_decode_kernel(FlashArgs a) {
   pdl_launch_dependents();
   if (a.pages_after_wait) pdl_wait();
   extern __shared__ __align__(128) unsigned char smem[];
-  constexpr int T = W * 32, KEYS = W * 16, PER = 64 / KEYS;      // threads; keys a step; steps a page
-  constexpr int TILE = KEYS * HD * 2;
+  constexpr int TILE = 64 * HD * 2;
   constexpr int EPL = HD / 32;
   const uint32_t sK = smem_u32(smem), sV = sK + S * TILE;
   const uint32_t sQ = sV + S * TILE;          // [16][HD]
@@ -390,10 +387,10 @@ __global__ void __launch_bounds__(W * 32) attn_decode_kernel(FlashArgs a) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) slope_r[h] = a.slopes != nullptr && g + 8 * h < rows ? a.slopes[head0 + g + 8 * h] * kLog2e : 0.0f;
   // this slice's page numbers, fetched once so that the page loop does not wait for the table
-  __shared__ int my_pages[T];
+  __shared__ int my_pages[kFlashThreads];
   __shared__ int ticket;
   if (my_lo + tid <= my_hi) my_pages[tid] = table[my_lo + tid];
-  auto page_of = [&](int page) { return page - my_lo < T ? my_pages[page - my_lo] : table[page]; };
+  auto page_of = [&](int page) { return page - my_lo < kFlashThreads ? my_pages[page - my_lo] : table[page]; };
   __syncthreads();
 
   float o[HD / 8][4];
@@ -401,20 +398,18 @@ __global__ void __launch_bounds__(W * 32) attn_decode_kernel(FlashArgs a) {
   for (int i = 0; i < HD / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
   float m_r[2] = {-INFINITY, -INFINITY}, l_r[2] = {0.0f, 0.0f};
 
-  // the slice's steps: pages, or the halves of pages that hold visible keys
-  const int step_lo = max(my_lo * PER, key_lo / KEYS), step_hi = min(my_hi * PER + PER - 1, pos / KEYS);
-  auto fetch = [&](int step) {      // one commit group per step, empty beyond the slice
-    if (step <= step_hi) {
-      const int st = (step - step_lo) % S;
-      const size_t base = (((size_t)page_of(step / PER) * a.kv_heads + kh) * 64 + step % PER * KEYS) * HD;
-      load_page<HD, T, KEYS>(smem, st * TILE, a.k_pool + base, pos + 1 - step * KEYS, tid);
-      load_page<HD, T, KEYS>(smem, (S + st) * TILE, a.v_pool + base, pos + 1 - step * KEYS, tid);
+  auto fetch = [&](int page) {      // one commit group per page, empty beyond the slice
+    if (page <= my_hi) {
+      const int st = (page - my_lo) % S;
+      const size_t base = ((size_t)page_of(page) * a.kv_heads + kh) * 64 * HD;
+      load_page<HD, kFlashThreads>(smem, st * TILE, a.k_pool + base, pos + 1 - page * 64, tid);
+      load_page<HD, kFlashThreads>(smem, (S + st) * TILE, a.v_pool + base, pos + 1 - page * 64, tid);
     }
     cp_async_commit();
   };
   if (my_lo <= my_hi) {
 #pragma unroll
-    for (int d = 0; d < S - 1; ++d) fetch(step_lo + d);
+    for (int d = 0; d < S - 1; ++d) fetch(my_lo + d);
   }
   // The fused form's gains and rotation factors for this lane: weights and tables, asked for before the wait.
   float q_gain[EPL], k_gain[EPL], cos_l[EPL], sin_l[EPL];
@@ -439,7 +434,7 @@ __global__ void __launch_bounds__(W * 32) attn_decode_kernel(FlashArgs a) {
     if (fused) {
       const int rows_per_token = a.heads + 2 * a.qkv_kv_heads;
       const __nv_bfloat16* raw = a.qkv + (size_t)tok * rows_per_token * HD;
-      for (int row = warp; row < 16; row += W) {
+      for (int row = warp; row < 16; row += kFlashThreads / 32) {
         float v[EPL];
         if (row < rows) {
           const int head = head0 + row;
@@ -469,7 +464,7 @@ __global__ void __launch_bounds__(W * 32) attn_decode_kernel(FlashArgs a) {
         }
       }
     } else {
-      for (int i = tid; i < 16 * (HD / 8); i += T) {
+      for (int i = tid; i < 16 * (HD / 8); i += kFlashThreads) {
         const int row = i / (HD / 8), ch = i % (HD / 8);
         uint4 val = make_uint4(0, 0, 0, 0);
         if (row < rows) val = *reinterpret_cast<const uint4*>(a.q + ((size_t)tok * a.heads + head0 + row) * HD + ch * 8);
@@ -478,23 +473,23 @@ __global__ void __launch_bounds__(W * 32) attn_decode_kernel(FlashArgs a) {
     }
     uint32_t qf[HD / 16][4];
 
-    for (int step = step_lo; step <= step_hi; ++step) {
-      const int stage = (step - step_lo) % S;
-      fetch(step + S - 1);       // into the buffer that the step before this one has left
-      cp_async_wait<S - 1>();    // all but the newest groups: this step's keys and values have landed
+    for (int page = my_lo; page <= my_hi; ++page) {
+      const int stage = (page - my_lo) % S;
+      fetch(page + S - 1);       // into the buffer that the page before this one has left
+      cp_async_wait<S - 1>();    // all but the newest groups: this page has landed
       __syncthreads();
-      if (owns_last && step == pos / KEYS) {     // put the new token's key and value where the cache copy has a stale row
-        if (warp < 2) put_row<HD>(smem + ((warp == 0 ? 0 : S) + stage) * TILE, pos % KEYS, lane, new_kv);
+      if (owns_last && page == page_hi) {     // put the new token's key and value where the cache copy has a stale row
+        if (warp < 2) put_row<HD>(smem + ((warp == 0 ? 0 : S) + stage) * TILE, pos % 64, lane, new_kv);
         __syncthreads();
       }
-      if (step == step_lo) {
+      if (page == my_lo) {
 #pragma unroll
         for (int kb = 0; kb < HD / 16; ++kb) {
           const int row = lane & 15, col = kb * 16 + ((lane >> 4) << 3);
           ldmatrix_x4(qf[kb], sQ + swz<HD>(row, col));
         }
       }
-      const int key0 = step * KEYS + warp * 16;     // this warp's 16 keys of the step
+      const int key0 = page * 64 + warp * 16;     // this warp's 16 keys of the page
       if (key0 <= pos && key0 + 15 >= key_lo) {
         const uint32_t kS = sK + stage * TILE, vS = sV + stage * TILE;
         float s[2][4];
@@ -569,15 +564,15 @@ __global__ void __launch_bounds__(W * 32) attn_decode_kernel(FlashArgs a) {
   if (tid == 0)
     prefetch_share(a.next, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), gridDim.x * gridDim.y * gridDim.z);
 
-  // merge the warps (each saw different keys) through shared memory
+  // merge the four warps (each saw different keys) through shared memory
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     l_r[h] += __shfl_xor_sync(0xffffffffu, l_r[h], 1);
     l_r[h] += __shfl_xor_sync(0xffffffffu, l_r[h], 2);
   }
-  float* mo = reinterpret_cast<float*>(smem);            // [W warps][16 rows][HD]
-  float* mm = mo + W * 16 * HD;                          // [W][16]
-  float* ml = mm + W * 16;                               // [W][16]
+  float* mo = reinterpret_cast<float*>(smem);            // [4 warps][16 rows][HD]
+  float* mm = mo + 4 * 16 * HD;                          // [4][16]
+  float* ml = mm + 4 * 16;                               // [4][16]
   __syncthreads();
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -589,15 +584,15 @@ __global__ void __launch_bounds__(W * 32) attn_decode_kernel(FlashArgs a) {
       *reinterpret_cast<float2*>(mo + (warp * 16 + row) * HD + i * 8 + 2 * t4) = make_float2(o[i][2 * h], o[i][2 * h + 1]);
   }
   __syncthreads();
-  for (int idx = tid; idx < rows * HD; idx += T) {
+  for (int idx = tid; idx < rows * HD; idx += kFlashThreads) {
     const int row = idx / HD, d = idx % HD;
     float m = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < W; ++w) m = fmaxf(m, mm[w * 16 + row]);
+    for (int w = 0; w < 4; ++w) m = fmaxf(m, mm[w * 16 + row]);
     const float m_use = m == -INFINITY ? 0.0f : m;
     float l = 0.0f, acc = 0.0f;
 #pragma unroll
-    for (int w = 0; w < W; ++w) {
+    for (int w = 0; w < 4; ++w) {
       const float f = exp2f(mm[w * 16 + row] - m_use);
       l += ml[w * 16 + row] * f;
       acc += mo[(w * 16 + row) * HD + d] * f;
@@ -632,7 +627,7 @@ __global__ void __launch_bounds__(W * 32) attn_decode_kernel(FlashArgs a) {
   }
   __syncthreads();
   if (ticket != a.splits - 1) return;
-  for (int idx = tid; idx < rows * HD; idx += T) {
+  for (int idx = tid; idx < rows * HD; idx += kFlashThreads) {
     const int row = idx / HD, d = idx % HD;
     const int head = head0 + row;
     const size_t base = ((size_t)seq * a.heads + head) * a.splits;
@@ -684,38 +679,32 @@ static int launch_prefill(const FlashArgs& a, int n_seqs, int max_count, cudaStr
   return check_launch("attention (prefill)");
 }
 
-// Two page buffers instead of three when that makes all blocks resident at once: with three buffers two blocks fit
-// an SM (296 in all), with two buffers three (444).
-static int decode_stages(long long blocks) {
-  const int sms = sm_count();
-  return (blocks > 2ll * sms && blocks <= 3ll * sms) ? 2 : 3;
+// Two page buffers instead of three when that makes all blocks resident at once: at heads of 128 two blocks fit an SM with three
+// buffers (296 in all), three with two (444). The same again from the third round of two on, where rounds of three are fewer; up to
+// there both take two rounds, and long sequences are faster with a page more on its way. 16 / 8 heads of 128, fused, us with three / two
+// buffers: 64 sequences (512 blocks) of 100 to 600 keys 27.6 / 25.6, of 700 39.3 / 46.0, of 2,048 92 / 119; 80 of 700 54.5 / 49.1; 128 of 32 to 512
+// 38.4 / 33.5, 300 to 900 67.8 / 60.9; 256 of 10 to 300 53.5 / 43.2, of 700 127.7 / 118.8. Heads of 64 fit four times with three.
+// (Steps of half a page by two warps, four blocks an SM, were faster below 600 blocks on short sequences, 64 of 32 to 192 keys 12.0 / 10.0, slower
+// than either above; their sums are of other keys, and the error against 64 bits was a thousandth larger.)
+static int decode_stages(int head_dim, long long blocks, long long sms) {
+  return (blocks > 2 * sms && blocks <= 3 * sms) || (head_dim == 128 && blocks > 4 * sms) ? 2 : 3;
 }
 
-// Warps per block. Heads of 64 fit an SM four times with whole pages already (16 / 8 heads, fused, us with pages / half pages: 64
-// sequences of 32 to 512 keys 12.1 / 18.1, 200 to 900 19.6 / 27.3). Heads of 128 take half pages where the blocks are more than 3 an SM
-// and do not just exceed the four that fit: between 4 and 6 an SM the second round of four is nearly empty and three rounds of two
-// are shorter. us: 48 sequences of 200 to 900 keys 26 / 35; 64 of 32 to 192 12.3 / 10.2, of 700 39.3 / 34.0; 80 of 300 to 900 43.8 / 48.8, of
-// 700 53.4 / 62.3; 104 of 700 57.4 / 64.8; 128 of 32 to 192 23.5 / 20.5, of 300 to 900 65.7 / 67.3; 200 of 100 to 600 67.7 / 62.7; 256 46.4 / 37.5
-// (32 to 192), 120.9 / 116.4 (300 to 900).
-static int decode_warps(int head_dim, long long blocks, long long sms) {
-  return head_dim == 128 && blocks > 3 * sms && !(blocks > 4 * sms && blocks <= 6 * sms) ? 2 : 4;
-}
-
-template <int HD, int S, int W>
+template <int HD, int S>
 static int launch_decode_staged(const FlashArgs& a, int n_seqs, cudaStream_t s) {
   const int G = a.heads / a.kv_heads;
   const int row_tiles = (G + 15) / 16;
-  const int tiles_bytes = 2 * S * 16 * W * HD * 2 + 16 * HD * 2;
-  const int merge_bytes = (W * 16 * HD + 2 * W * 16) * 4;
+  const int tiles_bytes = 2 * S * 64 * HD * 2 + 16 * HD * 2;
+  const int merge_bytes = (4 * 16 * HD + 2 * 4 * 16) * 4;
   const int smem = tiles_bytes > merge_bytes ? tiles_bytes : merge_bytes;
   static std::atomic<unsigned long long> allowed;
-  const cudaError_t e = allow_shared((const void*)attn_decode_kernel<HD, S, W>, smem, allowed);
+  const cudaError_t e = allow_shared((const void*)attn_decode_kernel<HD, S>, smem, allowed);
   if (e != cudaSuccess) return fail(2, "attention (decode): cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
   dim3 grid(a.splits * row_tiles, a.kv_heads, n_seqs);
   if (a.qkv != nullptr)      // the fused form asks for its pages before it waits for the kernel in front of it
-    launch_prefetching(attn_decode_kernel<HD, S, W>, dim3(grid), dim3(W * 32), smem, s, a);
+    launch_prefetching(attn_decode_kernel<HD, S>, dim3(grid), dim3(kFlashThreads), smem, s, a);
   else
-    launch(attn_decode_kernel<HD, S, W>, dim3(grid), dim3(W * 32), smem, s, a);
+    launch(attn_decode_kernel<HD, S>, dim3(grid), dim3(kFlashThreads), smem, s, a);
   return check_launch("attention (decode)");
 }
 
@@ -723,17 +712,15 @@ template <int HD>
 static int launch_decode(const FlashArgs& a, int n_seqs, cudaStream_t s) {
   const int row_tiles = (a.heads / a.kv_heads + 15) / 16;
   const long long blocks = (long long)a.splits * row_tiles * a.kv_heads * n_seqs;
-  if constexpr (HD == 128)
-    if (decode_warps(HD, blocks, sm_count()) == 2) return launch_decode_staged<HD, 3, 2>(a, n_seqs, s);
-  return decode_stages(blocks) == 2 ? launch_decode_staged<HD, 2, 4>(a, n_seqs, s) : launch_decode_staged<HD, 3, 4>(a, n_seqs, s);
+  return decode_stages(HD, blocks, sm_count()) == 2 ? launch_decode_staged<HD, 2>(a, n_seqs, s) : launch_decode_staged<HD, 3>(a, n_seqs, s);
 }
 
 }  // namespace slb
 
 using namespace slb;
 
-// Warps a block of the single-token kernel has (4: whole pages a step, 2: half pages), on a device of `sms` SMs.
-extern "C" int slb_attention_decode_warps(int head_dim, long long blocks, int sms) { return decode_warps(head_dim, blocks, sms); }
+// Page buffers of the single-token kernel's blocks, on a device of `sms` SMs.
+extern "C" int slb_attention_decode_stages(int head_dim, long long blocks, int sms) { return decode_stages(head_dim, blocks, sms); }
 SLB_TIMELINE_SETTER(attention_flash)
 
 // 1 when the tensor-core kernels take this shape, else 0 (the general kernel then serves it).

@@ -1,7 +1,6 @@
-"""Single-token attention of batches that fill the GPU several times over (csrc/attention_flash.cu, attn_decode_kernel with two
-warps a block and steps of half a page), post-processed queries and the fused form, against float64: positions around the edges of
-half pages and pages and several hundred keys (the ring of buffers goes round many times), windows and chunks that begin inside a
-page's first or second half."""
+"""Single-token attention of batches that fill the GPU several times over (csrc/attention_flash.cu, attn_decode_kernel with three
+page buffers and with two), post-processed queries and the fused form, against float64: positions around the edges of a warp's keys
+and of pages and several hundred keys (the ring of buffers goes round many times), windows and chunks that begin anywhere in a page."""
 
 import math
 
@@ -39,8 +38,8 @@ d = lambda a: None if a is None else torch.as_tensor(a).to(DEV)
 ints = lambda a: d(np.asarray(a, dtype=np.int32))
 
 
-# 64 x 8, 75 x 6 and 460 x 1 blocks of one slice; (40 heads, 2 kv heads): two tiles of query rows, 2 x 2 x 120 blocks
-@pytest.mark.parametrize("n,heads,kv_heads", [(64, 16, 8), (75, 24, 6), (460, 3, 1), (120, 40, 2)])
+# 64 x 8, 75 x 6 and 460 x 1 blocks of one slice: three page buffers; (160 sequences of 40 heads, 2 kv heads): two tiles of query rows, 2 x 2 x 160 blocks, two
+@pytest.mark.parametrize("n,heads,kv_heads", [(64, 16, 8), (75, 24, 6), (460, 3, 1), (160, 40, 2)])
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("window", [0, 45, 100, 77, 200, -48, -96])
 def test_post_processed_queries(n, heads, kv_heads, hd, window):
@@ -55,8 +54,9 @@ def test_post_processed_queries(n, heads, kv_heads, hd, window):
 
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("window", [0, 100, 77, -96])
-def test_fused_form(hd, window):
-    n, heads, kv_heads, eps = 64, 16, 8, 1e-5
+@pytest.mark.parametrize("n", [64, 80])      # three page buffers; two at heads of 128
+def test_fused_form(n, hd, window):
+    heads, kv_heads, eps = 16, 8, 1e-5
     gen = torch.Generator().manual_seed(hd + window)
     pasts, scale, rows = batch(n), 1.0 / math.sqrt(hd), heads + 2 * kv_heads
     k_pool, v_pool, table, ks, vs = make_cache([p + 1 for p in pasts], kv_heads, hd, BF, gen)
@@ -87,3 +87,24 @@ def test_fused_form(hd, window):
         torch.testing.assert_close(got[page, :, row].float(), want[page, :, row].float(), rtol=2e-2, atol=2e-2)
         got[page, :, row] = want[page, :, row]
         assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("window", [0, 77, -96])
+def test_a_sequences_bits_do_not_depend_on_the_batch(hd, window):
+    """Any number of sequences beside it, three page buffers or two: the same bits for a sequence."""
+    n, heads, kv_heads = 80, 16, 8
+    gen = torch.Generator().manual_seed(hd + window)
+    pasts, scale = batch(n), 1.0 / math.sqrt(hd)
+    k_pool, v_pool, table, _, _ = make_cache([p + 1 for p in pasts], kv_heads, hd, BF, gen)
+    k_pool, v_pool, table, q = d(k_pool), d(v_pool), d(table), d(torch.randn(n, heads, hd, generator=gen).to(BF))
+
+    def run(a, b):
+        out = torch.full((b - a, heads * hd), float("nan"), dtype=BF, device=DEV)
+        ops().attention_decode(q[a:b].contiguous(), k_pool, v_pool, out, ints(range(b - a + 1)), ints(pasts[a:b]), table[a:b].contiguous(), heads, kv_heads, hd,
+                               window, scale, 1, None)
+        return out
+
+    together = run(0, n)
+    for a, b in ((0, 16), (16, 32), (20, 60), (15, 79), (63, 64)):
+        assert torch.equal(run(a, b), together[a:b])

@@ -66,11 +66,11 @@ def test_timeline_groups_block_records_into_launches():
     assert (second["first_enter"], second["last_enter"], second["last_leave"]) == (2000, 2600, 3600)
 
 
-def test_single_token_attention_takes_half_pages_where_they_were_faster():
-    """Heads of 128 from three blocks an SM on, but for the loads that just exceed the four blocks that fit; heads of 64 never."""
-    warps = lambda hd, blocks: ops.lib().dll.slb_attention_decode_warps(hd, ctypes.c_longlong(blocks), SMS)
-    assert [warps(128, b) for b in (8, 444, 445, 512, 592, 593, 640, 888, 889, 1024, 2048)] == [4, 4, 2, 2, 2, 4, 4, 4, 2, 2, 2]
-    assert all(warps(64, b) == 4 for b in (8, 512, 640, 1024, 2048))
+def test_single_token_attention_has_two_page_buffers_where_they_were_faster():
+    """Where all blocks are resident with two and not with three, and at heads of 128 from the third round on."""
+    stages = lambda hd, blocks: ops.lib().dll.slb_attention_decode_stages(hd, ctypes.c_longlong(blocks), SMS)
+    assert [stages(128, b) for b in (8, 296, 297, 444, 445, 512, 592, 593, 640, 1024, 2048)] == [3, 3, 2, 2, 3, 3, 3, 2, 2, 2, 2]
+    assert [stages(64, b) for b in (8, 296, 297, 444, 445, 512, 593, 1024, 2048)] == [3, 3, 2, 2, 3, 3, 3, 3, 3]
 
 
 def test_sampler_blocks_fill_their_sm():
