@@ -318,15 +318,23 @@ def attention_f32_supported(heads: int, kv_heads: int, head_dim: int, value_dim:
     return dtype == torch.float32 and head_dim in (64, 128) and value_dim == head_dim and heads // kv_heads <= 16
 
 
-def attention_f32_scratch_floats(n_seqs: int, heads: int, head_dim: int, table_stride: int) -> int:
-    """Scratch of a step of single tokens: a chunk (two pages) leaves its weighted values, maximum and sum there."""
-    return n_seqs * heads * ((table_stride + 1) // 2) * (head_dim + 2)
+def attention_f32_scratch_floats(n_seqs: int, heads: int, head_dim: int, table_stride: int, kv_heads: int = 0, tokens: int = 0,
+                                 max_count: int = 1, max_keys: int = 0) -> int:
+    """Scratch with which ``attention_f32`` spreads a sequence's keys over several blocks: a chunk (two pages) leaves its
+    weighted values, maximum and sum there. 0: the step needs none. Without ``kv_heads``: the most that single tokens need."""
+    if not kv_heads:
+        return n_seqs * heads * ((table_stride + 1) // 2) * (head_dim + 2)
+    fn = lib().dll.slb_attention_f32_scratch
+    fn.argtypes = [ctypes.c_int] * 8
+    fn.restype = ctypes.c_longlong
+    return fn(n_seqs, tokens or n_seqs, max_count, heads, kv_heads, head_dim, table_stride, max_keys)
 
 
 def attention_f32(q, k_pool, v_pool, out, seq_start, past, counts, block_table, max_count: int, heads: int, kv_heads: int,
-                  head_dim: int, window: int, scale: float, scratch, stream=None, sinks=None) -> None:
-    """Causal attention in true float32. Results do not depend on how a sequence was cut into steps. ``scratch`` (for
-    ``max_count`` 1): ``attention_f32_scratch_floats`` floats."""
+                  head_dim: int, window: int, scale: float, scratch, stream=None, sinks=None, max_keys: int = 0) -> None:
+    """Causal attention in true float32. Results do not depend on how a sequence was cut into steps, nor on ``scratch``:
+    ``attention_f32_scratch_floats`` floats or more, which steps of several tokens a sequence can do without. ``max_keys``: a
+    promise that no sequence has more keys after this step (0: as many as its table holds)."""
     _cuda(q, k_pool, v_pool, out, seq_start, past, counts, block_table, sinks, scratch)
     T, n = q.shape[0], block_table.shape[0]
     _need(q.shape == (T, heads, head_dim) and out.shape == (T, heads * head_dim), "attention_f32: shapes disagree")
@@ -337,7 +345,7 @@ def attention_f32(q, k_pool, v_pool, out, seq_start, past, counts, block_table, 
     _need(sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == heads), "attention_f32: sinks are float32, one per head")
     _need(seq_start.numel() >= n and past.numel() >= n and counts.numel() >= n, "attention_f32: per-sequence tables")
     lib().call("slb_attention_f32", _p(q), _p(k_pool), _p(v_pool), _p(out), _p(seq_start), _p(past), _p(counts), _p(block_table),
-               block_table.shape[1], n, int(max_count), heads, kv_heads, head_dim, int(window), float(scale), _p(sinks),
+               block_table.shape[1], n, T, int(max_count), int(max_keys), heads, kv_heads, head_dim, int(window), float(scale), _p(sinks),
                _p(scratch), scratch.numel() if scratch is not None else 0, stream if stream is not None else current_stream())
 
 

@@ -171,10 +171,12 @@ class GQAAttention(Part):
         hd, vd = self.key_run, self.value_run
         flash = ops.flash_supported(hd, self.ctx.dtype) and vd == hd
         if ops.attention_f32_supported(s.heads, s.kv_heads, hd, vd, self.ctx.dtype):
-            scratch = (ws.take((ops.attention_f32_scratch_floats(b.n, s.heads, hd, table.shape[1]),), torch.float32)
-                       if b.max_count == 1 else None)
+            # (a recording of a step of many tokens serves steps that start at position 0, or only others; one of single tokens both)
+            keys = b.max_count if b.fresh and b.max_count > 1 else 0
+            floats = ops.attention_f32_scratch_floats(b.n, s.heads, hd, table.shape[1], s.kv_heads, q.shape[0], b.max_count, keys)
+            scratch = ws.take((floats,), torch.float32) if floats else None
             ops.attention_f32(q, view.k_pool, view.v_pool, y, b.seq_start, b.past, b.counts, table, b.max_count, s.heads,
-                              s.kv_heads, hd, view.window, self.scale, scratch, b.stream, sinks=self.sinks)
+                              s.kv_heads, hd, view.window, self.scale, scratch, b.stream, sinks=self.sinks, max_keys=keys)
         elif not flash:
             ops.attention(q, view.k_pool, view.v_pool, y, b.tok_seq, b.tok_pos, table, s.heads, s.kv_heads,
                           hd, view.window, self.scale, b.stream, sinks=self.sinks, value_dim=vd)

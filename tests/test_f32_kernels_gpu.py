@@ -131,3 +131,69 @@ def test_gemm_f32_second_operand_written_by_the_kernel_in_front(M):
         assert torch.equal(straight, wait)
         ops().gemm_f32(x, w, straight, static_weight=True)       # (written long ago by now)
         assert torch.equal(straight, wait)
+
+
+def step_f32(q, k_pool, v_pool, table, pasts, counts, heads, kv_heads, hd, window, sinks=None, scratch=True, fresh=False):
+    """One step as parts/attention.py runs it (``scratch=False``: without scratch, so that no sequence's keys are cut)."""
+    o = ops()
+    d = lambda a: torch.as_tensor(np.asarray(a, dtype=np.int32)).to(DEV)
+    keys = max(counts) if fresh else 0
+    floats = o.attention_f32_scratch_floats(len(counts), heads, hd, table.shape[1], kv_heads, q.shape[0], max(counts), keys)
+    out = torch.full((q.shape[0], heads * hd), float("nan"), device=DEV)
+    buf = torch.full((floats + 64,), float("nan"), device=DEV) if scratch else None
+    o.attention_f32(q, k_pool, v_pool, out, d(np.concatenate([[0], np.cumsum(counts)])), d(pasts), d(counts), table, max(counts), heads, kv_heads, hd,
+                    window, 1.0 / math.sqrt(hd), buf, sinks=sinks, max_keys=keys)
+    assert buf is None or torch.isnan(buf[floats:]).all()
+    return out, floats
+
+
+# Portions on a past: up to 16 rows a group (heads of the group x tokens; 2, 4, 8 and 16 rows), then tiles of 64 rows, cut along
+# the keys and not; windows and chunks of positions that begin inside a page and leave some rows of a portion without a key of it.
+@pytest.mark.parametrize("heads,kv_heads,hd", [(4, 2, 128), (5, 1, 64), (8, 8, 64), (16, 1, 128), (3, 3, 128), (12, 2, 64)])
+@pytest.mark.parametrize("window,sink", [(0, False), (0, True), (50, False), (200, True), (-96, False), (3, False)])
+def test_attention_f32_portions(heads, kv_heads, hd, window, sink):
+    pasts, most = [0, 70, 640, 129, 1000, 63, 126, 253], 40
+    gen = torch.Generator().manual_seed(heads + hd + window)
+    k_pool, v_pool, table, ks, vs = make_cache([p + most for p in pasts], kv_heads, hd, torch.float32, gen)
+    k_pool, v_pool, table = k_pool.to(DEV), v_pool.to(DEV), table.to(DEV)
+    dense_q = torch.randn(len(pasts), most, heads, hd, generator=gen)
+    sinks = torch.randn(heads, generator=gen).to(DEV) if sink else None
+    alone = torch.stack([step_f32(dense_q[:, t].contiguous().to(DEV), k_pool, v_pool, table, [p + t for p in pasts], [1] * len(pasts),
+                                  heads, kv_heads, hd, window, sinks)[0] for t in range(most)], 1)      # single tokens
+    for i, p in enumerate(pasts):
+        for t in (0, 1, 2, 39):
+            pos = p + t
+            lo = max(0, pos - window + 1) if window > 0 else (pos // -window * -window if window < 0 else 0)
+            kk, vv = (a[i][lo:pos + 1].double().repeat_interleave(heads // kv_heads, 1) for a in (ks, vs))
+            s = torch.einsum("hd,jhd->hj", dense_q[i, t].double(), kk) / math.sqrt(hd)
+            s = torch.cat([s, sinks.cpu().double()[:, None]], 1) if sink else s
+            want = torch.einsum("hj,jhd->hd", torch.softmax(s, 1)[:, :kk.shape[0]], vv)
+            torch.testing.assert_close(alone[i, t].cpu().double().view(heads, hd), want, rtol=1e-5, atol=5e-6)
+    cut = 0
+    for counts in ([2] * 8, [3] * 8, [1, 4, 2, 3, 1, 4, 2, 1], [8, 1, 5, 7, 8, 2, 3, 6], [16] * 8, [9, 16, 1, 12, 3, 15, 2, 5], [17, 1, 40, 33, 20, 2, 3, 31]):
+        for some in (list(range(8)), [4], [2, 4]):
+            own = [counts[i] for i in some]
+            q = torch.cat([dense_q[i, :counts[i]] for i in some]).contiguous().to(DEV)
+            want = torch.cat([alone[i, :counts[i]] for i in some])
+            args = (q, k_pool, v_pool, table[some].contiguous(), [pasts[i] for i in some], own, heads, kv_heads, hd, window, sinks)
+            got, floats = step_f32(*args)
+            cut += floats > 0
+            assert torch.equal(got, want)
+            assert max(own) == 1 or torch.equal(step_f32(*args, scratch=False)[0], want)
+    assert cut
+    got = step_f32(dense_q[0].contiguous().to(DEV), k_pool, v_pool, table[:1].contiguous(), [0], [most], heads, kv_heads, hd, window, sinks, fresh=True)[0]
+    assert torch.equal(got, alone[0])
+
+
+def test_attention_f32_many_sequences_need_no_scratch():
+    """A batch that fills the GPU with a block a (sequence, kv head): the same bits as each sequence by itself."""
+    heads, kv_heads, hd, n = 16, 8, 64, 80
+    gen = torch.Generator().manual_seed(5)
+    pasts = [(37 * i) % 500 for i in range(n)]
+    k_pool, v_pool, table, _, _ = make_cache([p + 1 for p in pasts], kv_heads, hd, torch.float32, gen)
+    k_pool, v_pool, table, q = k_pool.to(DEV), v_pool.to(DEV), table.to(DEV), torch.randn(n, heads, hd, generator=gen).to(DEV)
+    got, floats = step_f32(q, k_pool, v_pool, table, pasts, [1] * n, heads, kv_heads, hd, 0)
+    assert floats == 0
+    for i in range(0, n, 7):
+        one, floats = step_f32(q[i:i + 1].contiguous(), k_pool, v_pool, table[i:i + 1].contiguous(), pasts[i:i + 1], [1], heads, kv_heads, hd, 0)
+        assert floats > 0 and torch.equal(one[0], got[i])

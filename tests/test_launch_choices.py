@@ -77,3 +77,22 @@ def test_sampler_blocks_fill_their_sm():
     """Few rows: a block an SM, as large as it can be; more rows: two blocks of half the size."""
     threads = ops.lib().dll.slb_sample_threads
     assert threads(1) == threads(18) == 1024 and threads(19) == threads(64) == 512
+
+
+def test_float32_attention_scratch():
+    """Scratch of the 32-bit attention: none where blocks have a sequence to themselves, never more than 256 MB, never more than the
+    form that every single-token step could have needed, and the same for every replay of a step's shape."""
+    f = ops.attention_f32_scratch_floats
+    wide = 640                                     # 40,960 keys
+    assert f(256, 16, 128, wide, 8) == f(64, 16, 64, wide, 8) == f(64, 32, 64, wide, 8, 128, 2) == 0      # blocks enough without cutting
+    assert f(591, 16, 128, wide, 1) == 0           # would be 1.5 GB
+    for n in (1, 2, 8, 30, 64, 100, 300):
+        for heads, kv in ((16, 8), (16, 1), (32, 8), (8, 8)):
+            for stride in (1, 2, 3, 64, wide):
+                assert 0 <= f(n, heads, 128, stride, kv) <= min(f(n, heads, 128, stride), 1 << 26)
+                for count in (1, 2, 5, 20, 64, 300):
+                    assert 0 <= f(n, heads, 128, stride, kv, n * count, count) <= 1 << 26
+    assert f(1, 16, 128, 64, 8) == 16 * 32 * 130
+    assert f(1, 16, 128, 64, 8, 20, 20) == 20 * 16 * 32 * 130        # a second turn: 8 tiles, cut along the keys
+    assert f(1, 16, 128, 64, 8, 100, 100, 100) == 0                  # a prompt of one chunk
+    assert f(8, 16, 128, 64, 8, 3200, 400) == 0                      # tiles enough
