@@ -19,6 +19,14 @@ __host__ __device__ inline int segment_length(int K) {
   return len < 128 ? 128 : len;
 }
 
+// Tiles that a block of the streaming kernel takes side by side, with `room` blocks for `tiles` tiles: no more than its warps have
+// segments for, and none while blocks are to be had, where joining the tiles' sums takes as long as forming them (K below 64) or
+// where three and more segments keep the block busy (8 rows x 12,288 x 384: 14.3 us, two side by side 16.4).
+static int groups_of(int K, int tiles, int room) {
+  const int segments = (K + segment_length(K) - 1) / segment_length(K), most = kMaxSegments / segments, want = (tiles + room - 1) / room;
+  return K < 64 || segments > 2 ? 1 : want < most ? want : most;
+}
+
 struct GemmF32Args {
   const float* A;
   const float* W;
@@ -33,7 +41,8 @@ struct GemmF32Args {
 // can deliver (a lane's 16-byte read costs its full 16 bytes of 128 a cycle, broadcast or not). So warp w of a block owns segment
 // w of K, and streams its part of the block's weight rows (NT features), with the token rows' values for the same k, through a
 // ring of its own: CH k values a stage, D stages, 16-byte asynchronous copies, no barrier between warps until a tile's sums are
-// joined. A block goes from tile to tile (tile + gridDim.x) with the ring running on, so its copies never drain. Where the
+// joined. With one or two segments (K up to 256) and more tiles than blocks a block takes several tiles side by side (SIDE), group
+// g of its warps tile base + g (16 rows x 32,768 x 96: 22.5 us one at a time, 16.4 side by side). A block goes from tile to tile with the ring running on, so its copies never drain. Where the
 // caller says that no kernel writes W, the first stages' weights are asked for before the wait for the kernel in front. LM lanes along the rows and 32 / LM along the features
 // make each lane's block R x CN as square as the tile allows. 0.6B sizes, 8 rows, us before (one chain per output over all of K, slices of
 // 32 k values behind barriers) / now: q/k/v 25.1 / 5.9, o 50.2 / 7.6, gate and up 34.9 / 9.1, down 74.5 / 10.8, head 479 / 145; 64 rows:
@@ -50,9 +59,9 @@ struct RowsShape {
   static constexpr int kBlocksPerSm = kSmem <= 113 * 1024 ? 2 : 1;
 };
 
-template <int MP, int NT, int CH, int D, bool VEC>
+template <int MP, int NT, int CH, int D, bool VEC, bool SIDE>
 __global__ void __launch_bounds__(256, (RowsShape<MP, NT, CH, D, VEC>::kBlocksPerSm))
-gemm_f32_rows_kernel(GemmF32Args a, int seg, int tiles) {
+gemm_f32_rows_kernel(GemmF32Args a, int seg, int tiles, int groups) {
   using S = RowsShape<MP, NT, CH, D, VEC>;
   extern __shared__ __align__(16) float smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -60,8 +69,9 @@ gemm_f32_rows_kernel(GemmF32Args a, int seg, int tiles) {
   float* ring = smem + warp * (D * S::kStage);
   float* join = smem + kMaxSegments * D * S::kStage;
   const int m0 = blockIdx.y * MP, rows = min(MP, a.M - m0);
-  const int k_begin = warp * seg, k_len = max(0, min(seg, a.K - k_begin));
-  const int chunks = (k_len + CH - 1) / CH, segments = (a.K + seg - 1) / seg;
+  const int segments = (a.K + seg - 1) / seg, group = SIDE ? warp / segments : 0, stride = SIDE ? gridDim.x * groups : gridDim.x;
+  const int k_begin = (SIDE ? warp % segments : warp) * seg, k_len = SIDE && group >= groups ? 0 : max(0, min(seg, a.K - k_begin));
+  const int chunks = (k_len + CH - 1) / CH;
 
   // A copy brings kCopy k values of one row; a warp's copy instruction kRowsPer rows (or 1 / kTurns of one). Lane: row lr, k value lk.
   constexpr int kCopy = VEC ? 4 : 1, kPerRow = CH / kCopy;
@@ -83,7 +93,7 @@ gemm_f32_rows_kernel(GemmF32Args a, int seg, int tiles) {
     }
   };
   // the stage after the last one asked for: its tile and its chunk
-  int ask_tile = blockIdx.x, ask_chunk = 0, ask_slot = 0;
+  int ask_tile = SIDE ? blockIdx.x * groups + group : blockIdx.x, ask_chunk = 0, ask_slot = 0;
   auto ask_weights = [&]() {
     const int n0 = ask_tile * NT;
     copy_rows(ring + ask_slot * S::kStage, a.W + (size_t)(n0 + lr) * a.ldw + k_begin + lk, a.ldw, a.N - n0, NT, ask_chunk * CH);
@@ -92,7 +102,7 @@ gemm_f32_rows_kernel(GemmF32Args a, int seg, int tiles) {
     copy_rows(ring + slot * S::kStage + NT * S::kRow, a_lane, a.lda, rows, MP, chunk * CH);
   };
   auto advance = [&]() {
-    if (++ask_chunk == chunks) { ask_chunk = 0; ask_tile += gridDim.x; }
+    if (++ask_chunk == chunks) { ask_chunk = 0; ask_tile += stride; }
     if (++ask_slot == D) ask_slot = 0;
   };
 
@@ -115,9 +125,9 @@ gemm_f32_rows_kernel(GemmF32Args a, int seg, int tiles) {
 
   constexpr int kOut = (MP * NT + 255) / 256;
   int slot = 0, buffer = 0;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const int n0 = tile * NT;
-    float old[kOut];
+  for (int base = SIDE ? blockIdx.x * groups : blockIdx.x; base < tiles; base += stride) {
+    const int n0 = base * NT;
+    float old[kOut];      // (of the first tile; the others' are read when they are needed)
 #pragma unroll
     for (int i = 0; i < kOut; ++i) {
       const int idx = tid + 256 * i, r = idx / NT, n = n0 + idx % NT;
@@ -186,6 +196,16 @@ gemm_f32_rows_kernel(GemmF32Args a, int seg, int tiles) {
       if (a.bias) v += a.bias[n];
       a.C[(size_t)(m0 + r) * a.ldc + n] = a.accumulate ? old[i] + v : v;
     }
+    for (int idx = MP * NT + tid; SIDE && idx < groups * (MP * NT); idx += 256) {
+      const int g = idx / (MP * NT), e = idx % (MP * NT), r = e / NT, n = n0 + g * NT + e % NT;
+      if (r >= rows || n >= a.N) continue;
+      const float* p = join + (buffer * kMaxSegments + g * segments) * (MP * NT) + e;
+      float v = p[0];
+      for (int s = 1; s < segments; ++s) v += p[s * (MP * NT)];
+      if (a.bias) v += a.bias[n];
+      float* c = a.C + (size_t)(m0 + r) * a.ldc + n;
+      *c = a.accumulate ? *c + v : v;
+    }
     if (S::kJoinBuffers == 2) buffer ^= 1;      // two buffers: the next tile's barrier stands between these reads and the next writes
     else __syncthreads();
   }
@@ -197,14 +217,14 @@ gemm_f32_rows_kernel(GemmF32Args a, int seg, int tiles) {
 // enough. What bounds it is the FMA pipe and, level with it, what shared memory delivers (a k value is RT + 8 floats read per thread
 // for 8 * RT FMAs). Operands go through registers into shared memory k-major, kTileK k values at a time, two buffers: a warp's
 // reads are then float4 of four rows or features; the FMAs go in packed pairs of neighbouring features. The sums of finished
-// segments wait in shared memory, each thread its own. 3,000 rows x 6,144 x 1,024: 784 us, 48 TFLOP/s, as without packing and
+// segments wait in shared memory, each thread its own (SINGLE: K is one segment, and they stay in registers). 3,000 rows x 6,144 x 1,024: 784 us, 48 TFLOP/s, as without packing and
 // segments before; measured and left: tiles of 64 x 128 with 8 x 16 outputs a thread and transposing 4-byte copies (856 us: a
 // quarter less to read from shared memory, but two warps a scheduler do not cover its latency), row-major operands with pairs
 // along k (910 us).
 constexpr int kTileK = 16, kTileN = 128, kTileWRow = kTileN + 4;
 constexpr int tile_smem(int rt) { return (2 * kTileK * (16 * rt + 4 + kTileWRow) + 256 * rt * 8) * 4; }
 
-template <int RT, bool VEC>
+template <int RT, bool VEC, bool SINGLE>
 __global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(GemmF32Args a, int seg) {
   extern __shared__ __align__(16) float smem[];
   constexpr int BM = 16 * RT, kARow = BM + 4, kBuffer = kTileK * (kARow + kTileWRow);
@@ -257,8 +277,9 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(GemmF32Args a, in
   for (int i = 0; i < RT; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+  if (!SINGLE)
 #pragma unroll
-  for (int e = 0; e < 2 * RT; ++e) totals[e * 256] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int e = 0; e < 2 * RT; ++e) totals[e * 256] = make_float4(0.f, 0.f, 0.f, 0.f);
   put(0);
   __syncthreads();
 
@@ -295,7 +316,7 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(GemmF32Args a, in
       for (int k = 0; k < kn; ++k) one(k);
     }
     left -= kTileK;
-    if (left == 0 || !more) {      // a segment is done (segments are whole multiples of 64)
+    if (!SINGLE && (left == 0 || !more)) {      // a segment is done (segments are whole multiples of 64)
       left = seg;
 #pragma unroll
       for (int i = 0; i < RT; ++i)
@@ -322,7 +343,8 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(GemmF32Args a, in
     if (gm >= a.M) continue;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const float4 t = totals[(2 * i + j) * 256];
+      const float4 t = SINGLE ? make_float4(low_half(acc[i][2 * j]), high_half(acc[i][2 * j]), low_half(acc[i][2 * j + 1]), high_half(acc[i][2 * j + 1]))
+                              : totals[(2 * i + j) * 256];
       const float tv[4] = {t.x, t.y, t.z, t.w};
       float* c = a.C + (size_t)gm * a.ldc + n0 + 4 * tx + 64 * j;
 #pragma unroll
@@ -337,46 +359,74 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(GemmF32Args a, in
   }
 }
 
-template <int MP, int NT, int CH, int D, bool VEC>
-static int launch_rows(const GemmF32Args& a, cudaStream_t s) {
+template <int MP, int NT, int CH, int D, bool VEC, bool SIDE>
+static int launch_rows_form(const GemmF32Args& a, int tiles, int row_tiles, int room, int groups, cudaStream_t s) {
   using S = RowsShape<MP, NT, CH, D, VEC>;
   static_assert(S::kSmem <= 227 * 1024, "the ring must fit shared memory");
-  const auto kernel = gemm_f32_rows_kernel<MP, NT, CH, D, VEC>;
+  const auto kernel = gemm_f32_rows_kernel<MP, NT, CH, D, VEC, SIDE>;
   static std::atomic<unsigned long long> allowed;
   const cudaError_t e = allow_shared((const void*)kernel, S::kSmem, allowed);
   if (e != cudaSuccess) return fail(2, "gemm_f32: cannot reserve %d bytes of shared memory: %s", S::kSmem, cudaGetErrorString(e));
+  const int shares = (tiles + groups - 1) / groups;
+  launch_with(a.early ? pdl_mode() != 0 : pdl_mode() == 1, kernel, dim3(shares < room ? shares : room, row_tiles), dim3(256), S::kSmem, s, a, segment_length(a.K), tiles, groups);
+  return check_launch("gemm_f32 (few rows)");
+}
+template <int MP, int NT, int CH, int D, bool VEC>
+static int launch_rows(const GemmF32Args& a, cudaStream_t s) {
+  using S = RowsShape<MP, NT, CH, D, VEC>;
   const int tiles = (a.N + NT - 1) / NT, row_tiles = (a.M + MP - 1) / MP;
   SLB_REQUIRE(row_tiles < 65536, "gemm_f32: M=%d needs more than 65535 row tiles", a.M);
   const int room = S::kBlocksPerSm * sm_count() / row_tiles > 1 ? S::kBlocksPerSm * sm_count() / row_tiles : 1;
-  launch_with(a.early ? pdl_mode() != 0 : pdl_mode() == 1, kernel, dim3(tiles < room ? tiles : room, row_tiles), dim3(256), S::kSmem, s, a, segment_length(a.K), tiles);
-  return check_launch("gemm_f32 (few rows)");
+  const int groups = groups_of(a.K, tiles, room);
+  return groups > 1 ? launch_rows_form<MP, NT, CH, D, VEC, true>(a, tiles, row_tiles, room, groups, s)
+                    : launch_rows_form<MP, NT, CH, D, VEC, false>(a, tiles, row_tiles, room, 1, s);
 }
 
-// Which kernel and tile a product takes, from what a round over the SMs costs (nanoseconds per k value, B200, products of 1,024 to
-// 6,144 features): a round of tiles with one block an SM, a round with two, and a round of the streaming kernel's 64 x 32 tiles.
-// The sums of rounds meet the measured times within 5 % (us at 1,500 rows x 6,144 x 1,024: 8 / 6 / 4 rows a thread
-// 399 / 479 / 494; 1,500 x 1,024 x 2,048: 219 / 176 / 251; 300 x 1,024 x 2,048: 218 / 176 / 137, streaming 81).
-constexpr int kRoundAlone[3] = {107, 86, 67}, kRoundTwo[3] = {191, 155, 120}, kRoundRows = 21;      // 8, 6, 4 rows a thread
+// Which kernel and tile a product takes: the sum of its rounds over the SMs, in nanoseconds, fitted to 2,239 products of 32 to 4,099
+// by 130 to 32,768 with 1 to 3,000 rows on a B200 (the sums meet the times above a launch's 7 us within 4 to 7 % rms, 20 % at worst). A round
+// costs a fixed part, which decides where K is small, and a part per k value; tiles of several rounds run two a SM. us, streaming / tiles:
+// 600 rows x 1,024 x 77 43 / 18; 128 x 6,144 x 160 41 / 18; 48 x 32,768 x 160 87 / 29; 300 x 1,024 x 2,048 84 / 142.
+struct TileCost {
+  double alone, alone_k, two, two_k;      // a round with one tile an SM; with two
+};
+constexpr TileCost kTile8{830, 104, 2490, 193}, kTile6{850, 82.6, 1720, 155.6}, kTile4{140, 66, 1110, 121}, kTile8Odd{1650, 105.4, 2910, 199};
 
-static int round_of(int rt) { return rt == 8 ? 0 : (rt == 6 ? 1 : 2); }
-static long long tiles_of(const GemmF32Args& a, int rt) {
-  return (long long)((a.N + kTileN - 1) / kTileN) * ((a.M + 16 * rt - 1) / (16 * rt));
-}
-static long long tile_cost(const GemmF32Args& a, int rt) {
-  const long long sms = sm_count(), tiles = tiles_of(a, rt), rest = tiles % (2 * sms);
-  return tiles / (2 * sms) * kRoundTwo[round_of(rt)] + (rest == 0 ? 0 : (rest <= sms ? kRoundAlone : kRoundTwo)[round_of(rt)]);
-}
-
-// Rounds of the streaming kernel with its largest tile (one block an SM; a block keeps to its 64 rows), times their cost.
-static long long rows_cost(const GemmF32Args& a) {
-  const long long sms = sm_count(), down = (a.M + 63) / 64, across = (a.N + 31) / 32;
-  const long long blocks = down < sms ? (sms / down < across ? sms / down : across) : 1;
-  return (across + blocks - 1) / blocks * ((blocks * down + sms - 1) / sms) * kRoundRows;
+static long long tiles_of(int M, int N, int rt) { return (long long)((N + kTileN - 1) / kTileN) * ((M + 16 * rt - 1) / (16 * rt)); }
+static double tile_cost(int M, int N, int K, int rt, const TileCost& c) {
+  const long long sms = sm_count(), tiles = tiles_of(M, N, rt), rest = tiles % (2 * sms);
+  const double alone = c.alone + c.alone_k * K, two = c.two + c.two_k * K;
+  return (double)(tiles / (2 * sms)) * two + (rest == 0 ? 0.0 : rest <= sms ? alone : two);
 }
 
-template <int RT, bool VEC>
-static int launch_tile(const GemmF32Args& a, cudaStream_t s) {
-  const auto kernel = gemm_f32_tile_kernel<RT, VEC>;
+// The streaming kernel's tiles of mp rows by nt features, one block an SM: per tile of a round, per k value of it, per k value of a chain;
+// one tile a block at a time, and several side by side.
+struct RowsCost {
+  int mp, nt;
+  double tile, k, chain, side_tile, side_k, side_chain;
+};
+constexpr RowsCost kRows64{64, 32, 3880, 11.8, 42, 1190, 12.2, 81}, kRows32{32, 32, 1030, 5.8, 26, 960, 5.6, 39}, kRowsOdd{64, 8, 430, 3.8, 37, 670, 0, 76};
+
+static double rows_cost(int M, int N, int K, const RowsCost& c) {
+  const long long sms = sm_count(), down = (M + c.mp - 1) / c.mp, tiles = (N + c.nt - 1) / c.nt, room = sms / down > 1 ? sms / down : 1;
+  const long long groups = groups_of(K, (int)tiles, (int)room), shares = (tiles + groups - 1) / groups, blocks = shares < room ? shares : room;
+  const long long rounds = (shares + blocks - 1) / blocks * ((blocks * down + sms - 1) / sms);
+  const int chain = K < segment_length(K) ? K : segment_length(K);
+  return rounds * (groups == 1 ? c.tile + c.k * K + c.chain * chain : groups * (c.side_tile + c.side_k * K) + c.side_chain * chain);
+}
+
+// 0: the streaming kernel; 8, 6 or 4: tiles with so many rows a thread. Up to 16 rows, and up to 64 where the features give the
+// streaming kernel's narrow tiles a round to themselves, nothing else comes near it.
+static int choose_f32(int M, int N, int K, bool vec) {
+  if (M <= 16 || (vec && M <= 64 && N < (M <= 32 ? 4096 : 2048))) return 0;
+  if (!vec) return rows_cost(M, N, K, kRowsOdd) <= tile_cost(M, N, K, 8, kTile8Odd) ? 0 : 8;
+  const double t8 = tile_cost(M, N, K, 8, kTile8), t6 = tile_cost(M, N, K, 6, kTile6), t4 = tile_cost(M, N, K, 4, kTile4);
+  const int rt = t8 <= t6 ? (t8 <= t4 ? 8 : 4) : (t6 <= t4 ? 6 : 4);
+  return rows_cost(M, N, K, M <= 32 ? kRows32 : kRows64) <= (rt == 8 ? t8 : rt == 6 ? t6 : t4) ? 0 : rt;
+}
+
+template <int RT, bool VEC, bool SINGLE>
+static int launch_tile_form(const GemmF32Args& a, cudaStream_t s) {
+  const auto kernel = gemm_f32_tile_kernel<RT, VEC, SINGLE>;
   // One block an SM is asked for (by its shared memory) where every tile gets an SM of its own: left to itself a kernel that
   // starts while the one before still runs finds half-empty SMs and doubles up there (1,500 x 1,024 x 2,048: 276 instead of 176 us).
   constexpr int kAlone = 116 * 1024;
@@ -385,14 +435,21 @@ static int launch_tile(const GemmF32Args& a, cudaStream_t s) {
   if (e != cudaSuccess) return fail(2, "gemm_f32: cannot reserve %d bytes of shared memory: %s", kAlone, cudaGetErrorString(e));
   const dim3 grid((a.N + kTileN - 1) / kTileN, (a.M + 16 * RT - 1) / (16 * RT));
   SLB_REQUIRE(grid.y < 65536, "gemm_f32: M=%d needs more than 65535 row tiles", a.M);
-  const int smem = tiles_of(a, RT) <= sm_count() ? kAlone : tile_smem(RT);
+  const int smem = tiles_of(a.M, a.N, RT) <= sm_count() ? kAlone : tile_smem(RT);
   launch_with(a.early ? pdl_mode() != 0 : pdl_mode() == 1, kernel, grid, dim3(256), smem, s, a, segment_length(a.K));
   return check_launch("gemm_f32 (tiles)");
+}
+template <int RT, bool VEC>
+static int launch_tile(const GemmF32Args& a, cudaStream_t s) {
+  return a.K <= segment_length(a.K) ? launch_tile_form<RT, VEC, true>(a, s) : launch_tile_form<RT, VEC, false>(a, s);
 }
 
 }  // namespace slb
 
 using namespace slb;
+
+// What slb_gemm_f32 takes: 0 the streaming kernel, 8, 6 or 4 tiles with so many rows a thread (vec: operands that 16-byte reads can take).
+extern "C" int slb_gemm_f32_choice(int M, int N, int K, int vec) { return choose_f32(M, N, K, vec != 0); }
 
 // static_weight: no kernel writes W (a loaded matrix), so that it may be read while the kernel in front of this one still runs.
 extern "C" int slb_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda,
@@ -404,14 +461,12 @@ extern "C" int slb_gemm_f32(const float* A, const float* W, const float* bias, f
   cudaStream_t s = (cudaStream_t)stream;
   const GemmF32Args a{A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, static_weight};
   const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
-  int rt = 8;
-  if (tile_cost(a, 6) < tile_cost(a, rt)) rt = 6;
-  if (tile_cost(a, 4) < tile_cost(a, rt)) rt = 4;
-  const bool few = M <= 64 || rows_cost(a) < tile_cost(a, rt);
-  if (!vec) {      // no 16-byte reads: copies of four bytes
+  const int rt = choose_f32(M, N, K, vec);
+  if (rt == 0 && !vec) {      // no 16-byte reads: copies of four bytes
     if (M <= 16) return launch_rows<16, 8, 32, 2, false>(a, s);
-    if (few) return launch_rows<64, 8, 32, 2, false>(a, s);
-  } else if (few) {
+    return launch_rows<64, 8, 32, 2, false>(a, s);
+  }
+  if (rt == 0) {
     // 32 features a tile where that still gives every SM one, else 16 or 8
     const int nt = N >= 4096 ? 32 : (N >= 2048 ? 16 : 8);
     if (M <= 1) return nt >= 16 ? launch_rows<1, 16, 64, 4, true>(a, s) : launch_rows<1, 8, 64, 4, true>(a, s);

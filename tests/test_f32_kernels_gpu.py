@@ -12,8 +12,8 @@ from test_kernels_gpu import DEV, make_cache, ops, plain_attention
 pytestmark = pytest.mark.gpu
 
 
-# Few rows: every row tile (1, 2, 4, 8, 16, 32, 64 rows), both feature tiles (8; 16 from 8,192 features on), segments of 128 and more,
-# a last segment that is short or missing, inner dimensions that no 16-byte copy takes. Many rows: tiles of 128, 96 and 64 rows.
+# Few rows: tiles of 1, 2, 8, 16, 32 and 64 rows by 8 features (16 from 2,048 features on, 32 from 4,096), segments of 128 and more, a last
+# segment that is short or missing, inner dimensions that no 16-byte copy takes. Many rows: tiles of 128 and 96 rows.
 @pytest.mark.parametrize("M,N,K", [(1, 8, 4), (1, 9, 132), (2, 8200, 96), (3, 17, 1028), (7, 8192, 260), (8, 1000, 1024), (9, 8195, 644),
                                    (16, 40, 3072), (20, 8200, 132), (33, 100, 1100), (64, 8197, 200), (65, 8, 2052), (100, 24, 77),
                                    (129, 1024, 1024), (700, 1000, 388), (1500, 1030, 64), (1500, 2304, 100), (1100, 6150, 36)])
@@ -38,6 +38,17 @@ def test_gemm_f32_error_and_rows(M, N, K):
     plain = torch.empty(M, N, device=DEV)
     ops().gemm_f32(a, w, plain)
     assert torch.equal(acc, plain + 2.0)
+
+
+# 16- and 32-feature tiles of every row tile with several segments and several tiles a block; inner dimensions of one to seven
+# segments, of one and two with tiles side by side in a block (up to eight and four, a last share that is not full), also off a multiple
+# of 4; tiles of 128, 96 and 64 rows with one segment and with several; many rows off a multiple of 4.
+@pytest.mark.parametrize("M,N,K", [(4, 4100, 1028), (3, 2050, 2052), (8, 2100, 1100), (16, 3000, 1028), (32, 2056, 2052), (1, 5003, 1032), (2, 2051, 516),
+                                   (5, 4100, 77), (64, 700, 130), (3, 33, 200), (20, 5000, 300), (60, 12291, 96), (1, 20011, 128), (12, 9001, 388), (64, 4099, 260),
+                                   (9, 700, 900), (300, 520, 1030), (1000, 1030, 77), (130, 6150, 333), (700, 300, 129), (2000, 700, 48), (450, 2050, 130), (600, 503, 160),
+                                   (300, 1030, 260), (128, 6144, 96), (48, 32801, 160), (7, 40001, 200), (2, 33000, 130), (16, 70001, 68), (1200, 6150, 260), (1500, 1030, 516)])
+def test_gemm_f32_groups_of_tiles_and_odd_inner_dimensions(M, N, K):
+    test_gemm_f32_error_and_rows(M, N, K)
 
 
 def run_f32(q, k_pool, v_pool, table, pasts, counts, heads, kv_heads, hd, window, sinks=None):
