@@ -406,6 +406,7 @@ constexpr float kBanned = -1e30f;      // logits below are no candidates' (bans 
 constexpr int kQuickList = 1024;       // candidates of a row at most
 constexpr int kSmallList = 512;        // up to this many entries are compared each with each
 
+template <int THREADS>
 struct Held {
   float4* mine;            // this thread's first float4; the next ones a block's threads apart
   int begin, end;          // its warp's stretch of tokens (row numbers), whole chunks of 128 but for the row's last
@@ -414,7 +415,7 @@ struct Held {
 #pragma unroll 2
     for (int c = 0; begin + 128 * c < end; ++c) {
       const int t = begin + 128 * c + 4 * lane;
-      const float4 v = mine[c * blockDim.x];
+      const float4 v = mine[c * THREADS];
       if (t < end) f(t, v.x);
       if (t + 1 < end) f(t + 1, v.y);
       if (t + 2 < end) f(t + 2, v.z);
@@ -578,7 +579,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
 
   const bool count_first = top_k > 0 && top_k < limit;
   const int chunks = (raw.n + 128 * kWarps - 1) / (128 * kWarps);
-  Held mine{held + threadIdx.x, part_begin + warp * chunks * 128, min(part_end, part_begin + (warp + 1) * chunks * 128), lane};
+  Held<THREADS> mine{held + threadIdx.x, part_begin + warp * chunks * 128, min(part_end, part_begin + (warp + 1) * chunks * 128), lane};
   bool quick = per_block <= kHeldTokens && (count_first ? top_k <= kQuickList : top_p < 1.0f);      // the same for all blocks of a row
   if (quick) {
     // the one read of the row; the largest value, bounds from below, and whether anything is no number. Banned tokens (minus
