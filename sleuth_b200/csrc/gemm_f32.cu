@@ -392,8 +392,8 @@ struct TileCost {
 constexpr TileCost kTile8{830, 104, 2490, 193}, kTile6{850, 82.6, 1720, 155.6}, kTile4{140, 66, 1110, 121}, kTile8Odd{1650, 105.4, 2910, 199};
 
 static long long tiles_of(int M, int N, int rt) { return (long long)((N + kTileN - 1) / kTileN) * ((M + 16 * rt - 1) / (16 * rt)); }
-static double tile_cost(int M, int N, int K, int rt, const TileCost& c) {
-  const long long sms = sm_count(), tiles = tiles_of(M, N, rt), rest = tiles % (2 * sms);
+static double tile_cost(int M, int N, int K, int rt, const TileCost& c, long long sms) {
+  const long long tiles = tiles_of(M, N, rt), rest = tiles % (2 * sms);
   const double alone = c.alone + c.alone_k * K, two = c.two + c.two_k * K;
   return (double)(tiles / (2 * sms)) * two + (rest == 0 ? 0.0 : rest <= sms ? alone : two);
 }
@@ -406,8 +406,8 @@ struct RowsCost {
 };
 constexpr RowsCost kRows64{64, 32, 3880, 11.8, 42, 1190, 12.2, 81}, kRows32{32, 32, 1030, 5.8, 26, 960, 5.6, 39}, kRowsOdd{64, 8, 430, 3.8, 37, 670, 0, 76};
 
-static double rows_cost(int M, int N, int K, const RowsCost& c) {
-  const long long sms = sm_count(), down = (M + c.mp - 1) / c.mp, tiles = (N + c.nt - 1) / c.nt, room = sms / down > 1 ? sms / down : 1;
+static double rows_cost(int M, int N, int K, const RowsCost& c, long long sms) {
+  const long long down = (M + c.mp - 1) / c.mp, tiles = (N + c.nt - 1) / c.nt, room = sms / down > 1 ? sms / down : 1;
   const long long groups = groups_of(K, (int)tiles, (int)room), shares = (tiles + groups - 1) / groups, blocks = shares < room ? shares : room;
   const long long rounds = (shares + blocks - 1) / blocks * ((blocks * down + sms - 1) / sms);
   const int chain = K < segment_length(K) ? K : segment_length(K);
@@ -418,10 +418,11 @@ static double rows_cost(int M, int N, int K, const RowsCost& c) {
 // streaming kernel's narrow tiles a round to themselves, nothing else comes near it.
 static int choose_f32(int M, int N, int K, bool vec) {
   if (M <= 16 || (vec && M <= 64 && N < (M <= 32 ? 4096 : 2048))) return 0;
-  if (!vec) return rows_cost(M, N, K, kRowsOdd) <= tile_cost(M, N, K, 8, kTile8Odd) ? 0 : 8;
-  const double t8 = tile_cost(M, N, K, 8, kTile8), t6 = tile_cost(M, N, K, 6, kTile6), t4 = tile_cost(M, N, K, 4, kTile4);
+  const int sms = sm_count();
+  if (!vec) return rows_cost(M, N, K, kRowsOdd, sms) <= tile_cost(M, N, K, 8, kTile8Odd, sms) ? 0 : 8;
+  const double t8 = tile_cost(M, N, K, 8, kTile8, sms), t6 = tile_cost(M, N, K, 6, kTile6, sms), t4 = tile_cost(M, N, K, 4, kTile4, sms);
   const int rt = t8 <= t6 ? (t8 <= t4 ? 8 : 4) : (t6 <= t4 ? 6 : 4);
-  return rows_cost(M, N, K, M <= 32 ? kRows32 : kRows64) <= (rt == 8 ? t8 : rt == 6 ? t6 : t4) ? 0 : rt;
+  return rows_cost(M, N, K, M <= 32 ? kRows32 : kRows64, sms) <= (rt == 8 ? t8 : rt == 6 ? t6 : t4) ? 0 : rt;
 }
 
 template <int RT, bool VEC, bool SINGLE>
