@@ -15,8 +15,8 @@
 //
 // Before, the general kernel read every key and value row once per query and head. 16 / 8 heads of 128, us before / now: eight
 // prompts of 400 tokens 2,034 / 197, single tokens at a context of 700 (batch 8) 41 / 16, at 4,000 (batch 1) 184 / 23. Portions (cold caches),
-// the general kernel / tiles of 64 rows walking all keys / now: 2 tokens on 4,000 keys 366 / 606 / 40, 32 391 / 610 / 60; 64 sequences of 2 on 500
-// 239 / 281 / 106. Where the general kernel was as fast: up to a dozen keys in all (12 against 13), 16 query heads a group on less than 60 (11 / 22).
+// the general kernel / tiles of 64 rows walking all keys / now: 2 tokens on 4,000 keys 366 / 606 / 40, 32 391 / 610 / 67; 64 sequences of 2 on 500
+// 239 / 281 / 108. Where the general kernel was as fast: up to a dozen keys in all (12 against 13), 16 query heads a group on less than 60 (11 / 22).
 #include <math.h>
 
 #include "packed_f32.cuh"

@@ -26,7 +26,7 @@ namespace slb {
 constexpr int kMoeTile = 32;        // rows (pairs) of a product tile
 constexpr int kMoeCols = 64;        // output columns of a product tile
 constexpr int kMoeK = 32;           // inner-dimension slice staged in shared memory
-constexpr int kMoeFewPairs = 64;    // up to this many (token, choice) pairs a step runs a warp per output instead of tiles
+constexpr int kMoeFewPairs = 64;    // up to this many (token, choice) pairs a step takes kernels of its own (moe_few_*) instead of tiles
 
 // Router logits for many tokens: z[t, e] = w[e] . h[t] + b[e], float32, k ascending. A block takes 32 tokens and 16
 // experts; the tokens' rows and the experts' rows go through shared memory 128 values at a time; a lane is a token,
@@ -536,9 +536,10 @@ __global__ void __launch_bounds__(128) moe_mma_kernel(const __nv_bfloat16* __res
   }
 }
 
-// ---- few pairs (single-token steps): a warp per output, every weight row streamed once per pair that uses it ----
+// ---- few pairs (single-token steps) ----
+// Two kernels with a warp per output, every weight row streamed once per pair that uses it.
 // (act rows lie in the order of the pairs here: nothing needs the expert order, so a step of few pairs skips the layout.)
-// These two serve float32 and widths that are no multiples of 32; the kernels behind them the rest.
+// They serve float32, widths that are no multiples of 32 and small matrices; the kernels behind them the rest.
 // grid (pairs, column groups of 8): act[pair, j] = f(gate_e[j] . h[token]) * (up_e[j] . h[token]).
 template <typename T>
 __global__ void __launch_bounds__(256) moe_few_gate_up_kernel(const T* __restrict__ h, const T* __restrict__ w_gu,
@@ -1033,7 +1034,7 @@ extern "C" int slb_moe_route(const void* h, const float* w_router, const float* 
 // E: the experts that have matrices; `identity` more may be among the choices (numbers E ..). store: x = the sum instead of x += .
 // act: [tokens * top, ff] in the run dtype; y: float32 [tokens * top, dim]; x: the float32 stream [tokens, dim]; extra: null,
 // or float32 [tokens, dim] rows that the same kernel adds into the stream (steps of few pairs only).
-// choice (from slb_moe_route) serves steps of few pairs, which run a warp per output instead of tiles and need neither
+// choice (from slb_moe_route) serves steps of few pairs, which have kernels of their own instead of tiles and need neither
 // the counts nor the expert-ordered list (`place` is accepted for callers that have it and is not read).
 extern "C" int slb_moe_experts(const void* h, const void* w_gu, const void* w_down, const int* counts, const int* list,
                                const int* choice, const int* place, const float* weight, void* act, float* y, float* x,
