@@ -682,8 +682,8 @@ __device__ __forceinline__ int take_rows(unsigned long long& with, int g, int& p
 // grid (pairs, groups of 64 / PARTS columns): act[pair, j] = f(gate_e[j] . h[token]) * (up_e[j] . h[token]), for the pairs that share the
 // expert of pair blockIdx.x, if it is the first of them. A warp takes one of PARTS parts of the width for 8 columns: a quarter, so that a
 // warp has many loads to ask for and the blocks, which all wait for the choices first, are few rounds; an eighth where there are few
-// columns. us a layer, both products, eighths / quarters: width 2,048, 64 experts of 1,408, 6 a token, 8 tokens 130 / 123; 1,024, 16 of 768, 4 a
-// token, 1 token 10.6 / 11.2, 16 tokens 30.4 / 27.0; 1,024, 16 of 512, 2 a token, 1 token 7.8 / 8.8; 512, 32 of 512, 4 a token, 4 tokens 15.6 / 14.0.
+// columns (single tokens, the usual step there, are faster with it). us a layer, both products, eighths / quarters: width 2,048, 64 experts of
+// 1,408, 6 a token, 8 tokens 130 / 123; 1,024, 16 of 768, 4 a token, 1 token 10.6 / 11.2, 16 tokens 30.4 / 27.0; 1,024, 16 of 512, 2 a token, 1 token 7.8 / 8.8; 512, 32 of 512, 4 a token, 4 tokens 15.6 / 14.0.
 template <int PARTS>
 __global__ void __launch_bounds__(256, 3) moe_few_gate_up_mma_kernel(MoeFewArgs a) {
   pdl_enter();
@@ -1065,7 +1065,7 @@ extern "C" int slb_moe_experts(const void* h, const void* w_gu, const void* w_do
                          (int)pairs, top, dim, ff, E, store, gate};
       // The parts depend on the matrices alone, so that a token's bits do not depend on the tokens beside it.
       const auto gate_up = [&](auto kernel, int parts) { launch(kernel, dim3((unsigned)pairs, (ff + 64 / parts - 1) / (64 / parts)), block, 0, s, a); };
-      if (ff <= 512 && dim >= 1024) gate_up(moe_few_gate_up_mma_kernel<8>, 8);
+      if (dim >= 1024 && ff <= (dim < 2048 ? 1024 : 512)) gate_up(moe_few_gate_up_mma_kernel<8>, 8);
       else gate_up(moe_few_gate_up_mma_kernel<4>, 4);
       // Long rows in more parts, short ones whole where the columns make blocks enough (2,048 x 768, 8 of 128 experts a token, 8 tokens: 99 / 93 us
       // in halves / whole; 1,024 x 3,584, 2 of 8, 1 token: 21.9 / 19.1 in halves / quarters).
