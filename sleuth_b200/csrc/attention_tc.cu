@@ -191,7 +191,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   trace.mark(1);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- scores: loads Q and the key pages, issues S_j = Q K_j^T one page ahead of the softmax. A page's keys are
       // asked for before the products of the page before are issued, its number a page earlier still ----
       constexpr uint32_t idesc_s = instr_desc(kAtRows, 64);
@@ -235,7 +235,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       trace.mark(2);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- values: loads the value pages, issues O += P_j V_j as soon as the softmax has written P_j ----
       constexpr uint32_t idesc_o = instr_desc(kAtRows, HD, true);
       auto page_of = [&](int i) { return i < n_pages ? table[page_lo + i] : 0; };
@@ -509,10 +509,10 @@ attn_tc_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   trace.mark(1);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- scores: Q once, two key pages per step, S_j = Q K_j^T a step ahead of the softmax. The two pages of a
-      // stage lie one behind the other in each 64-wide half of the head, so one product of N = 128 covers both (an
-      // instruction costs the same time whatever its N); the page numbers of the step after next are asked for a
+      // stage lie one behind the other in each 64-wide half of the head, so one product of N = 128 covers both (96
+      // cycles an instruction, two of N = 64 take 2 x 68); the page numbers of the step after next are asked for a
       // step early, and a step's keys are asked for before the products of the step before are issued ----
       constexpr uint32_t idesc_s2 = instr_desc(kAtRows, 128), idesc_s1 = instr_desc(kAtRows, 64);
       auto page_of = [&](int i) { return i < n_pages ? table[page_lo + i] : 0; };
@@ -560,7 +560,7 @@ attn_tc_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       trace.mark(2);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- values: two value pages per step, O += P_j V_j as soon as the softmax has written P_j ----
       constexpr uint32_t idesc_o = instr_desc(kAtRows, HD, true);
       auto page_of = [&](int i) { return i < n_pages ? table[page_lo + i] : 0; };

@@ -388,7 +388,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   }
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- producer ----
       int it = 0;
       bool ok = true;
@@ -424,36 +424,33 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       trace.mark(2);
     }
   } else if (warp == 1 && rank == 0) {
-    // ---- MMA issuer: the whole warp walks the loop (its counters and descriptors then live in uniform registers),
-    // one lane issues the products and the commits; of a pair, the even block's ----
-    constexpr uint32_t idesc = instr_desc(kRows, BN);
-    constexpr uint32_t kAll = 0xffffffffu;
-    int it = 0, t = 0;
-    bool ok = true;
-    bool next_ready = false;
-    for (int tile = worker; tile < total && ok; tile += n_workers, ++t) {
-      const int buf = t & 1;
-      if (t >= 2 && !__all_sync(kAll, mbar_wait(tempty0 + 8 * buf, ((t / 2) - 1) & 1))) {   // the epilogue has drained this accumulator
-        if (lane == 0) atomicExch(a.status, 4);
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t acc = tmem + (uint32_t)(buf * BN);
-      for (int kt = 0; kt < k_tiles; ++kt, ++it) {
-        const int s = it % S;
-        if (!next_ready && !__all_sync(kAll, mbar_wait(full0 + 8 * s, (it / S) & 1))) {
-          if (lane == 0) atomicExch(a.status, 2);
-          ok = false;
+    // ---- MMA issuer (of a pair, the even block's) ----
+    if (elect_one()) {
+      constexpr uint32_t idesc = instr_desc(kRows, BN);
+      int it = 0, t = 0;
+      bool ok = true, next_ready = false;
+      for (int tile = worker; tile < total && ok; tile += n_workers, ++t) {
+        const int buf = t & 1;
+        if (t >= 2 && !mbar_wait(tempty0 + 8 * buf, ((t / 2) - 1) & 1)) {      // the epilogue has drained this accumulator
+          atomicExch(a.status, 4);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // A look at the next stage's barrier goes out before this stage's products: its answer (a couple of
-        // hundred cycles away) is back by the time they are issued, so a loaded stage costs no wait of its own.
-        const int sn = (it + 1) % S;
-        const uint32_t probe = mbar_test(full0 + 8 * sn, ((it + 1) / S) & 1);
-        const uint32_t sa = tiles + s * STAGE, sb = sa + A_BYTES;
-        const uint64_t da = smem_desc(sa), db = smem_desc(sb);
-        if (lane == 0) {
+        const uint32_t acc = tmem + (uint32_t)(buf * BN);
+        for (int kt = 0; kt < k_tiles; ++kt, ++it) {
+          const int s = it % S;
+          if (!next_ready && !mbar_wait(full0 + 8 * s, (it / S) & 1)) {
+            atomicExch(a.status, 2);
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          // A look at the next stage's barrier goes out before this stage's products: its answer (a couple of
+          // hundred cycles away) is back by the time they are issued, so a loaded stage costs no wait of its own.
+          const int sn = (it + 1) % S;
+          const uint32_t probe = mbar_test(full0 + 8 * sn, ((it + 1) / S) & 1);
+          const uint32_t sa = tiles + s * STAGE, sb = sa + A_BYTES;
+          const uint64_t da = smem_desc(sa), db = smem_desc(sb);
 #pragma unroll
           for (int k4 = 0; k4 < kTcBK / 16; ++k4) {  // 16 elements = 32 bytes further along K inside the swizzle row
             if constexpr (PAIR) mma_bf16_ss_pair(acc, da + (uint64_t)(k4 * 2), db + (uint64_t)(k4 * 2), idesc, (kt > 0 || k4 > 0) ? 1u : 0u);
@@ -461,14 +458,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
           }
           if constexpr (PAIR) mma_commit_pair(empty0 + 8 * s);      // both blocks' stages
           else mma_commit(empty0 + 8 * s);           // fires when these MMAs have read the stage
+          next_ready = probe != 0;
         }
-        next_ready = __all_sync(kAll, probe != 0);
+        if (ok) {                                    // fires when the whole tile has been accumulated
+          if constexpr (PAIR) mma_commit_pair(tfull0 + 8 * buf);
+          else mma_commit(tfull0 + 8 * buf);
+        }
       }
-      if (ok && lane == 0) {                                    // fires when the whole tile has been accumulated
-        if constexpr (PAIR) mma_commit_pair(tfull0 + 8 * buf);
-        else mma_commit(tfull0 + 8 * buf);
-      }
-      __syncwarp();
     }
   } else if (warp >= 2) {
     // ---- epilogue: warps 2..5, tensor-memory lanes 32 * (warp % 4) .. + 31 ----
@@ -566,6 +562,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
     }
   }
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   if constexpr (PAIR) {
     cluster_sync_all();        // neither block frees tensor memory, or leaves, while the other may still be signalled

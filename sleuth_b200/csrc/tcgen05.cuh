@@ -85,6 +85,16 @@ __host__ __device__ constexpr uint32_t instr_desc(int M, int N, bool b_mn_major 
          ((uint32_t)(M >> 4) << 24);
 }
 
+// True in one lane of a converged warp, always the same one. Products and commits are issued under this and not under `lane == 0`:
+// the compiler knows of elect.sync that one thread runs what follows, and hands descriptors to the tensor core without a loop over
+// the lanes that might be active. Cycles from one tcgen05.mma (128 rows, K = 16) to the next, back to back, under a lane test / under elect_one:
+// N = 16 144 / 54, N = 64 144 / 68, N = 128 144 / 96 (A from tensor memory: 144 / 72), N = 256 161 / 160.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void mma_bf16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                             uint32_t accumulate) {
   asm volatile(
