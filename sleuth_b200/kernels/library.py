@@ -192,6 +192,8 @@ _SIGNATURES = {
     "slb_unit_post": [P, L, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, P],
     "slb_diff_combine": [P, P, L, P, I, I, I, F, F, F, I, I, P],
     "slb_streams_fill": [P, P, L, I, I, P],
+    "slb_head_pages": [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
+    "slb_head_rows": [P, P, P, L, P, I, I, I, I, P],
     "slb_hyper_read": [P, P, P, P, L, I, I, F, I, P],
     "slb_hyper_write": [P, P, P, P, L, I, I, F, P],
     "slb_streams_sum": [P, P, L, I, I, P],

@@ -1066,6 +1066,38 @@ def head_prompt_attention(q, kv, k_rot, out, cos, sin, seq_start, counts, max_co
                _p(sinks), stream if stream is not None else current_stream())
 
 
+def head_pages(q, kv, k_rot, q_out, k_pages, v_pages, cos, sin, tok_seq, tok_pos, seq_start, plain_dim: int, value_dim: int, rotated: int,
+               stream=None) -> None:
+    """Queries, keys and values of whole prompts (operands as for ``head_prompt_attention``) in rows as wide as the tcgen05 attention
+    takes, zeros at their ends: queries turned into ``q_out`` [T, heads, width], keys and values into the per-head pages of the step
+    (``prompt_pages``; ``latent_post`` writes their table and clears the value rows behind every sequence's last token)."""
+    _cuda(q, kv, k_rot, q_out, k_pages, v_pages, cos, sin, tok_seq, tok_pos, seq_start)
+    T, H, dk = q.shape
+    W, P = q_out.shape[2], k_rot.shape[1]
+    _need(dk == plain_dim + P and kv.shape == (T, H * (plain_dim + value_dim)) and k_rot.shape[0] == T and q_out.shape == (T, H, W)
+          and k_pages.shape == v_pages.shape and tuple(k_pages.shape[1:]) == (H, 64, W), "head_pages: shapes")
+    _need(all(x.dtype == torch.bfloat16 and x.is_contiguous() for x in (q, kv, k_rot, q_out, k_pages, v_pages)), "head_pages: contiguous bfloat16")
+    _need(tok_seq.numel() >= T and tok_pos.numel() >= T, "head_pages: per-token tables")
+    if rotated:
+        _need(cos is not None and cos.dtype == torch.float32 and cos.shape[1] == rotated // 2, "head_pages: rotation tables")
+    lib().call("slb_head_pages", _p(q), _p(kv), _p(k_rot), _p(q_out), _p(k_pages), _p(v_pages), _p(cos), _p(sin), _p(tok_seq), _p(tok_pos),
+               _p(seq_start), T, H, plain_dim, P, value_dim, rotated, W, stream if stream is not None else current_stream())
+
+
+def head_rows(rows, y, gate=None, head_gate=None, stream=None) -> None:
+    """y[t, h, :] = the first channels of rows[t, h, :] (bfloat16 [T, heads, width]) times sigmoid(gate): ``gate`` bfloat16 like ``y``
+    [T, heads * value width], or ``head_gate`` float32 [T, heads] (unit column stride), or neither."""
+    _cuda(rows, y, gate)
+    T, H, W = rows.shape
+    dv = y.shape[1] // H
+    _need(y.shape == (T, H * dv) and rows.dtype == y.dtype == torch.bfloat16 and rows.is_contiguous() and y.is_contiguous(), "head_rows: shapes or dtypes")
+    _need(gate is None or (gate.shape == y.shape and gate.dtype == torch.bfloat16 and gate.is_contiguous()), "head_rows: gate")
+    _need(head_gate is None or (head_gate.is_cuda and head_gate.dtype == torch.float32 and head_gate.shape == (T, H) and head_gate.stride(1) == 1),
+          "head_rows: a head's gates are float32 [tokens, heads]")
+    stride = 0 if head_gate is None else (head_gate.stride(0) if T > 1 else H)
+    lib().call("slb_head_rows", _p(rows), _p(gate), _p(head_gate), stride, _p(y), T, H, dv, W, stream if stream is not None else current_stream())
+
+
 def latent_gate(val, g, y, stream=None) -> None:
     """y[t, h, :] = val[h, t, :] * sigmoid(g[t, h, :]); val [heads, T, width], g and y [T, heads * width]."""
     _cuda(val, g, y)

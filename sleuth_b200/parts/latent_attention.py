@@ -170,12 +170,13 @@ class LatentAttention(Part):
         cq = ws.take((T, s.q_rank), dt) if s.q_rank else None
         fresh = getattr(b, "fresh", False) and b.max_count >= PER_HEAD_PROMPT_TOKENS
         paged = fresh and self._prompt_takes_pages(b, T)
-        per_head = fresh and (paged or ops.head_prompt_supported(dn, P, dv, dt))
+        width = 0 if paged or not fresh else self._prompt_row_width(b)
+        per_head = fresh and (paged or width or ops.head_prompt_supported(dn, P, dv, dt))
         c_out = ws.take((T, R), dt) if per_head else None
         k_out = ws.take((T, P), dt) if per_head else None
         own = None
-        if paged:
-            shape = (ops.prompt_pages(T, b.n), H, 64, dn)
+        if paged or width:
+            shape = (ops.prompt_pages(T, b.n), H, 64, width or dn)
             k_pages, v_pages = ws.take(shape, dt), ws.take(shape, dt)
             own = (ws.take((b.n, -(-b.max_count // 64)), torch.int32), b.seq_start, v_pages)
         ops.latent_post(lat, self.q_gain, self.c_gain, cos, sin, cq, view.pool if view.writes else None, b.tok_seq,
@@ -198,6 +199,17 @@ class LatentAttention(Part):
             g = lat[:, s.q_rank + R + P:s.q_rank + R + P + H]
         else:
             g = self.gate.forward(h, ws=ws, stream=b.stream) if self.gate is not None else None
+        if width:
+            # rows as wide as the tcgen05 attention takes, zeros at their ends
+            kv = self.ukv.forward(c_out, ws=ws, stream=b.stream)
+            q_rows, y_rows, y = ws.take((T, H, width), dt), ws.take((T, H, width), dt), ws.take((T, H * dv), dt)
+            ops.head_pages(q, kv, k_out, q_rows, k_pages, v_pages, cos, sin, b.tok_seq, b.tok_pos, b.seq_start, dn, dv, rotated, b.stream)
+            ops.attention_tc(q_rows, k_pages, v_pages, y_rows.view(T, H * width), b.seq_start, b.past, b.counts, own[0], b.max_count, H, H,
+                             width, view.window, s.scale, b.stream, max_keys=b.max_count, sinks=self.sinks)
+            ops.head_rows(y_rows, y, gate=None if self.head_gate else g, head_gate=g if self.head_gate else None, stream=b.stream)
+            self.o.forward(y, ws=ws, stream=b.stream, next_read=getattr(b, "next_read", None), **result_target(b, x))
+            ws.release(mark)
+            return
         if per_head:
             kv = self.ukv.forward(c_out, ws=ws, stream=b.stream)
             val = ws.take((H, T, dv), dt)
@@ -228,6 +240,17 @@ class LatentAttention(Part):
         return (s.rot_dim == 0 and s.plain_dim == s.value_dim and not self.head_gate
                 and use_tc_attention(s.heads, s.heads, s.plain_dim, self.ctx.dtype, b.max_count, s.scale)
                 and use_tc(T, 2 * s.heads * s.plain_dim, s.kv_rank))
+
+    def _prompt_row_width(self, b) -> int:
+        """The width of rows in which the step's whole prompts go through the tcgen05 attention with zeros at the rows' ends; 0 where
+        they do not: wider heads, odd widths, sequences that do not fill that kernel's tiles. 2,048 tokens, 16 heads of 64 + 32 key
+        and 64 value channels: 141 us a layer for the attention of heads as they are on mma.sync, 56 this way."""
+        s = self.spec
+        dk = s.plain_dim + s.rot_dim
+        if s.plain_dim % 8 or s.rot_dim % 8 or s.value_dim % 8 or max(dk, s.value_dim) > 128:
+            return 0
+        width = 64 if max(dk, s.value_dim) <= 64 else 128
+        return width if use_tc_attention(s.heads, s.heads, width, self.ctx.dtype, b.max_count, s.scale) else 0
 
     def _step_takes(self, dt) -> bool:
         s = self.spec
