@@ -552,14 +552,19 @@ def decode_scratch_floats(n_seqs: int, heads: int, head_dim: int, splits: int) -
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias=None, accumulate: bool = False,
-             stream=None, static_weight: bool = False) -> None:
-    """out[M, N] (+)= a[M, K] @ w[N, K]^T (+ bias), all float32, plain FMA. ``static_weight``: no kernel writes ``w`` (a loaded
-    matrix), so it may be read before the kernel in front has finished."""
+             stream=None, static_weight: bool = False, form=None) -> None:
+    """out[M, N] (+)= a[M, K] @ w[N, K]^T (+ bias), all float32, every product and sum to float32. ``static_weight``: no kernel
+    writes ``w`` (a loaded matrix), so it may be read before the kernel in front has finished. ``form`` = (tokens of a tile, blocks
+    that share K, warps that split) sends the product to the tensor-core kernel in that form; the bits do not depend on it."""
     _cuda(a, w, out, bias)
     M, K = a.shape
     N = w.shape[0]
     _need(w.shape[1] == K and out.shape == (M, N), "gemm_f32: shapes disagree")
     _need(a.dtype == w.dtype == out.dtype == torch.float32, "gemm_f32: float32 only")
+    if form is not None:
+        lib().call("slb_gemm_f32_tc", _p(a), _p(w), _p(bias), _p(out), M, N, K, K, K, N, int(accumulate), int(static_weight),
+                   *(int(f) for f in form or (0, 0, 0)), _p(_tc_status(a.device)), stream if stream is not None else current_stream())
+        return
     lib().call("slb_gemm_f32", _p(a), _p(w), _p(bias), _p(out), M, N, K, K, K, N, int(accumulate), int(static_weight),
                stream if stream is not None else current_stream())
 
