@@ -701,6 +701,26 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: str, stre
                stream if stream is not None else current_stream())
 
 
+def stream_supported(M: int, N: int, K: int) -> bool:
+    """Whether the weight-streaming tcgen05 kernel takes this problem."""
+    return 1 <= M <= 128 and N >= 1 and K >= 64 and K % 8 == 0
+
+
+def gemm_stream(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: str, stream=None, gate=None, static_weight: bool = False,
+                splits: int = 0) -> None:
+    """out = x[M, K] @ w^T for up to 128 rows, the weights streamed through the tcgen05 tensor cores as the instruction's rows. Modes as
+    for ``gemm_skinny``. ``splits``: blocks that share K (0: the launcher's rule); ``static_weight`` as for ``gemm_f32``."""
+    _cuda(x, w, out)
+    M, K = x.shape
+    N = out.shape[1]
+    _need(x.dtype == w.dtype == torch.bfloat16 and w.shape[1] == K and out.shape[0] == M and out.is_contiguous() and x.is_contiguous()
+          and w.is_contiguous(), "gemm_stream: shapes or dtypes")
+    _need(w.shape[0] == (2 * N if mode == "swiglu" else N), "gemm_stream: weight rows")
+    _need(out.dtype == (torch.bfloat16 if mode in ("bf16", "swiglu") else torch.float32), "gemm_stream: output dtype")
+    lib().call("slb_gemm_stream", _p(x), _p(w), _p(out), M, N, K, N, SKINNY_MODES[mode], *(_gate_args(gate) or (0, 0.0, 1.0)),
+               int(static_weight), int(splits), _p(_tc_status(x.device)), stream if stream is not None else current_stream())
+
+
 def gemm_tc_qkv(x, w, heads: int, kv_heads: int, head_dim: int, bias, q_gain, k_gain, cos, sin, eps: float, q_out,
                 k_pool, v_pool, tok_seq, tok_pos, block_table, stream=None) -> None:
     """The fused q/k/v projection of many tokens with everything ``qkv_post`` does in its epilogue, on the float32
