@@ -36,7 +36,7 @@ def test_every_form_gives_the_same_bits(M, N, K):
         try:
             ops().gemm_f32(a, w, out, form=form, static_weight=True)
         except RuntimeError as e:
-            assert "do not fit" in str(e) and form[1] == 2 and K >= 3000, form
+            assert "do not fit" in str(e) and form[1] in (2, 4) and form[2] == 8 and K > 2000, form
             continue
         assert torch.equal(out, want), form
         ops().gemm_f32(a, w, out, accumulate=True, form=form)
