@@ -4,6 +4,8 @@
   output element sums over k in one fixed order whatever the number of rows.
 * bfloat16 run, up to 32 rows (decode steps): the package's weight-streaming tensor-core kernel
   (``csrc/gemm_skinny.cu``), with the residual add or the float32 store in its epilogue.
+* bfloat16 run, 9 to 64 rows and large matrices: the package's tcgen05 kernel with the weights as the instruction's rows
+  (``csrc/gemm_stream.cu``), with the same epilogues.
 * bfloat16 run, 128 rows or more: the package's tcgen05/TMA kernel (``csrc/gemm_tc.cu``: operands by TMA into
   swizzled shared memory, accumulation in tensor memory, the same epilogues).
 * bfloat16 run, between those, or an inner dimension that is no multiple of 8 (TMA needs 16-byte rows): a library
@@ -52,6 +54,20 @@ def use_skinny(M: int, N: int, K: int, norm: bool = False) -> bool:
     if norm and (K > NORM_FUSE_MAX_K or M * K > NORM_FUSE_MAX_ELEMENTS):
         return False
     return M <= SKINNY_ROWS and ops.skinny_supported(M, N, K, norm)
+
+
+# The tcgen05 kernel with the weights as the instruction's rows pays where the stream of the weights outweighs its fixed part (some 2 us
+# more than the weight-streaming kernel's or the library's): from 8 M weights on. Whole runs, ms, without / with it: 4B sizes 16 ragged
+# prompts 183 / 175, 24 short ones 99 / 70 (the weight-streaming kernel goes over the rows twice there); 8B sizes 12 prompts 80 / 74, 64 225 / 221;
+# 0.6B sizes 24 22.7 / 23.9. From 65 rows on the library is ahead (100 rows x 4,096 x 4,096 15.3 / 20.5 us), and at 16 rows the weight-streaming
+# kernel at output matrices (151,936 x 1,024 65.5 / 69.5 us).
+STREAM_MIN_WEIGHTS, STREAM_MAX_WEIGHTS_16 = 8 << 20, 128 << 20
+
+
+def use_stream(M: int, N: int, K: int, gated: bool = False) -> bool:
+    weights = (2 * N if gated else N) * K
+    return (USE_TC and 8 < M <= 64 and weights >= STREAM_MIN_WEIGHTS and (M > 16 or weights <= STREAM_MAX_WEIGHTS_16)
+            and ops.stream_supported(M, N, K))
 
 
 def use_tc(M: int, N: int, K: int) -> bool:
@@ -169,6 +185,15 @@ class Linear:
             if out is None:
                 out = ws.take((M, self.out_features), torch.float32)
             ops.gemm_f32(h, self.weight, out, stream=stream, static_weight=True)
+            return out
+        if use_stream(M, self.out_features, self.in_features):
+            if into is not None:
+                ops.gemm_stream(h, self.weight, into, "add", stream, static_weight=True)
+                return into
+            want = out_dtype or (out.dtype if out is not None else self.dtype)
+            if out is None:
+                out = ws.take((M, self.out_features), want)
+            ops.gemm_stream(h, self.weight, out, "f32" if want == torch.float32 else "bf16", stream, static_weight=True)
             return out
         if use_skinny(M, self.out_features, self.in_features):
             if into is not None:

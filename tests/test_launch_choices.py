@@ -106,3 +106,11 @@ def test_float32_product_takes_what_was_faster():
                                (600, 1024, 77, 0, 8), (128, 6144, 77, 0, 8), (64, 503, 77, 0, 0), (80, 1024, 1030, 0, 0), (1500, 503, 1030, 0, 8), (12, 32768, 1030, 0, 0)]:
         assert (choice(M, N, K, vec) == 0) == (want == 0), (M, N, K, choice(M, N, K, vec))
     assert choice(1500, 6144, 1024, 1) == 8 and choice(1500, 1024, 2048, 1) == 6 and choice(600, 503, 160, 1) == 4
+
+
+def test_large_matrices_of_some_rows_are_streamed_through_the_tensor_cores():
+    """Where whole runs were timed with and without (4B, 8B and 0.6B sizes)."""
+    for M, N, K, gated, want in [(16, 2560, 9728, False, True), (16, 9728, 2560, True, True), (24, 6144, 2560, False, True), (64, 12288, 4096, True, True),
+                                 (8, 9728, 2560, True, False), (65, 12288, 4096, True, False), (24, 1024, 3072, False, False), (24, 3072, 1024, True, False),
+                                 (16, 151936, 2560, False, False), (24, 151936, 2560, False, True)]:
+        assert linear.use_stream(M, N, K, gated) == want, (M, N, K)
