@@ -551,6 +551,12 @@ def decode_scratch_floats(n_seqs: int, heads: int, head_dim: int, splits: int) -
     return 0 if splits <= 1 else n_seqs * heads * splits * (head_dim + 2)
 
 
+def f32_on_tensor_cores(N: int, K: int, w_address: int) -> bool:
+    """Whether the 32-bit products with a matrix [N, K] run on the tensor cores (csrc/gemm_f32_tc.cu) or as FMA chains
+    (csrc/gemm_f32.cu). The two add in different orders, so the rule may look at the matrix only, never at the number of rows."""
+    return K % 4 == 0 and K >= 256 and N >= 512 and N * K >= 1 << 19 and w_address % 16 == 0
+
+
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias=None, accumulate: bool = False,
              stream=None, static_weight: bool = False, form=None) -> None:
     """out[M, N] (+)= a[M, K] @ w[N, K]^T (+ bias), all float32, every product and sum to float32. ``static_weight``: no kernel
@@ -561,7 +567,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias=None, acc
     N = w.shape[0]
     _need(w.shape[1] == K and out.shape == (M, N), "gemm_f32: shapes disagree")
     _need(a.dtype == w.dtype == out.dtype == torch.float32, "gemm_f32: float32 only")
-    if form is not None:
+    if form is not None or f32_on_tensor_cores(N, K, w.data_ptr()):
         lib().call("slb_gemm_f32_tc", _p(a), _p(w), _p(bias), _p(out), M, N, K, K, K, N, int(accumulate), int(static_weight),
                    *(int(f) for f in form or (0, 0, 0)), _p(_tc_status(a.device)), stream if stream is not None else current_stream())
         return
