@@ -569,10 +569,22 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias=None, acc
     _need(a.dtype == w.dtype == out.dtype == torch.float32, "gemm_f32: float32 only")
     if form is not None or f32_on_tensor_cores(N, K, w.data_ptr()):
         lib().call("slb_gemm_f32_tc", _p(a), _p(w), _p(bias), _p(out), M, N, K, K, K, N, int(accumulate), int(static_weight),
-                   *(int(f) for f in form or (0, 0, 0)), _p(_tc_status(a.device)), stream if stream is not None else current_stream())
+                   -1, 0.0, 1.0, *(int(f) for f in form or (0, 0, 0)), _p(_tc_status(a.device)), stream if stream is not None else current_stream())
         return
     lib().call("slb_gemm_f32", _p(a), _p(w), _p(bias), _p(out), M, N, K, K, K, N, int(accumulate), int(static_weight),
                stream if stream is not None else current_stream())
+
+
+def gemm_f32_gated(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gate=None, stream=None, static_weight: bool = False, form=None) -> None:
+    """out[M, N] = act(a @ w[:N]^T) * (a @ w[N:]^T) in float32 on the tensor cores, with the bits of ``gemm_f32`` and ``gated_act`` one after
+    the other; only for matrices that ``f32_on_tensor_cores`` sends there. ``gate``, as for the other gated products: (name, limit, alpha)."""
+    _cuda(a, w, out)
+    M, K = a.shape
+    N = out.shape[1]
+    _need(w.shape == (2 * N, K) and out.shape[0] == M, "gemm_f32_gated: shapes disagree")
+    _need(a.dtype == w.dtype == out.dtype == torch.float32, "gemm_f32_gated: float32 only")
+    lib().call("slb_gemm_f32_tc", _p(a), _p(w), None, _p(out), M, N, K, K, K, N, 0, int(static_weight), *(_gate_args(gate) or (0, 0.0, 1.0)),
+               *(int(f) for f in form or (0, 0, 0)), _p(_tc_status(a.device)), stream if stream is not None else current_stream())
 
 
 SKINNY_MODES = {"bf16": 0, "f32": 1, "add": 2, "swiglu": 3}
