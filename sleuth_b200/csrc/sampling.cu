@@ -37,6 +37,8 @@ namespace slb {
 // size share an SM, so that one works while the other stands at a barrier. 8 rows of 151,936 in us, 512 / 1,024 threads: temperature
 // alone 37 / 25, top-k 3,000 100 / 70; 64 rows: 68 / 84, 255 / 310.
 constexpr int kFewRowsThreads = 1024, kManyRowsThreads = 512;
+// Short top-k lists of many long rows (LEAN): the row is not held, and four blocks of 256 threads fit an SM, all 512 blocks of 64 rows at once.
+constexpr int kLeanThreads = 256, kLeanTopK = 64;
 constexpr double kMassScale = 1099511627776.0;  // 2^40
 
 __device__ __forceinline__ unsigned int sort_key(float v) {
@@ -401,7 +403,7 @@ __device__ int warp_walk(int n, G get, float mx, unsigned int floor_key, float m
 // maximum, is added up over the team; the step in which the weight from above reaches the target is known then, and the few
 // tokens at or above it (for top-k), or in it (for top-p without top-k), are all that the exact decision needs.
 constexpr int kHeldTokens = 20480;     // tokens a block holds
-constexpr int kBins = 1024;
+constexpr int kBins = 1024, kLeanBins = 256;
 constexpr float kBanned = -1e30f;      // logits below are no candidates' (bans set the lowest value or minus infinity)
 constexpr int kQuickList = 1024;       // candidates of a row at most
 constexpr int kSmallList = 512;        // up to this many entries are compared each with each
@@ -425,14 +427,15 @@ struct Held {
 };
 
 // Which step a value lies in; never decreasing as the value falls.
-__device__ __forceinline__ int bin_of(float v, float mx, float per) { return min(kBins - 1, (int)((mx - v) * per)); }
+template <int BINS>
+__device__ __forceinline__ int bin_of(float v, float mx, float per) { return min(BINS - 1, (int)((mx - v) * per)); }
 
 // The step at which the weight of the team's histogram, added up from step 0, first reaches `target`, or -1; `above` = the
 // weight of the steps before it. LIMBS 1: counts; 3: masses in parts of 16, 16 and 9 bits (shared memory adds 32-bit words).
-template <int LIMBS, int THREADS>
+template <int LIMBS, int THREADS, int BINS>
 __device__ int find_bin(Team& team, const unsigned int* hist, unsigned long long target, unsigned long long& above) {
   SampleShared& sh = *team.sh;
-  constexpr int kPer = kBins / THREADS;
+  constexpr int kPer = BINS / THREADS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned long long h[kPer], mine = 0ull;
 #pragma unroll
@@ -441,7 +444,7 @@ __device__ int find_bin(Team& team, const unsigned int* hist, unsigned long long
 #pragma unroll
     for (int l = 0; l < LIMBS; ++l) {
       unsigned long long part = 0ull;
-      for (int c = 0; c < kSampleTeam; ++c) part += team.cluster.map_shared_rank(hist, c)[l * kBins + threadIdx.x * kPer + j];
+      for (int c = 0; c < kSampleTeam; ++c) part += team.cluster.map_shared_rank(hist, c)[l * BINS + threadIdx.x * kPer + j];
       t += part << (16 * l);
     }
     h[j] = t;
@@ -545,7 +548,11 @@ __device__ int gather_lists(Team& team, int* tokens, float* values, int* all_tok
   return n;
 }
 
-template <int THREADS>
+// LEAN: what the block keeps of its part of the row is one maximum a thread. The step in which the k-th largest of the row's thread
+// maxima lies bounds the k-th largest value from below, and tightly (the largest values mostly fall to different threads); the values at or
+// above it are collected in a second read of the row, which L2 then holds. One atomic addition a thread in place of one a token, a quarter of
+// the steps, and no shared memory but the lists.
+template <int THREADS, bool LEAN>
 __global__ void __cluster_dims__(kSampleTeam, 1, 1) __launch_bounds__(THREADS, 1024 / THREADS)
 sample_kernel(const float* __restrict__ logits, long long ld, int limit, float temperature, int top_k, float top_p,
               float min_p, const float* __restrict__ uniform, int* __restrict__ out) {
@@ -559,7 +566,8 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
   extern __shared__ __align__(16) unsigned long long dynamic[];
   unsigned long long* warp_hist = dynamic;         // general path: [warps][256]
   float4* held = reinterpret_cast<float4*>(dynamic);                                        // quick path: [kHeld][threads]
-  unsigned int* bins = reinterpret_cast<unsigned int*>(dynamic + kHeldTokens / 2);          // quick path: [3][kBins]
+  constexpr int BINS = LEAN ? kLeanBins : kBins, kBinsAt = LEAN ? kQuickList / 2 + kWarps * 256 : kHeldTokens / 2;      // LEAN: behind the joined list's values and what is worked out on it
+  unsigned int* bins = reinterpret_cast<unsigned int*>(dynamic + kBinsAt);                  // quick path: [LEAN ? 1 : 3][BINS]
   Team team{cg::this_cluster(), &sh, false, kSampleTeam};
   const int r = blockIdx.x / kSampleTeam, rank = (int)team.cluster.block_rank();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -577,10 +585,10 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
   bool listed = false, cut = false;      // cut: floor_key says already what top-p leaves
   int n_listed = 0;
 
-  const bool count_first = top_k > 0 && top_k < limit;
+  const bool count_first = LEAN || (top_k > 0 && top_k < limit);
   const int chunks = (raw.n + 128 * kWarps - 1) / (128 * kWarps);
   Held<THREADS> mine{held + threadIdx.x, part_begin + warp * chunks * 128, min(part_end, part_begin + (warp + 1) * chunks * 128), lane};
-  bool quick = per_block <= kHeldTokens && (count_first ? top_k <= kQuickList : top_p < 1.0f);      // the same for all blocks of a row
+  bool quick = (LEAN || per_block <= kHeldTokens) && (count_first ? top_k <= kQuickList : top_p < 1.0f);      // the same for all blocks of a row
   if (quick) {
     // the one read of the row; the largest value, bounds from below, and whether anything is no number. Banned tokens (minus
     // infinity, or the lowest value) count for no bound.
@@ -588,9 +596,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
     float most = -INFINITY, least = INFINITY;
     bool bad = false;
     auto allowed = [](float v) { return v < kBanned ? INFINITY : v; };
-#pragma unroll 5
-    for (int c = 0; mine.begin + 128 * c < mine.end; ++c) {
-      const int t = mine.begin + 128 * c + 4 * lane;
+    auto four_at = [&](int t) {
       float4 v = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
       if (t + 3 < mine.end && aligned) {
         v = *reinterpret_cast<const float4*>(row + t);
@@ -600,10 +606,15 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
         if (t + 2 < mine.end) v.z = row[t + 2];
         if (t + 3 < mine.end) v.w = row[t + 3];
       }
+      return v;
+    };
+#pragma unroll 5
+    for (int c = 0; mine.begin + 128 * c < mine.end; ++c) {
+      const float4 v = four_at(mine.begin + 128 * c + 4 * lane);
       bad = bad || v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w;
       most = fmaxf(most, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
       if (!count_first) least = fminf(least, fminf(fminf(allowed(v.x), allowed(v.y)), fminf(allowed(v.z), allowed(v.w))));
-      mine.mine[c * THREADS] = v;
+      if constexpr (!LEAN) mine.mine[c * THREADS] = v;
     }
     // At least as many values as there are warps (threads) with a maximum of their own reach the smallest of those maxima.
     const float warp_most = warp_max(most);
@@ -615,7 +626,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
     const int any_bad = __syncthreads_or(bad ? 1 : 0);
     const int f = team.flip();
     if (threadIdx.x == 0) { sh.x.max[f] = most_block; sh.x.low = low_block; sh.x.bad = any_bad; sh.count = 0; }
-    for (int i = threadIdx.x; i < 3 * kBins; i += blockDim.x) bins[i] = 0u;
+    for (int i = threadIdx.x; i < (LEAN ? 1 : 3) * BINS; i += blockDim.x) bins[i] = 0u;
     team.cluster.sync();
     float row_most = -INFINITY, row_low = INFINITY;
     for (int c = 0; c < kSampleTeam; ++c) {
@@ -625,22 +636,40 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
       quick = quick && x->bad == 0;
     }
     const float size = fmaxf(fabsf(row_most), fabsf(row_low));
-    const float width = (row_most - row_low) / kBins;
+    const float width = (row_most - row_low) / BINS;
     quick = quick && size < 1e30f;      // (not for infinities)
     if (count_first) {
       // Candidates are taken one step below the k-th value's: a step must be wider than what rounds to the same quotient.
       quick = quick && width > 1e-5f * size && width > 1e-30f * temperature && temperature > 1e-30f;
       if (quick) {
-        const float per = (kBins - 0.5f) / (row_most - row_low);
-        mine.each([&](int, float x) { if (x >= row_low) atomicAdd(&bins[bin_of(x, row_most, per)], 1u); });
+        const float per = (BINS - 0.5f) / (row_most - row_low);
+        if constexpr (LEAN) {
+          if (most >= row_low) atomicAdd(&bins[bin_of<BINS>(most, row_most, per)], 1u);
+        } else {
+          mine.each([&](int, float x) { if (x >= row_low) atomicAdd(&bins[bin_of<BINS>(x, row_most, per)], 1u); });
+        }
         team.cluster.sync();
         unsigned long long above;
-        const int bin = find_bin<1, THREADS>(team, bins, (unsigned long long)top_k, above);
-        quick = bin >= 0 && bin < kBins - 2;
+        const int bin = find_bin<1, THREADS, BINS>(team, bins, (unsigned long long)top_k, above);
+        quick = bin >= 0 && bin < BINS - 2;
         if (quick) {
-          mine.each([&](int t, float x) {
-            if (x >= row_low && bin_of(x, row_most, per) <= bin + 1) keep_candidate(sh, cand_token, cand_value, t, x);
-          });
+          auto keep = [&](int t, float x) {
+            if (x >= row_low && bin_of<BINS>(x, row_most, per) <= bin + 1) keep_candidate(sh, cand_token, cand_value, t, x);
+          };
+          if constexpr (LEAN) {
+#pragma unroll 5
+            for (int c = 0; mine.begin + 128 * c < mine.end; ++c) {      // (beyond the end: minus infinity, below every bound)
+              const int t = mine.begin + 128 * c + 4 * lane;
+              const float4 v = four_at(t);
+              if (fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)) < row_low) continue;
+              keep(t, v.x);
+              keep(t + 1, v.y);
+              keep(t + 2, v.z);
+              keep(t + 3, v.w);
+            }
+          } else {
+            mine.each(keep);
+          }
           int* all_token = reinterpret_cast<int*>(bins);
           float* all_value = reinterpret_cast<float*>(dynamic);      // the held row is not needed any more where the list fits
           const int n = gather_lists(team, cand_token, cand_value, all_token, all_value, rank, kQuickList);
@@ -687,7 +716,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
           const unsigned long long m = mass_of(v, mx);
           part += m;
           if (v >= lowest) {
-            unsigned int* at = bins + bin_of(v, mx, per);
+            unsigned int* at = bins + bin_of<kBins>(v, mx, per);
             atomicAdd(at, (unsigned int)(m & 0xffffull));
             atomicAdd(at + kBins, (unsigned int)((m >> 16) & 0xffffull));
             atomicAdd(at + 2 * kBins, (unsigned int)(m >> 32));
@@ -697,12 +726,12 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
         unsigned long long target = (unsigned long long)ceil((double)top_p * (double)total), above;
         if (target < 1ull) target = 1ull;
         if (target > total) target = total;
-        const int bin = find_bin<3, THREADS>(team, bins, target, above);
+        const int bin = find_bin<3, THREADS, kBins>(team, bins, target, above);
         quick = bin >= 0 && bin < kBins - 1;
         if (quick) {
           mine.each([&](int t, float x) {
             const float v = x / temperature;
-            if (v >= lowest && bin_of(v, mx, per) == bin) keep_candidate(sh, cand_token, cand_value, t, v);
+            if (v >= lowest && bin_of<kBins>(v, mx, per) == bin) keep_candidate(sh, cand_token, cand_value, t, v);
           });
           // block 0 has the histogram's place for the list and what is worked out on it (it still holds its part of the row)
           int* all_token = reinterpret_cast<int*>(bins);
@@ -977,6 +1006,9 @@ extern "C" int slb_argmax_static_max_rows() { return kStaticArgmaxRows; }
 // Threads of a block for so many rows: all an SM takes while every block of a row's eight has an SM to itself.
 extern "C" int slb_sample_threads(int rows) { return (long long)rows * kSampleTeam <= sm_count() ? kFewRowsThreads : kManyRowsThreads; }
 
+// Whether rows go through the lean form.
+extern "C" int slb_sample_lean(int rows, int limit, int top_k) { return top_k > 0 && top_k <= kLeanTopK && top_k < limit && limit >= 98304 && rows > 32; }
+
 extern "C" int slb_sample(const float* logits, long long ld, int rows, int limit, float temperature, int top_k,
                           float top_p, float min_p, const float* uniform, int* out, void* stream) {
   SLB_REQUIRE(rows >= 0 && limit > 0 && ld >= limit, "sample: rows=%d limit=%d ld=%lld", rows, limit, ld);
@@ -986,14 +1018,18 @@ extern "C" int slb_sample(const float* logits, long long ld, int rows, int limit
               (double)top_p, (double)min_p);
   if (rows == 0) return 0;
   // the quick path's row and histogram; the general path's warp histograms and candidates lie in the same place
-  constexpr size_t hist_bytes = kHeldTokens * sizeof(float) + 3 * kBins * sizeof(unsigned int);
+  constexpr int hist_bytes = kHeldTokens * sizeof(float) + 3 * kBins * sizeof(unsigned int);
+  constexpr int lean_bytes = kLeanThreads / 32 * 2048 + 2 * kCandidates * sizeof(int);
   static_assert(kMostWarps * 256 * sizeof(unsigned long long) + 2 * kCandidates * sizeof(int) <= kHeldTokens * sizeof(float), "the general path's place");
-  const bool few = slb_sample_threads(rows) == kFewRowsThreads;
-  const auto kernel = few ? sample_kernel<kFewRowsThreads> : sample_kernel<kManyRowsThreads>;
-  static std::atomic<unsigned long long> allowed[2];
-  const cudaError_t e = allow_shared((const void*)kernel, (int)hist_bytes, allowed[few]);
-  if (e != cudaSuccess) return fail(2, "sample: cannot reserve %d bytes of shared memory: %s", (int)hist_bytes, cudaGetErrorString(e));
-  launch(kernel, dim3(rows * kSampleTeam), dim3(few ? kFewRowsThreads : kManyRowsThreads), hist_bytes, (cudaStream_t)stream, logits, ld, limit, temperature, top_k, top_p,
+  static_assert(2 * kCandidates * sizeof(int) <= kLeanThreads / 32 * 2048, "the general path's joined list");
+  static_assert(kQuickList * 4 + kLeanThreads / 32 * 2048 + kQuickList * 4 <= lean_bytes, "the lean path's place (the joined list's tokens lie where the steps were)");
+  const bool lean = slb_sample_lean(rows, limit, top_k) != 0, few = slb_sample_threads(rows) == kFewRowsThreads;
+  const auto kernel = lean ? sample_kernel<kLeanThreads, true> : few ? sample_kernel<kFewRowsThreads, false> : sample_kernel<kManyRowsThreads, false>;
+  const int threads = lean ? kLeanThreads : few ? kFewRowsThreads : kManyRowsThreads, bytes = lean ? lean_bytes : hist_bytes;
+  static std::atomic<unsigned long long> allowed[3];
+  const cudaError_t e = allow_shared((const void*)kernel, bytes, allowed[lean ? 2 : few ? 1 : 0]);
+  if (e != cudaSuccess) return fail(2, "sample: cannot reserve %d bytes of shared memory: %s", bytes, cudaGetErrorString(e));
+  launch(kernel, dim3(rows * kSampleTeam), dim3(threads), (size_t)bytes, (cudaStream_t)stream, logits, ld, limit, temperature, top_k, top_p,
          min_p, uniform, out);
   return check_launch("sample");
 }
