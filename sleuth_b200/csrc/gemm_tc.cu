@@ -643,17 +643,18 @@ static int launch_tc(const CUtensorMap& mx, const CUtensorMap& mw, const TcArgs&
 }
 
 // Whether two blocks share tiles of 256 rows. SLEUTH_B200_GEMM_PAIR=0/1 decides for every product of at least 256
-// rows; otherwise pairs take the products of many rows, where they were measured faster (Qwen3-0.6B shapes, one
-// B200: level at 2,048 rows, 3 to 12 % faster from 4,096 on, slower below 2,048). The q/k/v form, whose epilogue
-// weighs more than its products, gained nothing below 16,384 rows and stays with single blocks.
-static bool pair_pays(int M) {
+// rows; otherwise pairs take the products of many rows and, from 512 rows on, those with large matrices (single blocks / pairs, us: 512 rows x
+// 2,560 x 9,728 45.0 / 40.9, 1,024 80.7 / 71.6, 2,048 x 4,096 x 12,288 168 / 146; 512 x 1,024 x 3,072 16.3 / 18.4, 2,048 20.4 / 21.5,
+// 4,096 42.0 / 40.9; 256 x 2,560 x 9,728 34.8 / 38.9). The q/k/v form, whose epilogue weighs more than its products, gained nothing below
+// 16,384 rows and stays with single blocks.
+static bool pair_pays(int M, long long weights) {
   static int forced = -2;
   if (forced == -2) {
     const char* e = getenv("SLEUTH_B200_GEMM_PAIR");
     forced = e ? (e[0] == '0' ? 0 : 1) : -1;
   }
   if (M < 256) return false;
-  return forced >= 0 ? forced != 0 : M >= 4096;
+  return forced >= 0 ? forced != 0 : M >= 4096 || (M >= 512 && weights >= 8ll << 20);
 }
 
 }  // namespace slb
@@ -701,7 +702,7 @@ static int gemm_tc_run(const void* X, const void* W, void* C, int M, int N, int 
   // within one round a narrower tile is a little faster (more SMs stream operands), while a second round costs
   // nearly twice (768 rows: 17 us with 96 tiles of 64 columns, 28 us with 192 of 32). When even the widest tile
   // needs several rounds, the widest is the most efficient.
-  const bool pair = pair_pays(M);
+  const bool pair = pair_pays(M, (gated ? 2ll : 1ll) * N * K);
   const long long m_tiles = pair ? (M + 255) / 256 : (M + 127) / 128;
   const int sms = sm_count(), workers = pair ? sms / 2 : sms;
   int bn = 256;
