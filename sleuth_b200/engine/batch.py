@@ -67,6 +67,7 @@ class MetaStager:
         self.cap = 0
         self.dev = None
         self.hosts, self.events = [], []
+        self._host_np, self._plans = [], {}
         self.turn = 0
         self.generation = 0
         self.last_upload_bytes = 0
@@ -85,7 +86,9 @@ class MetaStager:
             self.dev[:self.FEED].copy_(old[:self.FEED])
             torch.cuda.synchronize(self.device)
         self.hosts = [torch.zeros(capacity, dtype=torch.int32).pin_memory() for _ in range(self.RING)]
+        self._host_np = [h.numpy() for h in self.hosts]
         self.events = [None] * self.RING
+        self._plans = {}
         self.generation += 1
 
     def layout(self, n: int, T: int, W: int, n_floats: int):
@@ -99,6 +102,26 @@ class MetaStager:
             off[f"table{g}"] = (o, n * self.stride)
             o += _round(n * self.stride)
         return off, o
+
+    def _plan(self, n: int, T: int, W: int, nf: int, via_feed: bool):
+        """Offsets, total, device views and copy ranges of a batch of these sizes: they depend on the sizes and the buffers alone, so
+        the last few dozen sizes' are kept until the buffers are replaced."""
+        key = (n, T, W, nf, via_feed)
+        plan = self._plans.get(key)
+        if plan is None:
+            off, total = self.layout(n, T, W, nf)
+            if total > self.cap:
+                self._grow(max(total, 2 * self.cap))
+            if len(self._plans) >= 64:
+                self._plans.clear()
+            view = {name: self.dev[o:o + size] for name, (o, size) in off.items()}
+            fixed = dict(token_ids=self.feed if via_feed else view["token_ids"], ids_map=view["ids_map"] if via_feed else None,
+                         floats=view["floats"].view(torch.float32) if nf else None,
+                         **{name: view[name] for name in ("tok_seq", "tok_pos", "seq_start", "past", "counts", "slots", "rows")})
+            tables = [view[f"table{g}"].view(n, self.stride) for g in range(self.n_groups)]
+            copies = {first: (self.dev[first:total], [h[first:total] for h in self.hosts]) for first in (0, self.FEED)}
+            plan = self._plans[key] = (off, total, fixed, tables, copies)
+        return plan
 
     @property
     def feed(self) -> torch.Tensor:
@@ -118,14 +141,12 @@ class MetaStager:
         if tokens is None and feed_map is None:
             raise ValueError("a step needs its tokens: from the host, or a map into the device-side feed")
         nf = 0 if floats is None else int(floats.shape[0])
-        off, total = self.layout(n, T, W, nf)
-        if total > self.cap:
-            self._grow(max(total, 2 * self.cap))
+        off, total, fixed, views, copies = self._plan(n, T, W, nf, via_feed)
         i = self.turn
         self.turn = (self.turn + 1) % self.RING
         if self.events[i] is not None:
             self.events[i].synchronize()
-        host = self.hosts[i].numpy()
+        host = self._host_np[i]
 
         counts_a = np.asarray(counts, dtype=np.int32)
         pasts_a = np.asarray(pasts, dtype=np.int32)
@@ -161,25 +182,20 @@ class MetaStager:
             o, size = off[f"table{g}"]
             host[o:o + size] = t.reshape(-1)
 
-        st = stream if stream is not None else torch.cuda.current_stream(self.device)
-        with torch.cuda.stream(st):
-            self.dev[first:total].copy_(self.hosts[i][first:total], non_blocking=True)
-            self.last_upload_bytes = 4 * (total - first)
-            ev = torch.cuda.Event()
-            ev.record(st)
-        self.events[i] = ev
-
-        def view(name):
-            o, size = off[name]
-            return self.dev[o:o + size]
-
-        fl = view("floats").view(torch.float32) if nf else None
+        current = torch.cuda.current_stream(self.device)
+        st = stream if stream is not None else current
+        on_dev, on_host = copies[first]
+        self.last_upload_bytes = 4 * (total - first)
+        if self.events[i] is None:
+            self.events[i] = torch.cuda.Event()
+        if st == current:
+            on_dev.copy_(on_host[i], non_blocking=True)
+        else:
+            with torch.cuda.stream(st):
+                on_dev.copy_(on_host[i], non_blocking=True)
+        self.events[i].record(st)
         return StepBatch(
-            n=n, T=T, stream=st.cuda_stream, token_ids=self.feed if via_feed else view("token_ids"),
-            ids_map=view("ids_map") if via_feed else None, tok_seq=view("tok_seq"),
-            tok_pos=view("tok_pos"), seq_start=view("seq_start"), past=view("past"), counts=view("counts"),
-            slots=view("slots"), rows=view("rows"),
-            tables=[view(f"table{g}").view(n, self.stride) for g in range(self.n_groups)], floats=fl,
+            n=n, T=T, stream=st.cuda_stream, tables=list(views), **fixed,
             host_counts=list(map(int, counts)), host_past=list(map(int, pasts)), host_slots=list(map(int, slots)),
             max_count=int(counts_a.max()) if n else 0, max_len=int((pasts_a + counts_a).max()) if n else 0,
             fresh=bool(n) and not bool(pasts_a.any()))
