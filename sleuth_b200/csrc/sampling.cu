@@ -17,7 +17,7 @@
 //
 // Cost: a row's eighth is read once into shared memory, and one histogram over values between a lower bound and the row's
 // maximum finds the short list that holds the answer (the quick path, below). 64 rows of 151,936, top-k 50, top-p 0.9: 247 us
-// before (six passes over the row, four of them with 64 KB of histograms to clear and add up), 55 us now. Calls and rows for
+// before (six passes over the row, four of them with 64 KB of histograms to clear and add up), 55 us with the row held, 39 us with thread maxima (LEAN, below). Calls and rows for
 // which that cannot work (neither top-k nor top-p, top-k beyond the list, rows longer than the blocks hold, NaN or infinite
 // maxima, more candidates than fit) take the general path: a radix descent over the sort keys, eight bits a pass.
 #include <math.h>
@@ -37,8 +37,10 @@ namespace slb {
 // size share an SM, so that one works while the other stands at a barrier. 8 rows of 151,936 in us, 512 / 1,024 threads: temperature
 // alone 37 / 25, top-k 3,000 100 / 70; 64 rows: 68 / 84, 255 / 310.
 constexpr int kFewRowsThreads = 1024, kManyRowsThreads = 512;
-// Short top-k lists of many long rows (LEAN): the row is not held, and four blocks of 256 threads fit an SM, all 512 blocks of 64 rows at once.
-constexpr int kLeanThreads = 256, kLeanTopK = 64;
+// Short top-k lists of many rows (LEAN): the row is not held, and four blocks of 256 threads fit an SM, all 512 blocks of 64 rows at once.
+// us, held / lean: 18 rows of 151,936, k 50 45 / 31, 64 rows 68 / 39, of 8,000 49 / 23; 64 rows of 151,936, k 200 96 / 74, k 400 150 / 193 (the list's
+// own work wants more threads); 8 rows, k 50 27 / 31.
+constexpr int kLeanThreads = 256, kLeanTopK = 200, kLeanRows = 18, kLeanTokens = 8000;
 constexpr double kMassScale = 1099511627776.0;  // 2^40
 
 __device__ __forceinline__ unsigned int sort_key(float v) {
@@ -1007,7 +1009,7 @@ extern "C" int slb_argmax_static_max_rows() { return kStaticArgmaxRows; }
 extern "C" int slb_sample_threads(int rows) { return (long long)rows * kSampleTeam <= sm_count() ? kFewRowsThreads : kManyRowsThreads; }
 
 // Whether rows go through the lean form.
-extern "C" int slb_sample_lean(int rows, int limit, int top_k) { return top_k > 0 && top_k <= kLeanTopK && top_k < limit && limit >= 98304 && rows > 32; }
+extern "C" int slb_sample_lean(int rows, int limit, int top_k) { return top_k > 0 && top_k <= kLeanTopK && limit >= kLeanTokens && rows >= kLeanRows; }
 
 extern "C" int slb_sample(const float* logits, long long ld, int rows, int limit, float temperature, int top_k,
                           float top_p, float min_p, const float* uniform, int* out, void* stream) {
