@@ -167,7 +167,7 @@ __device__ __forceinline__ void ft_add_up(const GemmF32TcArgs& a, const float* s
   }
 }
 
-// GATED: a tile is 64 gate rows of W and the 64 up rows that match them; the other way round of the features is plain.
+// GATED: a tile is 64 gate rows of W and the 64 up rows that match them. SPLIT: K is shared by a cluster, which has one tile.
 template <int NT, int R, int WORKERS, bool SPLIT, bool GATED>
 __global__ void __launch_bounds__(FtShape<NT, WORKERS>::kThreads, WORKERS == 8 ? 2 : 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GemmF32TcArgs a) {

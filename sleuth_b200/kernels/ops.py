@@ -788,7 +788,9 @@ def gemm_tc_check(device) -> None:
         raise RuntimeError(f"a wait inside a tcgen05 kernel gave up (code {code}; product: 1 = free stage, 2 = loaded "
                            f"stage, 3 = finished accumulator, 4 = drained accumulator; attention: 20 = shared memory "
                            f"misaligned, 21-27 = producer and MMA waits, 28-32 = softmax waits; persistent single-token kernel: 40 = grid "
-                           f"barrier, 41 = a ring slot that did not fill, 42 = a ring slot that did not empty; 99 = the wait "
+                           f"barrier, 41 = a ring slot that did not fill, 42 = a ring slot that did not empty; 32-bit product: 61 = free chunk, 62 = split "
+                           f"chunk, 63 = loaded chunk, 64 = multiplied chunk, 65 = up values; streamed product: 71 = free slice, 72 = loaded slice, "
+                           f"73 = finished sums; 99 = the wait "
                            f"probe of the tests); "
                            f"its results are not valid")
 
