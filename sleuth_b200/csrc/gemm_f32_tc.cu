@@ -492,7 +492,9 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemm_f32_few_kernel(const __gr
   tc_fence_after();
   const uint32_t tmem = warp != 17 ? *tmem_slot : 0u, tA = tmem + kFewBuffers * kFewTokens;
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // (no sums go to a block that has not begun)
-  pdl_launch_dependents();
+  // Not by the loading warp, which has not waited for the allocation: a block of the next kernel that found this one's tensor memory still
+  // free would take it and then wait for this grid, which could not go on without it.
+  if (warp != 17) pdl_launch_dependents();
   const int mine = kFtFeatures / a.splits, half = mine / 2;                  // features of an output share
 
   if (warp == 17) {
