@@ -23,6 +23,7 @@ struct GsArgs {
   int up_row0;          // kGsGated: first up row of W
   int early;            // no kernel writes W: it is fetched before the wait for the kernel in front
   int splits;           // blocks of a cluster
+  int four;             // C's rows take four values at a time (16 bytes of float32, 8 of bfloat16); else one by one
   GateAct gate;
   int* status;
 };
@@ -88,7 +89,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   auto place = [&](int i, int& t, int& f, bool& four) {
     t = rank + i / per * a.splits;
     f = i % per * 4;
-    four = n0 + f + 4 <= a.N && a.ldc % 4 == 0;
+    four = a.four && n0 + f + 4 <= a.N;
     return i < items && n0 + f < a.N;
   };
   auto old_values = [&](int i) {
@@ -282,7 +283,7 @@ extern "C" int slb_gemm_stream(const void* X, const void* W, void* C, int M, int
                                int static_weight, int splits, int* status, void* stream) {
   SLB_REQUIRE(slb_gemm_stream_supported(M, N, K), "gemm_stream: M=%d N=%d K=%d is not taken (1 to 128 rows, K a multiple of 8 and at least 64)", M, N, K);
   SLB_REQUIRE(mode >= 0 && mode <= 3 && ldc >= N && status != nullptr && kind >= kGateSilu && kind <= kGateLast, "gemm_stream: mode=%d ldc=%d N=%d kind=%d", mode, ldc, N, kind);
-  SLB_REQUIRE(((uintptr_t)X % 16 == 0) && ((uintptr_t)W % 16 == 0) && ((uintptr_t)C % 16 == 0), "gemm_stream: X, W and C must be 16-byte aligned");
+  SLB_REQUIRE(((uintptr_t)X % 16 == 0) && ((uintptr_t)W % 16 == 0), "gemm_stream: X and W must be 16-byte aligned");
   SLB_REQUIRE(splits >= 0 && splits <= 8 && splits <= (K + kGsK - 1) / kGsK, "gemm_stream: %d blocks for K=%d", splits, K);
   const bool gated_mode = mode == kGsGated;
   const int cols = gated_mode ? kGsFeatures / 2 : kGsFeatures, tiles = (N + cols - 1) / cols;
@@ -292,7 +293,9 @@ extern "C" int slb_gemm_stream(const void* X, const void* W, void* C, int M, int
   if (rc) return rc;
   rc = gs_map(&mx, X, M, K, nt);
   if (rc) return rc;
-  const GsArgs a{C, M, N, K, ldc, mode, N, static_weight, splits ? splits : gs_splits(tiles, K), GateAct{kind, limit, alpha}, status};
+  const int width = mode == kGsF32 || mode == kGsAddF32 ? 4 : 2;
+  const GsArgs a{C, M, N, K, ldc, mode, N, static_weight, splits ? splits : gs_splits(tiles, K), ldc % 4 == 0 && (uintptr_t)C % (4 * width) == 0,
+                 GateAct{kind, limit, alpha}, status};
   cudaStream_t s = (cudaStream_t)stream;
   switch (nt) {
     case 16: return launch_gs<16>(mw, mx, a, tiles, s);

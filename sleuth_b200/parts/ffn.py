@@ -62,9 +62,9 @@ class GatedMLP(Part):
         if not self.fused:
             gu = self.gate_up.forward(h, ws=ws, stream=b.stream)
             ops.gated_act(gu, act, self.spec.activation, b.stream, self.spec.limit, self.spec.alpha)
-        elif self.ctx.dtype == torch.bfloat16 and linear.use_stream(T, self.spec.intermediate, self.spec.hidden, gated=True):
-            ops.gemm_stream(h.tensor() if isinstance(h, Normed) else h, self.gate_up.weight, act, "swiglu", b.stream, gate=self.gate,
-                            static_weight=True)
+        elif (self.ctx.dtype == torch.bfloat16 and linear.use_stream(T, self.spec.intermediate, self.spec.hidden, gated=True)
+              and linear.streams(rows := h.tensor() if isinstance(h, Normed) else h, self.gate_up.weight, gated=True)):
+            ops.gemm_stream(rows, self.gate_up.weight, act, "swiglu", b.stream, gate=self.gate, static_weight=True)
         elif self.ctx.dtype == torch.bfloat16 and linear.use_skinny(T, self.spec.intermediate, self.spec.hidden):
             # norm in the product's prologue (when handed the stream), activation in its epilogue
             if (isinstance(h, Normed) and h.gain is not None and FUSE_NORM and self.silu

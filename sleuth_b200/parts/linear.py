@@ -71,6 +71,14 @@ def use_stream(M: int, N: int, K: int, gated: bool = False) -> bool:
             and ops.stream_supported(M, N, K))
 
 
+def streams(h: torch.Tensor, weight: torch.Tensor, gated: bool = False) -> bool:
+    """Whether the product of these goes to that kernel, which reads rows that lie one behind the other from 16-byte boundaries on; what
+    does not lie so stays with the kernels that took it before."""
+    rows = weight.shape[0]
+    return (use_stream(h.shape[0], rows // 2 if gated else rows, weight.shape[1], gated) and h.is_contiguous()
+            and not h.data_ptr() % 16 and not weight.data_ptr() % 16)
+
+
 def use_tc(M: int, N: int, K: int) -> bool:
     return USE_TC and M >= TC_ROWS and ops.tc_supported(M, N, K)
 
@@ -187,7 +195,7 @@ class Linear:
                 out = ws.take((M, self.out_features), torch.float32)
             ops.gemm_f32(h, self.weight, out, stream=stream, static_weight=True)
             return out
-        if use_stream(M, self.out_features, self.in_features):
+        if streams(h, self.weight):
             if into is not None:
                 ops.gemm_stream(h, self.weight, into, "add", stream, static_weight=True)
                 return into

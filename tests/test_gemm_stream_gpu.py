@@ -50,3 +50,37 @@ def test_other_gates():
         ops().gemm_stream(x, w, out, "swiglu", gate=gate)
         ops().gated_act(full.bfloat16(), plain, gate[0], None, gate[1], gate[2])
         torch.testing.assert_close(out.float(), plain.float(), rtol=3e-2, atol=3e-2)
+
+
+@pytest.mark.parametrize("mode", ["bf16", "f32", "add", "swiglu"])
+@pytest.mark.parametrize("M,N,K,offset", [(13, 131, 576, 1), (64, 132, 520, 1), (20, 260, 576, 2), (33, 1027, 1024, 3)])
+def test_results_that_lie_off_16_bytes(mode, M, N, K, offset):
+    """A result at any element's address, rows of any length: the same bits as in a buffer of its own."""
+    g = torch.Generator().manual_seed(N + offset)
+    x = torch.randn(M, K, generator=g).bfloat16().to(DEV)
+    w = (torch.randn((2 if mode == "swiglu" else 1) * N, K, generator=g) / 16).bfloat16().to(DEV)
+    dtype = torch.bfloat16 if mode in ("bf16", "swiglu") else torch.float32
+    own = torch.full((M, N), 0.5, device=DEV, dtype=dtype)
+    around = torch.full((M * N + offset + 8,), 0.5, device=DEV, dtype=dtype)
+    ops().gemm_stream(x, w, own, mode, splits=2)
+    ops().gemm_stream(x, w, around[offset:offset + M * N].view(M, N), mode, splits=2)
+    assert torch.equal(around[offset:offset + M * N].view(M, N), own)
+    assert (around[:offset] == 0.5).all() and (around[offset + M * N:] == 0.5).all()
+
+
+def test_chunked_step_with_an_odd_vocabulary():
+    """A step cut into chunks whose later logits begin at a row off 16 bytes gives the logits of the uncut step."""
+    from sleuth_b200.engine.engine import Engine
+    vocab = 8209
+    cfg = {"architectures": ["Qwen3ForCausalLM"], "model_type": "qwen3", "vocab_size": vocab, "hidden_size": 1024, "intermediate_size": 256,
+           "num_hidden_layers": 1, "num_attention_heads": 4, "num_key_value_heads": 2, "head_dim": 64, "rope_theta": 1e4, "rms_norm_eps": 1e-6,
+           "attention_bias": False, "tie_word_embeddings": False, "max_position_embeddings": 256}
+    gen = torch.Generator().manual_seed(2)
+    prompts = [torch.randint(0, vocab, (50,), generator=gen).tolist() for _ in range(30)]
+    logits = []
+    for most in (8192, 50 * 13, 50 * 17):
+        eng = Engine.from_config(cfg, seed=3, dtype="bf16", max_seq_len=64, max_tokens=30 * 64, max_sequences=32, max_step_tokens=most)
+        logits.append(eng.step([(s, p, (len(p) - 1,)) for s, p in zip(eng.open(30), prompts)]).cpu())
+    for other in logits[1:]:
+        # the layers' products run on other kernels for other numbers of rows: bfloat16 roundings of one layer
+        torch.testing.assert_close(other, logits[0], rtol=0, atol=0.03 * float(logits[0].abs().max()))

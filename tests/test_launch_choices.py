@@ -4,6 +4,7 @@ attention cuts a sequence into, and when a product normalises its own input."""
 import ctypes
 
 import pytest
+import torch
 
 from sleuth_b200.kernels import ops
 from sleuth_b200.parts import linear
@@ -114,3 +115,14 @@ def test_large_matrices_of_some_rows_are_streamed_through_the_tensor_cores():
                                  (8, 9728, 2560, True, False), (65, 12288, 4096, True, False), (24, 1024, 3072, False, False), (24, 3072, 1024, True, False),
                                  (16, 151936, 2560, False, False), (24, 151936, 2560, False, True)]:
         assert linear.use_stream(M, N, K, gated) == want, (M, N, K)
+
+
+def test_rows_that_lie_otherwise_stay_with_the_other_kernels():
+    """The streaming kernel reads rows one behind the other from 16-byte boundaries on; strided rows and odd addresses go on as before."""
+    w = torch.empty(4096 * 2560 + 8, dtype=torch.bfloat16)
+    weight, shifted = w[:4096 * 2560].view(4096, 2560), w[1:4096 * 2560 + 1].view(4096, 2560)
+    wide = torch.empty(40, 2568, dtype=torch.bfloat16)
+    h = torch.empty(40 * 2560 + 1, dtype=torch.bfloat16)
+    assert linear.streams(h[:-1].view(40, 2560), weight) and linear.streams(h[:-1].view(40, 2560), weight, gated=True)
+    assert not linear.streams(h[1:].view(40, 2560), weight) and not linear.streams(h[:-1].view(40, 2560), shifted)
+    assert not linear.streams(wide[:, :2560], weight)
