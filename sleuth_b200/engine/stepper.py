@@ -42,6 +42,8 @@ class StepEntry:
 
 
 class Stepper:
+    STATUS_EVERY = 8
+
     def __init__(self, model, cache, device, max_len: int | None = None, max_step_tokens: int = 8192,
                  use_graphs: bool = True, max_graph_batch: int = 256):
         self.model, self.cache = model, cache
@@ -63,6 +65,7 @@ class Stepper:
         self.check_kernels = os.environ.get("SLEUTH_B200_CHECK", "0") == "1"   # read the kernels' status word after each step
         self._status_host: torch.Tensor | None = None     # pinned copy of the kernels' status word, read one step late
         self._status_event = None
+        self._steps_unseen = 0              # single-token steps since the word was last copied
         self._graph_own: dict = {}          # own kernel launches captured in each graph
         self.graph_kernel_launches = 0      # own kernel launches replayed through graphs so far
         ops.lib()   # build or load the kernels now; fail here, loudly, if that is impossible
@@ -119,10 +122,7 @@ class Stepper:
             acc += len(e.want)
         for chunk in chunks:
             self._run_chunk(entries, slots, toks, chunk, out, out_base)
-        if self.check_kernels:
-            ops.gemm_tc_check(self.device)
-        else:
-            self._status_later()
+        self._look_at_status()
         return out
 
     def _cut(self, toks) -> list:
@@ -144,10 +144,22 @@ class Stepper:
                 done[i] = start + take
 
     # ------------------------------------------------------------ the kernels' status word ----
+    def _look_at_status(self, single_tokens: bool = False) -> None:
+        """After every step: with ``check_kernels`` read the kernels' status word now, else start a copy of it. Single-token steps,
+        whose products wait on barriers too (float32 runs, 9 to 64 sequences of large models), take turns: a copy costs some 10 us of
+        the host's time, as much as a hundredth of a short step, and one in ``STATUS_EVERY`` tells of all that came before."""
+        if self.check_kernels:
+            ops.gemm_tc_check(self.device)
+            return
+        self._steps_unseen = self._steps_unseen + 1 if single_tokens else self.STATUS_EVERY
+        if self._steps_unseen >= self.STATUS_EVERY:
+            self._steps_unseen = 0
+            self._status_later()
+
     def _status_later(self) -> None:
-        """After a step of many tokens (the tcgen05 kernels serve those): start a copy of the kernels' status word
-        to pinned memory. It is looked at when the next step begins, without waiting for the device, and at
-        ``check_status``; a bounded wait that gave up inside a kernel is then reported one step late instead of never."""
+        """Start a copy of the kernels' status word to pinned memory. It is looked at when the next step begins, without waiting for the
+        device, and at ``check_status``; a bounded wait that gave up inside a kernel is then reported late instead of never: one
+        step after a step of many tokens, ``STATUS_EVERY`` after one of single tokens."""
         status = ops.tc_status(self.device)
         if status is None:
             return
@@ -322,6 +334,7 @@ class Stepper:
             self.model.forward(b, self.cache, self.ws, logits)
             self._seen_decode.add(gkey)
         book.commit(slots, new_lens)
+        self._look_at_status(single_tokens=True)
         return logits
 
     def _capture(self, b, logits):

@@ -404,6 +404,35 @@ def test_the_stepper_reports_a_given_up_wait_one_step_late(model_folders):
     eng.close([slot])
 
 
+@pytest.mark.parametrize("fed", [False, True])
+def test_a_given_up_wait_is_reported_in_single_token_steps_too(model_folders, fed, monkeypatch):
+    """A server that only goes on token by token hears of it: within the steps that a look at the status word takes turns over, or
+    in the step itself where every step is checked."""
+    from sleuth_b200.kernels import ops
+    eng = load(model_folders["D"], "bf16")
+    ids = requests_for("D", [200], seed=2)[0]
+    (slot,) = eng.open(1)
+    eng.step([(slot, ids[:100], (99,))])
+    token = (lambda i: eng.stepper.decode_fed([slot], [0])) if fed else (lambda i: eng.step([(slot, ids[i:i + 1], (0,))]))
+    for i in range(100, 104):                                    # launch by launch, recorded, replayed
+        token(i)
+    eng.stepper.check_status()
+    ops.tc_wait_probe("cuda:0", polls=1000, code=99)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="code 99"):
+        for i in range(104, 104 + eng.stepper.STATUS_EVERY + 2):
+            token(i)
+            torch.cuda.synchronize()
+    token(130)
+    eng.stepper.check_status()
+    monkeypatch.setattr(eng.stepper, "check_kernels", True)
+    token(131)
+    ops.tc_wait_probe("cuda:0", polls=1000, code=99)
+    with pytest.raises(RuntimeError, match="code 99"):
+        token(132)
+    eng.close([slot])
+
+
 def test_context_full_through_the_entry_point(model_folders):
     import sleuth_b200 as sb
     eng = sb.load(model_folders["A"], dtype="fp32", max_seq_len=20, max_tokens=256)
