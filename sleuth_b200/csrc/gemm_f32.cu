@@ -9,16 +9,9 @@
 // for any batch. With few rows the segments are the only parallelism a narrow matrix has; shorter chains also round less.
 // (The reference has no such path on the GPU: its float32 models run under bfloat16 autocast there,
 // sleuth/forge/infer/generate.py:76-77.)
-#include "packed_f32.cuh"
+#include "gemm_f32_split.cuh"
 
 namespace slb {
-
-constexpr int kMaxSegments = 8;
-// k values in a segment: an eighth of K in whole 64s, at least 128.
-__host__ __device__ inline int segment_length(int K) {
-  const int len = ((K + kMaxSegments * 64 - 1) / (kMaxSegments * 64)) * 64;
-  return len < 128 ? 128 : len;
-}
 
 // Tiles that a block of the streaming kernel takes side by side, with `room` blocks for `tiles` tiles: no more than its warps have
 // segments for, and none while blocks are to be had, where joining the tiles' sums takes as long as forming them (K below 64) or

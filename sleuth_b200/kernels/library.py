@@ -149,7 +149,7 @@ _SIGNATURES = {
     "slb_decode_layers": [P, P],
     "slb_gemm_tc_qkv": [P, P, I, I, I, I, I, P, P, P, P, P, F, P, P, P, P, P, P, I, P, P],
     "slb_gemm_f32": [P, P, P, P, I, I, I, I, I, I, I, I, P],
-    "slb_gemm_f32_tc": [P, P, P, P, I, I, I, I, I, I, I, I, I, F, F, I, I, I, P, P],
+    "slb_gemm_f32_tc": [P, P, P, P, I, I, I, I, I, I, I, I, I, F, F, I, P, L, P, P],
     "slb_penalize": [P, L, I, I, P, P, I, F, P, P, I, P],
     "slb_argmax": [P, L, I, I, P, P, L, P],
     "slb_sample": [P, L, I, I, F, I, F, F, P, P, P],

@@ -553,38 +553,47 @@ def decode_scratch_floats(n_seqs: int, heads: int, head_dim: int, splits: int) -
 
 def f32_on_tensor_cores(N: int, K: int, w_address: int) -> bool:
     """Whether the 32-bit products with a matrix [N, K] run on the tensor cores (csrc/gemm_f32_tc.cu) or as FMA chains
-    (csrc/gemm_f32.cu). The two add in different orders, so the rule may look at the matrix only, never at the number of rows."""
-    return K % 4 == 0 and K >= 256 and N >= 512 and N * K >= 1 << 19 and w_address % 16 == 0
+    (csrc/gemm_f32.cu). The two add in different orders, so the rule may look at the matrix only, never at the number of rows.
+    From K = 1,024 on: there the sums' error is below the FMA chains' for operands of one sign and of wide range too, and below it
+    few rows are quicker by FMA (2,048 x 512, one row 2.2 us against 2.8)."""
+    return K % 4 == 0 and K >= 1024 and N >= 512 and w_address % 16 == 0
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias=None, accumulate: bool = False,
-             stream=None, static_weight: bool = False, form=None) -> None:
-    """out[M, N] (+)= a[M, K] @ w[N, K]^T (+ bias), all float32, every product and sum to float32. ``static_weight``: no kernel
-    writes ``w`` (a loaded matrix), so it may be read before the kernel in front has finished. ``form`` = (tokens of a tile, blocks
-    that share K, warps that split) sends the product to the tensor-core kernel in that form; the bits do not depend on it."""
+             stream=None, static_weight: bool = False, form=None, next_read=None) -> None:
+    """out[M, N] (+)= a[M, K] @ w[N, K]^T (+ bias), all float32. ``static_weight``: no kernel writes ``w`` (a loaded matrix), so it may be
+    read before the kernel in front has finished. ``form`` asks for a kernel instead of leaving it to the rules: "fma" (FMA chains), or the
+    tensor-core product, whose bits do not depend on its form: 0 (its own rule), 1 (the kernel for few rows), 32, 64 or 128 (tokens of a tile).
+    ``next_read``, as for ``gemm_skinny``: the kernel for few rows asks the L2 cache for it."""
     _cuda(a, w, out, bias)
     M, K = a.shape
     N = w.shape[0]
     _need(w.shape[1] == K and out.shape == (M, N), "gemm_f32: shapes disagree")
     _need(a.dtype == w.dtype == out.dtype == torch.float32, "gemm_f32: float32 only")
-    if form is not None or f32_on_tensor_cores(N, K, w.data_ptr()):
+    if form != "fma" and (form is not None or f32_on_tensor_cores(N, K, w.data_ptr())):
         lib().call("slb_gemm_f32_tc", _p(a), _p(w), _p(bias), _p(out), M, N, K, K, K, N, int(accumulate), int(static_weight),
-                   -1, 0.0, 1.0, *(int(f) for f in form or (0, 0, 0)), _p(_tc_status(a.device)), stream if stream is not None else current_stream())
+                   -1, 0.0, 1.0, int(form or 0), _p(next_read) if _nbytes(next_read) else None, _nbytes(next_read), _p(_tc_status(a.device)), stream if stream is not None else current_stream())
         return
     lib().call("slb_gemm_f32", _p(a), _p(w), _p(bias), _p(out), M, N, K, K, K, N, int(accumulate), int(static_weight),
                stream if stream is not None else current_stream())
 
 
-def gemm_f32_gated(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gate=None, stream=None, static_weight: bool = False, form=None) -> None:
-    """out[M, N] = act(a @ w[:N]^T) * (a @ w[N:]^T) in float32 on the tensor cores, with the bits of ``gemm_f32`` and ``gated_act`` one after
-    the other; only for matrices that ``f32_on_tensor_cores`` sends there. ``gate``, as for the other gated products: (name, limit, alpha)."""
+def f32_form(M: int, N: int, K: int) -> int:
+    """The form that the tensor-core product of these sizes takes: 1, the kernel for few rows, or the tokens of a tile."""
+    return int(lib().dll.slb_gemm_f32_form(int(M), int(N), int(K)))
+
+
+def gemm_f32_gated(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gate=None, stream=None, static_weight: bool = False, next_read=None) -> None:
+    """out[M, N] = act(a @ w[:N]^T) * (a @ w[N:]^T) in float32 on the tensor cores, in the form for few rows, with the bits of
+    ``gemm_f32`` and ``gated_act`` one after the other; only for matrices that ``f32_on_tensor_cores`` sends there. ``gate``, as for the
+    other gated products: (name, limit, alpha)."""
     _cuda(a, w, out)
     M, K = a.shape
     N = out.shape[1]
     _need(w.shape == (2 * N, K) and out.shape[0] == M, "gemm_f32_gated: shapes disagree")
     _need(a.dtype == w.dtype == out.dtype == torch.float32, "gemm_f32_gated: float32 only")
     lib().call("slb_gemm_f32_tc", _p(a), _p(w), None, _p(out), M, N, K, K, K, N, 0, int(static_weight), *(_gate_args(gate) or (0, 0.0, 1.0)),
-               *(int(f) for f in form or (0, 0, 0)), _p(_tc_status(a.device)), stream if stream is not None else current_stream())
+               0, _p(next_read) if _nbytes(next_read) else None, _nbytes(next_read), _p(_tc_status(a.device)), stream if stream is not None else current_stream())
 
 
 SKINNY_MODES = {"bf16": 0, "f32": 1, "add": 2, "swiglu": 3}

@@ -250,7 +250,9 @@ class GQAAttention(Part):
             splits = ops.decode_splits(b.n, s.kv_heads, s.heads // s.kv_heads, table.shape[1])
             # the attention kernel gets onto the SMs too late to fetch ahead: the projection asks L2 for its first pages
             pages = ops.next_pages(view.k_pool, view.v_pool, table, b.past, splits, view.window)
-        qkv = self.qkv.forward(h, ws=ws, stream=b.stream, next_pages=pages)
+        # (float32: two launches lie between the two projections; the first one's blocks ask L2 for the second's matrix)
+        f32 = self.ctx.dtype == torch.float32
+        qkv = self.qkv.forward(h, ws=ws, stream=b.stream, next_pages=pages, next_read=self.o.weight if f32 else None)
         y = ws.take((T, s.heads * s.head_dim), self.ctx.dtype)
         if single:
             # one token per sequence: the attention kernel post-processes q/k/v itself and appends to the cache
@@ -269,7 +271,7 @@ class GQAAttention(Part):
                      view.k_pool if writes else None, view.v_pool if writes else None,
                      b.tok_seq, b.tok_pos, table, s.heads, kvh, s.head_dim, rot, s.qk_norm_eps, b.stream)
         self._attend(q, y, b, view, table, ws)
-        self.o.forward(y, ws=ws, stream=b.stream, **result_target(b, x))
+        self.o.forward(y, ws=ws, stream=b.stream, next_read=getattr(b, "next_read", None) if f32 else None, **result_target(b, x))
         ws.release(mark)
 
 

@@ -78,8 +78,8 @@ class GatedMLP(Part):
                 ops.gemm_skinny(hh, self.gate_up.weight, act, "swiglu", b.stream, self.down.weight, features=f, gate=self.gate)
         elif self.ctx.dtype == torch.bfloat16 and linear.use_tc(T, self.spec.intermediate, self.spec.hidden):
             ops.gemm_tc(h.tensor() if isinstance(h, Normed) else h, self.gate_up.weight, act, "swiglu", b.stream, gate=self.gate)
-        elif self.ctx.dtype == torch.float32 and T <= 64 and ops.f32_on_tensor_cores(2 * self.spec.intermediate, self.spec.hidden, self.gate_up.weight.data_ptr()):
-            ops.gemm_f32_gated(h.tensor() if isinstance(h, Normed) else h, self.gate_up.weight, act, self.gate, b.stream, static_weight=True)
+        elif self.ctx.dtype == torch.float32 and ops.f32_on_tensor_cores(2 * self.spec.intermediate, self.spec.hidden, self.gate_up.weight.data_ptr()) and ops.f32_form(T, 2 * self.spec.intermediate, self.spec.hidden) == 1:
+            ops.gemm_f32_gated(h.tensor() if isinstance(h, Normed) else h, self.gate_up.weight, act, self.gate, b.stream, static_weight=True, next_read=self.down.weight)
         else:
             gu = self.gate_up.forward(h, ws=ws, stream=b.stream)
             ops.gated_act(gu, act, self.spec.activation, b.stream, self.spec.limit, self.spec.alpha)

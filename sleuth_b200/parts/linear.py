@@ -189,11 +189,11 @@ class Linear:
             h = h.tensor()
         if self.dtype == torch.float32:
             if into is not None:
-                ops.gemm_f32(h, self.weight, into, accumulate=True, stream=stream, static_weight=True)
+                ops.gemm_f32(h, self.weight, into, accumulate=True, stream=stream, static_weight=True, next_read=next_read)
                 return into
             if out is None:
                 out = ws.take((M, self.out_features), torch.float32)
-            ops.gemm_f32(h, self.weight, out, stream=stream, static_weight=True)
+            ops.gemm_f32(h, self.weight, out, stream=stream, static_weight=True, next_read=next_read)
             return out
         if streams(h, self.weight):
             if into is not None:

@@ -126,3 +126,13 @@ def test_rows_that_lie_otherwise_stay_with_the_other_kernels():
     assert linear.streams(h[:-1].view(40, 2560), weight) and linear.streams(h[:-1].view(40, 2560), weight, gated=True)
     assert not linear.streams(h[1:].view(40, 2560), weight) and not linear.streams(h[:-1].view(40, 2560), shifted)
     assert not linear.streams(wide[:, :2560], weight)
+
+
+def test_float32_product_on_the_tensor_cores_takes_what_was_faster():
+    """Forms at which products were timed on a B200 (1: the kernel for few rows; else tokens of a tile), and the matrices that go there."""
+    form = ops.f32_form
+    for M, N, K, want in [(1, 4096, 1024, 1), (8, 19456, 2560, 1), (1, 151936, 1024, 1), (16, 1024, 3072, 1), (32, 6144, 1024, 1), (64, 1024, 2048, 1), (16, 151936, 1024, 32),
+                          (64, 6144, 1024, 64), (1500, 4096, 1024, 128), (1500, 1024, 3072, 128)]:
+        assert form(M, N, K) == want, (M, N, K, form(M, N, K))
+    assert ops.f32_on_tensor_cores(512, 1024, 0) and not ops.f32_on_tensor_cores(4096, 1020, 0) and not ops.f32_on_tensor_cores(511, 4096, 0)
+    assert not ops.f32_on_tensor_cores(512, 1030, 0) and not ops.f32_on_tensor_cores(512, 1024, 8)
