@@ -17,7 +17,8 @@
 //
 // Cost: a row's eighth is read once into shared memory, and one histogram over values between a lower bound and the row's
 // maximum finds the short list that holds the answer (the quick path, below). 64 rows of 151,936, top-k 50, top-p 0.9: 247 us
-// before (six passes over the row, four of them with 64 KB of histograms to clear and add up), 55 us with the row held, 39 us with thread maxima (LEAN, below). Calls and rows for
+// before (six passes over the row, four of them with 64 KB of histograms to clear and add up); now, on rows that no call has read before, 66 us with the row held and 32 us with thread maxima (LEAN,
+// below). Calls and rows for
 // which that cannot work (neither top-k nor top-p, top-k beyond the list, rows longer than the blocks hold, NaN or infinite
 // maxima, more candidates than fit) take the general path: a radix descent over the sort keys, eight bits a pass.
 #include <math.h>
@@ -37,10 +38,12 @@ namespace slb {
 // size share an SM, so that one works while the other stands at a barrier. 8 rows of 151,936 in us, 512 / 1,024 threads: temperature
 // alone 37 / 25, top-k 3,000 100 / 70; 64 rows: 68 / 84, 255 / 310.
 constexpr int kFewRowsThreads = 1024, kManyRowsThreads = 512;
-// Short top-k lists of many rows (LEAN): the row is not held, and four blocks of 256 threads fit an SM, all 512 blocks of 64 rows at once.
-// us, held / lean: 18 rows of 151,936, k 50 45 / 31, 64 rows 68 / 39, of 8,000 49 / 23; 64 rows of 151,936, k 200 96 / 74, k 400 150 / 193 (the list's
-// own work wants more threads); 8 rows, k 50 27 / 31.
-constexpr int kLeanThreads = 256, kLeanTopK = 200, kLeanRows = 18, kLeanTokens = 8000;
+// Short top-k lists of many rows (LEAN): the row is not held, and two blocks of 512 threads or, from 38 rows on, four of 256 fit an SM, all 512
+// blocks of 64 rows at once. Up to 50 tokens: where the largest values lie side by side the list is four times as long (four tokens a thread maximum),
+// and it is compared each with each. us of rows that no call has read before, held / lean: 18 rows of 151,936, k 50 40 / 23, 36 rows 49 / 39, 64 rows 66 / 32, of
+// 8,000 42 / 21; one value far above the others 67 / 61; rows sorted by value, 64 of 151,936 66 / 67, of 8,000 38 / 48 (k 64: 39 / 70, k 100 40 / 138);
+// rows for which neither can work (18 of 151,936 values within a thousandth, more than a thousand tie) 96 / 109.
+constexpr int kLeanTopK = 50, kLeanRows = 18, kLeanTokens = 8000;
 constexpr double kMassScale = 1099511627776.0;  // 2^40
 
 __device__ __forceinline__ unsigned int sort_key(float v) {
@@ -169,7 +172,7 @@ struct SampleShared {
   SampleExchange x;
   unsigned long long hist[256];
   unsigned long long total;
-  unsigned long long above;
+  unsigned long long above, inside;
   unsigned int prefix;
   int chosen;
   int count;
@@ -405,7 +408,8 @@ __device__ int warp_walk(int n, G get, float mx, unsigned int floor_key, float m
 // maximum, is added up over the team; the step in which the weight from above reaches the target is known then, and the few
 // tokens at or above it (for top-k), or in it (for top-p without top-k), are all that the exact decision needs.
 constexpr int kHeldTokens = 20480;     // tokens a block holds
-constexpr int kBins = 1024, kLeanBins = 256;
+constexpr int kBins = 1024, kLeanBins = 512;
+constexpr unsigned long long kCrowded = 16;      // thread maxima in the step that decides from which on it is cut again
 constexpr float kBanned = -1e30f;      // logits below are no candidates' (bans set the lowest value or minus infinity)
 constexpr int kQuickList = 1024;       // candidates of a row at most
 constexpr int kSmallList = 512;        // up to this many entries are compared each with each
@@ -433,9 +437,9 @@ template <int BINS>
 __device__ __forceinline__ int bin_of(float v, float mx, float per) { return min(BINS - 1, (int)((mx - v) * per)); }
 
 // The step at which the weight of the team's histogram, added up from step 0, first reaches `target`, or -1; `above` = the
-// weight of the steps before it. LIMBS 1: counts; 3: masses in parts of 16, 16 and 9 bits (shared memory adds 32-bit words).
+// weight of the steps before it, `inside` = its own. LIMBS 1: counts; 3: masses in parts of 16, 16 and 9 bits (shared memory adds 32-bit words).
 template <int LIMBS, int THREADS, int BINS>
-__device__ int find_bin(Team& team, const unsigned int* hist, unsigned long long target, unsigned long long& above) {
+__device__ int find_bin(Team& team, const unsigned int* hist, unsigned long long target, unsigned long long& above, unsigned long long& inside) {
   SampleShared& sh = *team.sh;
   constexpr int kPer = BINS / THREADS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -467,12 +471,14 @@ __device__ int find_bin(Team& team, const unsigned int* hist, unsigned long long
     if (acc < target && acc + h[j] >= target) {      // one thread and step at most
       sh.chosen = threadIdx.x * kPer + j;
       sh.above = acc;
+      sh.inside = h[j];
     }
     acc += h[j];
   }
   __syncthreads();
   const int found = sh.chosen;
   above = sh.above;
+  inside = sh.inside;
   __syncthreads();
   return found;
 }
@@ -550,9 +556,9 @@ __device__ int gather_lists(Team& team, int* tokens, float* values, int* all_tok
   return n;
 }
 
-// LEAN: what the block keeps of its part of the row is one maximum a thread. The step in which the k-th largest of the row's thread
+// LEAN: what a block keeps of the row is one maximum a thread. The step in which the k-th largest of the row's thread
 // maxima lies bounds the k-th largest value from below, and tightly (the largest values mostly fall to different threads); the values at or
-// above it are collected in a second read of the row, which L2 then holds. One atomic addition a thread in place of one a token, a quarter of
+// above it are collected in a second read of the row, which L2 then holds. One atomic addition a thread in place of one a token, half
 // the steps, and no shared memory but the lists.
 template <int THREADS, bool LEAN>
 __global__ void __cluster_dims__(kSampleTeam, 1, 1) __launch_bounds__(THREADS, 1024 / THREADS)
@@ -610,17 +616,38 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
       }
       return v;
     };
-#pragma unroll 5
-    for (int c = 0; mine.begin + 128 * c < mine.end; ++c) {
-      const float4 v = four_at(mine.begin + 128 * c + 4 * lane);
+    // LEAN: the row's threads take turns at four tokens each, so that large values side by side fall to many threads too
+    constexpr int kTurn = kSampleTeam * THREADS * 4;
+    const int lean_first = (rank * THREADS + threadIdx.x) * 4;
+    const bool row_aligned = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+    auto lean_at = [&](int t) {
+      if (t + 3 < limit && row_aligned) return *reinterpret_cast<const float4*>(row + t);
+      float4 v = make_float4(row[t], -INFINITY, -INFINITY, -INFINITY);
+      if (t + 1 < limit) v.y = row[t + 1];
+      if (t + 2 < limit) v.z = row[t + 2];
+      if (t + 3 < limit) v.w = row[t + 3];
+      return v;
+    };
+    auto look = [&](const float4& v) {
       bad = bad || v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w;
       most = fmaxf(most, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
-      if (!count_first) least = fminf(least, fminf(fminf(allowed(v.x), allowed(v.y)), fminf(allowed(v.z), allowed(v.w))));
-      if constexpr (!LEAN) mine.mine[c * THREADS] = v;
+    };
+    if constexpr (LEAN) {
+#pragma unroll 5
+      for (int t = lean_first; t < limit; t += kTurn) look(lean_at(t));
+    } else {
+#pragma unroll 5
+      for (int c = 0; mine.begin + 128 * c < mine.end; ++c) {
+        const float4 v = four_at(mine.begin + 128 * c + 4 * lane);
+        look(v);
+        if (!count_first) least = fminf(least, fminf(fminf(allowed(v.x), allowed(v.y)), fminf(allowed(v.z), allowed(v.w))));
+        mine.mine[c * THREADS] = v;
+      }
     }
     // At least as many values as there are warps (threads) with a maximum of their own reach the smallest of those maxima.
     const float warp_most = warp_max(most);
-    const int warps_with = (limit + chunks * 128 - 1) / max(1, chunks * 128);      // warps of the row that hold tokens, about
+    // warps of the row that hold tokens, about
+    const int warps_with = LEAN ? min(kSampleTeam * kWarps, (limit + 127) / 128) : (limit + chunks * 128 - 1) / max(1, chunks * 128);
     float low = top_k <= warps_with / 2 ? warp_most : most;
     low = allowed(count_first ? low : least);      // (threads without tokens have neither)
     const float low_block = -block_max(-low, sh.red);
@@ -645,33 +672,56 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
       quick = quick && width > 1e-5f * size && width > 1e-30f * temperature && temperature > 1e-30f;
       if (quick) {
         const float per = (BINS - 0.5f) / (row_most - row_low);
+        unsigned long long above, inside;
         if constexpr (LEAN) {
-          if (most >= row_low) atomicAdd(&bins[bin_of<BINS>(most, row_most, per)], 1u);
+          const int my_bin = bin_of<BINS>(most, row_most, per);
+          if (most >= row_low) atomicAdd(&bins[my_bin], 1u);
+          team.cluster.sync();
+          const int bin = find_bin<1, THREADS, BINS>(team, bins, (unsigned long long)top_k, above, inside);
+          // Fewer maxima than the list asks for (few tokens are allowed), or no whole step below: everything that is allowed.
+          const bool all = bin < 0 || bin >= BINS - 2;
+          // One value far above the others makes the steps wide: where many maxima share the step, it and the next are cut into steps again,
+          // if these are still wider than what rounds to the same quotient.
+          const float top2 = row_most - (float)bin / per, per2 = (BINS - 0.5f) * per * 0.5f;
+          int fine = -1;
+          if (!all && inside > kCrowded && 2.0f > 1e-5f * size * (BINS * per)) {
+            team.cluster.sync();
+            for (int i = threadIdx.x; i < BINS; i += blockDim.x) bins[i] = 0u;
+            __syncthreads();
+            if (most >= row_low && (my_bin == bin || my_bin == bin + 1)) atomicAdd(&bins[max(0, bin_of<BINS>(most, top2, per2))], 1u);
+            team.cluster.sync();
+            unsigned long long unused;
+            fine = find_bin<1, THREADS, BINS>(team, bins, (unsigned long long)top_k - above, unused, inside);
+            if (fine >= BINS - 2) fine = -1;
+          }
+          const float least_kept = all ? kBanned : fmaxf(row_low, fine < 0 ? row_most - ((float)bin + 2.5f) / per : top2 - ((float)fine + 2.5f) / per2);
+          auto keep = [&](int t, float x) {
+            if (x < least_kept) return;
+            if (!all) {
+              const int b = bin_of<BINS>(x, row_most, per);
+              if (b > bin + 1 || (fine >= 0 && b >= bin && bin_of<BINS>(x, top2, per2) > fine + 1)) return;
+            }
+            keep_candidate(sh, cand_token, cand_value, t, x);
+          };
+#pragma unroll 5
+          for (int t = lean_first; t < limit; t += kTurn) {      // (beyond the end: minus infinity, below every bound)
+            const float4 v = lean_at(t);
+            if (fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)) < least_kept) continue;
+            keep(t, v.x);
+            keep(t + 1, v.y);
+            keep(t + 2, v.z);
+            keep(t + 3, v.w);
+          }
         } else {
           mine.each([&](int, float x) { if (x >= row_low) atomicAdd(&bins[bin_of<BINS>(x, row_most, per)], 1u); });
-        }
-        team.cluster.sync();
-        unsigned long long above;
-        const int bin = find_bin<1, THREADS, BINS>(team, bins, (unsigned long long)top_k, above);
-        quick = bin >= 0 && bin < BINS - 2;
-        if (quick) {
-          auto keep = [&](int t, float x) {
+          team.cluster.sync();
+          const int bin = find_bin<1, THREADS, BINS>(team, bins, (unsigned long long)top_k, above, inside);
+          quick = bin >= 0 && bin < BINS - 2;
+          if (quick) mine.each([&](int t, float x) {
             if (x >= row_low && bin_of<BINS>(x, row_most, per) <= bin + 1) keep_candidate(sh, cand_token, cand_value, t, x);
-          };
-          if constexpr (LEAN) {
-#pragma unroll 5
-            for (int c = 0; mine.begin + 128 * c < mine.end; ++c) {      // (beyond the end: minus infinity, below every bound)
-              const int t = mine.begin + 128 * c + 4 * lane;
-              const float4 v = four_at(t);
-              if (fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)) < row_low) continue;
-              keep(t, v.x);
-              keep(t + 1, v.y);
-              keep(t + 2, v.z);
-              keep(t + 3, v.w);
-            }
-          } else {
-            mine.each(keep);
-          }
+          });
+        }
+        if (quick) {
           int* all_token = reinterpret_cast<int*>(bins);
           float* all_value = reinterpret_cast<float*>(dynamic);      // the held row is not needed any more where the list fits
           const int n = gather_lists(team, cand_token, cand_value, all_token, all_value, rank, kQuickList);
@@ -681,7 +731,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
             team.solo = true;
             mx = row_most / temperature;
             unsigned long long* scratch = dynamic + kQuickList / 2;
-            const unsigned int kth = list_threshold<true>(team, all_token, all_value, n, 0.0f, 0u, 0ull, (unsigned long long)top_k, scratch);
+            const unsigned int kth = list_threshold<true>(team, all_token, all_value, n, 0.0f, 0u, 0ull, (unsigned long long)min(top_k, n), scratch);
             const unsigned int b = (kth & 0x80000000u) ? (kth & 0x7fffffffu) : ~kth;     // back to the float
             floor_key = sort_key(__uint_as_float(b) / temperature);
             // in token order (the draw walks it), divided by the temperature
@@ -728,7 +778,8 @@ sample_kernel(const float* __restrict__ logits, long long ld, int limit, float t
         unsigned long long target = (unsigned long long)ceil((double)top_p * (double)total), above;
         if (target < 1ull) target = 1ull;
         if (target > total) target = total;
-        const int bin = find_bin<3, THREADS, kBins>(team, bins, target, above);
+        unsigned long long inside;
+        const int bin = find_bin<3, THREADS, kBins>(team, bins, target, above, inside);
         quick = bin >= 0 && bin < kBins - 1;
         if (quick) {
           mine.each([&](int t, float x) {
@@ -1011,6 +1062,13 @@ extern "C" int slb_sample_threads(int rows) { return (long long)rows * kSampleTe
 // Whether rows go through the lean form.
 extern "C" int slb_sample_lean(int rows, int limit, int top_k) { return top_k > 0 && top_k <= kLeanTopK && limit >= kLeanTokens && rows >= kLeanRows; }
 
+// Threads of a block for such a call. Lean blocks have 512 while two of them fit every SM that has any (rows that end on the general path
+// take as long as in the other form then), else 256, four of which fit.
+extern "C" int slb_sample_threads_of(int rows, int limit, int top_k) {
+  if (!slb_sample_lean(rows, limit, top_k)) return slb_sample_threads(rows);
+  return (long long)rows * kSampleTeam <= 2ll * sm_count() ? 512 : 256;
+}
+
 extern "C" int slb_sample(const float* logits, long long ld, int rows, int limit, float temperature, int top_k,
                           float top_p, float min_p, const float* uniform, int* out, void* stream) {
   SLB_REQUIRE(rows >= 0 && limit > 0 && ld >= limit, "sample: rows=%d limit=%d ld=%lld", rows, limit, ld);
@@ -1021,15 +1079,16 @@ extern "C" int slb_sample(const float* logits, long long ld, int rows, int limit
   if (rows == 0) return 0;
   // the quick path's row and histogram; the general path's warp histograms and candidates lie in the same place
   constexpr int hist_bytes = kHeldTokens * sizeof(float) + 3 * kBins * sizeof(unsigned int);
-  constexpr int lean_bytes = kLeanThreads / 32 * 2048 + 2 * kCandidates * sizeof(int);
   static_assert(kMostWarps * 256 * sizeof(unsigned long long) + 2 * kCandidates * sizeof(int) <= kHeldTokens * sizeof(float), "the general path's place");
-  static_assert(2 * kCandidates * sizeof(int) <= kLeanThreads / 32 * 2048, "the general path's joined list");
-  static_assert(kQuickList * 4 + kLeanThreads / 32 * 2048 + kQuickList * 4 <= lean_bytes, "the lean path's place (the joined list's tokens lie where the steps were)");
-  const bool lean = slb_sample_lean(rows, limit, top_k) != 0, few = slb_sample_threads(rows) == kFewRowsThreads;
-  const auto kernel = lean ? sample_kernel<kLeanThreads, true> : few ? sample_kernel<kFewRowsThreads, false> : sample_kernel<kManyRowsThreads, false>;
-  const int threads = lean ? kLeanThreads : few ? kFewRowsThreads : kManyRowsThreads, bytes = lean ? lean_bytes : hist_bytes;
-  static std::atomic<unsigned long long> allowed[3];
-  const cudaError_t e = allow_shared((const void*)kernel, bytes, allowed[lean ? 2 : few ? 1 : 0]);
+  const bool lean = slb_sample_lean(rows, limit, top_k) != 0;
+  const int threads = slb_sample_threads_of(rows, limit, top_k), form = lean ? (threads == 256 ? 3 : 2) : threads == kFewRowsThreads ? 1 : 0;
+  const auto kernel = form == 3 ? sample_kernel<256, true> : form == 2 ? sample_kernel<512, true> : form == 1 ? sample_kernel<kFewRowsThreads, false> : sample_kernel<kManyRowsThreads, false>;
+  // lean: the joined list's values, a histogram a warp, the steps (in their place, later, the joined list's tokens; the general path's candidates)
+  const int bytes = lean ? threads / 32 * 2048 + 2 * kCandidates * (int)sizeof(int) : hist_bytes;
+  static_assert(2 * kCandidates * sizeof(int) <= 256 / 32 * 2048, "the general path's joined list");
+  static_assert(kQuickList * 4 + kQuickList * 4 <= 2 * kCandidates * sizeof(int) && kLeanBins <= kQuickList, "the lean path's place");
+  static std::atomic<unsigned long long> allowed[4];
+  const cudaError_t e = allow_shared((const void*)kernel, bytes, allowed[form]);
   if (e != cudaSuccess) return fail(2, "sample: cannot reserve %d bytes of shared memory: %s", bytes, cudaGetErrorString(e));
   launch(kernel, dim3(rows * kSampleTeam), dim3(threads), (size_t)bytes, (cudaStream_t)stream, logits, ld, limit, temperature, top_k, top_p,
          min_p, uniform, out);

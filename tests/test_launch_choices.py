@@ -78,6 +78,9 @@ def test_sampler_blocks_fill_their_sm():
     """Few rows: a block an SM, as large as it can be; more rows: two blocks of half the size."""
     threads = ops.lib().dll.slb_sample_threads
     assert threads(1) == threads(18) == 1024 and threads(19) == threads(64) == 512
+    lean = ops.lib().dll.slb_sample_threads_of
+    assert lean(18, 151936, 50) == lean(37, 8000, 50) == 512 and lean(38, 151936, 50) == lean(64, 8000, 1) == 256
+    assert lean(17, 151936, 50) == 1024 and lean(64, 151936, 51) == lean(64, 7999, 50) == 512
 
 
 def test_float32_attention_scratch():
