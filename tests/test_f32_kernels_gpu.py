@@ -21,7 +21,7 @@ def test_gemm_f32_error_and_rows(M, N, K):
     g = torch.Generator().manual_seed(M * 7 + N)
     a, w, bias = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV), torch.randn(N, generator=g).to(DEV)
     out = torch.full((M, N), float("nan"), device=DEV)
-    ops().gemm_f32(a, w, out, bias)
+    ops().gemm_f32(a, w, out, bias, form="fma")
     ref = a.double() @ w.double().T + bias.double()
     # chains of half a segment, then the halves, at most eight segments and the bias: each step rounds by 2^-24 at most
     seg = max(128, -(-K // 512) * 64)
@@ -31,12 +31,12 @@ def test_gemm_f32_error_and_rows(M, N, K):
     for rows in (1, 2, 5, 12, 30, 60):
         if rows < M:
             some = torch.empty(rows, N, device=DEV)
-            ops().gemm_f32(a[M - rows:].contiguous(), w, some, bias)
+            ops().gemm_f32(a[M - rows:].contiguous(), w, some, bias, form="fma")
             assert torch.equal(some, out[M - rows:])
     acc = torch.full((M, N), 2.0, device=DEV)
-    ops().gemm_f32(a, w, acc, accumulate=True)
+    ops().gemm_f32(a, w, acc, accumulate=True, form="fma")
     plain = torch.empty(M, N, device=DEV)
-    ops().gemm_f32(a, w, plain)
+    ops().gemm_f32(a, w, plain, form="fma")
     assert torch.equal(acc, plain + 2.0)
 
 
@@ -124,7 +124,8 @@ def test_attention_f32_leaves_later_tokens_out():
 
 
 @pytest.mark.parametrize("M", [1, 8, 64, 700])
-def test_gemm_f32_second_operand_written_by_the_kernel_in_front(M):
+@pytest.mark.parametrize("form", ["fma", 1, 64, 128])
+def test_gemm_f32_second_operand_written_by_the_kernel_in_front(M, form):
     """A product may have for its second operand what the launch before it writes: the same bits as with a wait between the two.
     Only a caller that says that no kernel writes that operand has it read early."""
     g = torch.Generator().manual_seed(M)
@@ -135,12 +136,12 @@ def test_gemm_f32_second_operand_written_by_the_kernel_in_front(M):
         b = torch.randn(K, 512, generator=g).to(DEV)
         w = torch.full((N, K), float("nan"), device=DEV)
         torch.cuda.synchronize()
-        ops().gemm_f32(a, b, w)                      # some hundred microseconds
-        ops().gemm_f32(x, w, straight)
+        ops().gemm_f32(a, b, w, form=form)           # some hundred microseconds
+        ops().gemm_f32(x, w, straight, form=form)
         torch.cuda.synchronize()
-        ops().gemm_f32(x, w, wait)
+        ops().gemm_f32(x, w, wait, form=form)
         assert torch.equal(straight, wait)
-        ops().gemm_f32(x, w, straight, static_weight=True)       # (written long ago by now)
+        ops().gemm_f32(x, w, straight, static_weight=True, form=form)       # (written long ago by now)
         assert torch.equal(straight, wait)
 
 
