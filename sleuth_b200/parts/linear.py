@@ -57,18 +57,28 @@ def use_skinny(M: int, N: int, K: int, norm: bool = False) -> bool:
     return M <= SKINNY_ROWS and ops.skinny_supported(M, N, K, norm)
 
 
-# The tcgen05 kernel with the weights as the instruction's rows pays where the stream of the weights outweighs its fixed part (some 2 us
-# more than the weight-streaming kernel's or the library's): from 8 M weights on. Whole runs, ms, without / with it: 4B sizes 16 ragged
-# prompts 183 / 175, 24 short ones 99 / 70 (the weight-streaming kernel goes over the rows twice there); 8B sizes 12 prompts 80 / 74, 64 225 / 221;
-# 0.6B sizes 24 22.7 / 23.9. From 65 rows on the library is ahead (100 rows x 4,096 x 4,096 15.3 / 20.5 us), and at 16 rows the weight-streaming
-# kernel at output matrices (151,936 x 1,024 65.5 / 69.5 us).
-STREAM_MIN_WEIGHTS, STREAM_MAX_WEIGHTS_16 = 8 << 20, 128 << 20
-
-
+# The tcgen05 kernel with the weights as the instruction's rows has some 2 us more of fixed part than the kernels it competes with, and those differ
+# by the number of rows, so the line does too. us in a row of launches, other kernel / this one:
+#   17 to 32 rows (the weight-streaming kernel goes over the rows twice): from 8 M weights on. 24 rows x 2,048 x 4,096 7.9 / 6.7, 4,096 x 2,048 6.3 / 6.3.
+#   9 to 16 rows: the weight-streaming kernel keeps the smaller matrices. 4,096 x 2,560 5.9 / 6.3, 4,096 x 4,096 7.7 / 8.0, 2,048 x 8,192 8.6 / 9.1, but
+#     6,144 x 2,560 11.0 / 7.4, 16,384 x 1,024 10.2 / 8.1, 2,560 x 9,728 15.3 / 11.2; gated (rows of gate and up) 6,144 x 4,096 10.6 / 11.3,
+#     8,192 x 2,048 7.7 / 8.0, 12,288 x 2,560 14.7 / 12.5, 19,456 x 2,560 22.0 / 19.1. Not output matrices (151,936 x 1,024 65.5 / 69.5).
+#   33 to 64 rows: cuBLAS is ahead where there are many features (64 rows x 6,144 x 2,560 8.1 / 9.6, 16,384 x 1,024 8.1 / 10.6, 19,456 x 2,560 18.7 / 21.7),
+#     behind where the sums are long (4,096 x 4,096 10.1 / 10.0, 2,560 x 9,728 14.9 / 13.3, 2,048 x 8,192 13.1 / 10.8). Gated it has the activation kernel
+#     to pay as well (24,576 x 4,096 41.2 / 38.1, 9,216 x 1,024 8.6 / 8.4, but 19,456 x 2,560 21.8 / 22.7, 16,384 x 1,024 10.8 / 11.8).
+#   From 65 rows on the library is ahead (100 rows x 4,096 x 4,096 15.3 / 20.5).
 def use_stream(M: int, N: int, K: int, gated: bool = False) -> bool:
-    weights = (2 * N if gated else N) * K
-    return (USE_TC and 8 < M <= 64 and weights >= STREAM_MIN_WEIGHTS and (M > 16 or weights <= STREAM_MAX_WEIGHTS_16)
-            and ops.stream_supported(M, N, K))
+    features = 2 * N if gated else N
+    weights = features * K
+    if not USE_TC or not 8 < M <= 64 or weights < 8 << 20 or not ops.stream_supported(M, N, K):
+        return False
+    if M <= 16:
+        return (28 << 20 if gated else 10_000_000 if features > 4096 else 20 << 20) <= weights <= 128 << 20
+    if M <= 32:
+        return True
+    if gated:
+        return M <= 48 or weights < 16 << 20 or K >= 3072
+    return features <= 4096 and K >= 4096
 
 
 def streams(h: torch.Tensor, weight: torch.Tensor, gated: bool = False) -> bool:

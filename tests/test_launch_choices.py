@@ -113,10 +113,12 @@ def test_float32_product_takes_what_was_faster():
 
 
 def test_large_matrices_of_some_rows_are_streamed_through_the_tensor_cores():
-    """Where whole runs were timed with and without (4B, 8B and 0.6B sizes)."""
+    """Where products and whole runs were timed with and without (4B, 8B and 0.6B sizes, and such between them)."""
     for M, N, K, gated, want in [(16, 2560, 9728, False, True), (16, 9728, 2560, True, True), (24, 6144, 2560, False, True), (64, 12288, 4096, True, True),
                                  (8, 9728, 2560, True, False), (65, 12288, 4096, True, False), (24, 1024, 3072, False, False), (24, 3072, 1024, True, False),
-                                 (16, 151936, 2560, False, False), (24, 151936, 2560, False, True)]:
+                                 (16, 151936, 2560, False, False), (24, 151936, 2560, False, True), (16, 4096, 2560, False, False), (16, 4096, 4096, False, False),
+                              (16, 6144, 2560, False, True), (16, 3072, 4096, True, False), (16, 6144, 2560, True, True), (32, 4096, 2048, False, True), (33, 6144, 2560, False, False),
+                              (64, 8192, 2048, False, False), (64, 4096, 12288, False, True), (64, 9728, 2560, True, False), (48, 9728, 2560, True, True), (64, 4608, 1024, True, True)]:
         assert linear.use_stream(M, N, K, gated) == want, (M, N, K)
 
 
@@ -124,10 +126,10 @@ def test_rows_that_lie_otherwise_stay_with_the_other_kernels():
     """The streaming kernel reads rows one behind the other from 16-byte boundaries on; strided rows and odd addresses go on as before."""
     w = torch.empty(4096 * 2560 + 8, dtype=torch.bfloat16)
     weight, shifted = w[:4096 * 2560].view(4096, 2560), w[1:4096 * 2560 + 1].view(4096, 2560)
-    wide = torch.empty(40, 2568, dtype=torch.bfloat16)
-    h = torch.empty(40 * 2560 + 1, dtype=torch.bfloat16)
-    assert linear.streams(h[:-1].view(40, 2560), weight) and linear.streams(h[:-1].view(40, 2560), weight, gated=True)
-    assert not linear.streams(h[1:].view(40, 2560), weight) and not linear.streams(h[:-1].view(40, 2560), shifted)
+    wide = torch.empty(20, 2568, dtype=torch.bfloat16)
+    h = torch.empty(20 * 2560 + 1, dtype=torch.bfloat16)
+    assert linear.streams(h[:-1].view(20, 2560), weight) and linear.streams(h[:-1].view(20, 2560), weight, gated=True)
+    assert not linear.streams(h[1:].view(20, 2560), weight) and not linear.streams(h[:-1].view(20, 2560), shifted)
     assert not linear.streams(wide[:, :2560], weight)
 
 
