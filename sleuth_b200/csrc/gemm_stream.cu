@@ -1,7 +1,7 @@
-// bfloat16 matrix product for a few to 128 rows on the fifth-generation tensor cores: C[M, N] = X[M, K] * W[N, K]^T, float32 sums.
+// bfloat16 matrix product for a few to 64 rows on the fifth-generation tensor cores: C[M, N] = X[M, K] * W[N, K]^T, float32 sums.
 //
 // What bounds such a product is the stream of the weights. So the weights are the instruction's rows (128 features of a tile, however few
-// tokens there are) and the tokens its columns (NT = 16 to 128); K is shared out over a cluster of 1 to 8 blocks, so that narrow
+// tokens there are) and the tokens its columns (NT = 16 to 64); K is shared out over a cluster of 1 to 8 blocks, so that narrow
 // matrices too keep most SMs loading. A block has a ring of 64-wide slices, about 100 KB, in half an SM's shared memory, and where no
 // kernel writes W it asks for the ring's weights before the kernel in front has finished. Per slice one lane issues four tcgen05.mma; the
 // sums leave tensor memory through shared memory ([token][feature], in the ring's place), and each block of the cluster adds up the partial
@@ -274,20 +274,20 @@ static int gs_splits(int tiles, int K) {
 using namespace slb;
 
 // Whether the kernel takes the problem (rows of 16-byte multiples, whole gate and up tiles need nothing).
-extern "C" int slb_gemm_stream_supported(int M, int N, int K) { return M >= 1 && M <= 128 && N >= 1 && K >= 64 && K % 8 == 0; }
+extern "C" int slb_gemm_stream_supported(int M, int N, int K) { return M >= 1 && M <= 64 && N >= 1 && K >= 64 && K % 8 == 0; }
 
 // mode: 0 store bfloat16, 1 store float32, 2 add into float32, 3 gated activation (W: N gate rows, then N up rows). splits: 0 for the
 // rule's choice, else blocks that share K (1 to 8, at most the 64-wide slices of K). static_weight: no kernel writes W. `status`: a device
 // int that the caller zeroed; a bounded wait that gave up writes its code there.
 extern "C" int slb_gemm_stream(const void* X, const void* W, void* C, int M, int N, int K, int ldc, int mode, int kind, float limit, float alpha,
                                int static_weight, int splits, int* status, void* stream) {
-  SLB_REQUIRE(slb_gemm_stream_supported(M, N, K), "gemm_stream: M=%d N=%d K=%d is not taken (1 to 128 rows, K a multiple of 8 and at least 64)", M, N, K);
+  SLB_REQUIRE(slb_gemm_stream_supported(M, N, K), "gemm_stream: M=%d N=%d K=%d is not taken (1 to 64 rows, K a multiple of 8 and at least 64)", M, N, K);
   SLB_REQUIRE(mode >= 0 && mode <= 3 && ldc >= N && status != nullptr && kind >= kGateSilu && kind <= kGateLast, "gemm_stream: mode=%d ldc=%d N=%d kind=%d", mode, ldc, N, kind);
   SLB_REQUIRE(((uintptr_t)X % 16 == 0) && ((uintptr_t)W % 16 == 0), "gemm_stream: X and W must be 16-byte aligned");
   SLB_REQUIRE(splits >= 0 && splits <= 8 && splits <= (K + kGsK - 1) / kGsK, "gemm_stream: %d blocks for K=%d", splits, K);
   const bool gated_mode = mode == kGsGated;
   const int cols = gated_mode ? kGsFeatures / 2 : kGsFeatures, tiles = (N + cols - 1) / cols;
-  const int nt = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+  const int nt = M <= 16 ? 16 : M <= 32 ? 32 : 64;
   CUtensorMap mw, mx;
   int rc = gs_map(&mw, W, gated_mode ? 2ll * N : N, K, 64);
   if (rc) return rc;
@@ -300,7 +300,6 @@ extern "C" int slb_gemm_stream(const void* X, const void* W, void* C, int M, int
   switch (nt) {
     case 16: return launch_gs<16>(mw, mx, a, tiles, s);
     case 32: return launch_gs<32>(mw, mx, a, tiles, s);
-    case 64: return launch_gs<64>(mw, mx, a, tiles, s);
-    default: return launch_gs<128>(mw, mx, a, tiles, s);
+    default: return launch_gs<64>(mw, mx, a, tiles, s);
   }
 }

@@ -730,12 +730,12 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: str, stre
 
 def stream_supported(M: int, N: int, K: int) -> bool:
     """Whether the weight-streaming tcgen05 kernel takes this problem."""
-    return 1 <= M <= 128 and N >= 1 and K >= 64 and K % 8 == 0
+    return 1 <= M <= 64 and N >= 1 and K >= 64 and K % 8 == 0
 
 
 def gemm_stream(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: str, stream=None, gate=None, static_weight: bool = False,
                 splits: int = 0) -> None:
-    """out = x[M, K] @ w^T for up to 128 rows, the weights streamed through the tcgen05 tensor cores as the instruction's rows. Modes as
+    """out = x[M, K] @ w^T for up to 64 rows, the weights streamed through the tcgen05 tensor cores as the instruction's rows. Modes as
     for ``gemm_skinny``. ``splits``: blocks that share K (0: the launcher's rule); ``static_weight`` as for ``gemm_f32``."""
     _cuda(x, w, out)
     M, K = x.shape

@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("mode", ["bf16", "f32", "add", "swiglu"])
-@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (16, 200, 520), (17, 131, 1024), (33, 1024, 2048), (64, 66, 576), (65, 640, 1000), (128, 257, 3072)])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (16, 200, 520), (17, 131, 1024), (33, 1024, 2048), (64, 66, 576), (63, 640, 1000), (48, 257, 3072)])
 def test_product(mode, M, N, K):
     g = torch.Generator().manual_seed(M + N + K)
     x = torch.randn(M, K, generator=g).bfloat16().to(DEV)
