@@ -1,8 +1,9 @@
 // Whole prompts of heads whose keys and values have different widths, or whose keys have a rotated part, on the tcgen05 attention, which
 // takes keys and values of one width W (64 or 128) in pages: the step's per-head keys, values and queries are laid out in rows of W with
 // zeros at their ends (scores and outputs are the same numbers), and the outputs are taken out of such rows, gated, for the output
-// product. Both kernels are bound by their bytes, 16 a thread. 2,048 tokens, 16 heads of 64 + 32 key and 64 value channels, us a layer:
-// 141 with the attention on mma.sync; 20 + 31 (tcgen05 attention) + 5 now.
+// product. Pieces of 16 bytes a thread. 2,048 tokens, 16 heads of 64 + 32 key and 64 value channels, us a layer:
+// 141 with the attention on mma.sync; 20 + 31 (tcgen05 attention) + 5 now. The layout's 40 MB would take 6 us and the outputs' 13 MB 2 us at the rate of
+// a copy: what bounds the layout is each piece's index arithmetic (divisions by run-time sizes) and the rotated pieces' single loads.
 #include "common.cuh"
 
 namespace slb {

@@ -243,11 +243,16 @@ class LatentAttention(Part):
 
     def _prompt_row_width(self, b) -> int:
         """The width of rows in which the step's whole prompts go through the tcgen05 attention with zeros at the rows' ends; 0 where
-        they do not: wider heads, odd widths, sequences that do not fill that kernel's tiles. 2,048 tokens, 16 heads of 64 + 32 key
-        and 64 value channels: 141 us a layer for the attention of heads as they are on mma.sync, 56 this way."""
+        they do not: wider heads, odd widths, sequences that do not fill that kernel's tiles, and more than 32 heads with less than 256
+        tokens in the longest sequence, where laying out the rows costs more than the attention gains. us of a five-layer prompt step, heads as they are
+        / in padded rows (keys + rotated, values): 2,048 tokens, 16 heads of 64 + 32, 64 1,314 / 826; of 40 + 16, 40 1,782 / 762; of 64 + 64, 64
+        (8 heads) 1,139 / 726; of 96 + 32, 128 1,821 / 899; of 16 + 16, 16 1,056 / 725; 128 tokens, 16 heads 481 / 408, 32 heads 512 / 448, 128 heads
+        645 / 674, with 31 sequences of 16 beside them 1,842 / 1,895; 512 tokens of 128 heads 1,237 / 988. Widths that the mma.sync kernel does
+        not take (64 + 8, 24 + 8) ran through the latents before: 2,048 tokens 11,382 / 823. Four buffers of tokens x heads x width bfloat16 are
+        taken from the step's workspace."""
         s = self.spec
         dk = s.plain_dim + s.rot_dim
-        if s.plain_dim % 8 or s.rot_dim % 8 or s.value_dim % 8 or max(dk, s.value_dim) > 128:
+        if s.plain_dim % 8 or s.rot_dim % 8 or s.value_dim % 8 or max(dk, s.value_dim) > 128 or (s.heads > 32 and b.max_count < 256):
             return 0
         width = 64 if max(dk, s.value_dim) <= 64 else 128
         return width if use_tc_attention(s.heads, s.heads, width, self.ctx.dtype, b.max_count, s.scale) else 0

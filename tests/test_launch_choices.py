@@ -141,3 +141,15 @@ def test_float32_product_on_the_tensor_cores_takes_what_was_faster():
         assert form(M, N, K) == want, (M, N, K, form(M, N, K))
     assert ops.f32_on_tensor_cores(512, 1024, 0) and not ops.f32_on_tensor_cores(4096, 1020, 0) and not ops.f32_on_tensor_cores(511, 4096, 0)
     assert not ops.f32_on_tensor_cores(512, 1030, 0) and not ops.f32_on_tensor_cores(512, 1024, 8)
+
+
+def test_prompts_of_padded_heads_where_they_were_faster():
+    """Row widths of latent attention's whole prompts: head sizes, heads and longest sequences at which both ways were timed."""
+    from types import SimpleNamespace as N
+    from sleuth_b200.parts.latent_attention import LatentAttention
+    part = object.__new__(LatentAttention)
+    part.ctx = N(dtype=torch.bfloat16)
+    for heads, dn, P, dv, longest, want in [(16, 64, 32, 64, 2048, 128), (16, 40, 16, 40, 512, 64), (32, 64, 32, 64, 128, 128), (16, 64, 32, 64, 100, 0), (128, 64, 32, 64, 128, 0),
+                                            (128, 64, 32, 64, 512, 128), (16, 128, 64, 128, 2048, 0), (16, 60, 16, 64, 2048, 0), (16, 128, 0, 64, 2048, 128)]:
+        part.spec = N(heads=heads, plain_dim=dn, rot_dim=P, value_dim=dv, scale=0.1)
+        assert part._prompt_row_width(N(max_count=longest)) == want, (heads, dn, P, dv, longest)
