@@ -1,6 +1,7 @@
 // The true 32-bit matrix product: C[M, N] (+)= A[M, K] * W[N, K]^T (+ bias[N]), float32 in, float32 out,
 // plain FMA on the CUDA cores. No tensor-core mode of any kind is involved, so nothing is rounded below float32.
-// It serves small matrices and those whose rows no 16-byte reads take; the others go to the tensor cores (gemm_f32_tc.cu).
+// It serves matrices with an inner dimension below 1,024 or less than 512 features and those whose rows no 16-byte reads take; the others go to the
+// tensor cores (gemm_f32_tc.cu, gemm_f32_rows.cu).
 //
 // The order of every sum depends on K alone. K is cut into at most eight segments (segment_length); a segment is one
 // chain acc = fmaf(a[k], w[k], acc) with k ascending, and the segments' sums are added in ascending order. Both kernels

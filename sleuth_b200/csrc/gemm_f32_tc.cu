@@ -1,30 +1,33 @@
 // The 32-bit matrix product on the tensor cores: C[M, N] (+)= A[M, K] * W[N, K]^T (+ bias[N]), float32 in, float32 out.
 //
 // A float32 value is the sum of three bfloat16 values exactly (8 + 8 + 8 bits of its 24): x = x1 + x2 + x3 with x1 = bf16(x),
-// x2 = bf16(x - x1), x3 = x - x1 - x2, |x2| <= 2^-8 |x|, |x3| <= 2^-16 |x|. A product of two bfloat16 values is exact in float32, so a
-// float32 product is w1 a1 + (w1 a2 + w2 a1) + (w1 a3 + w2 a2 + w3 a1) and parts of either sign below 2^-24 of it, typically 2^-27,
+// x2 = bf16(x - x1), x3 = x - x1 - x2, |x2| <= 2^-8 |x|, |x3| <= 2^-16 |x|. (bfloat16 ends at 2^-133, so for values below 2^-110 this holds only of the
+// value times 2^24: both operands are split after that multiplication, and the result is divided by 2^48.) A product of two bfloat16 values is exact in
+// float32, so a product is w1 a1 + (w1 a2 + w2 a1) + (w1 a3 + w2 a2 + w3 a1) and parts of either sign below 2^-24 of it, typically 2^-27,
 // which are left out: six tcgen05 products of kind f16 in place of one FMA a value (splitting into exact partial products:
 // Dekker, 1971; Ozaki et al., 2012).
 //
-// Order of the sums: K is cut into chunks of 64. A chunk's six products are summed by the tensor core, the small ones first, so that
-// of the 24 instructions only the last four add at full size (its float32 sums are truncated, half a unit each on average). A chunk's
-// sum is then taken out of tensor memory, and the chunks' sums are added in float32, rounded to nearest, in ascending order:
-//     C = ((chunk 0 + chunk 1) + chunk 2) + ...   (+ bias, then added to the old value)
-// Every form below does exactly this, whatever tile it takes, however many blocks share K and whatever M is, so that a row's bits
-// depend neither on the rows beside it nor on how a sequence was cut into steps. Which products come here depends on W alone
-// (ops.f32_on_tensor_cores). Against the FMA kernels' chains of K / 8 roundings the sums are shorter. Error (2-norm, against 64 bits),
-// FMA chains / here: K 256 2.1e-7 / 0.9e-7, 1,024 2.1e-7 / 1.1e-7, 3,072 3.6e-7 / 1.5e-7, 9,728 6.3e-7 / 2.4e-7.
-// A result that is not finite (infinite or NaN operands, whose parts are NaN; a sum beyond the range) is formed again as one FMA chain.
+// Order of the sums: K is cut into chunks of 64, a chunk into two chains of 32. A chain's six products are summed by the tensor core, the small ones first,
+// so that of its twelve instructions only the last two add at full size (its float32 sums are truncated, which on operands of one sign is a bias; in
+// chains of 64 it came to 1.33 units of 2^-24, 0.8 here). Chains are taken out of tensor memory, and all further sums are float32, rounded to nearest: a
+// chunk is chain 0 + chain 1, two chunks make a pair, and the pairs are added in ascending order:
+//     C = ((pair 0 + pair 1) + pair 2) + ...   (+ bias, then added to the old value)
+// Every form does exactly this, here and in the kernel for few rows (gemm_f32_rows.cu), whatever tile it takes and whatever M is, so that a row's
+// bits depend neither on the rows beside it nor on how a sequence was cut into steps. Which products come here depends on W alone
+// (ops.f32_on_tensor_cores). Error (2-norm, against 64 bits), FMA chains / here: normal operands, K 1,024 2.1e-7 / 0.9e-7, 3,072 3.6e-7 / 1.2e-7, 9,728
+// 6.3e-7 / 1.8e-7; of one sign 0.74e-7 / 0.68e-7, 1.2e-7 / 0.9e-7, 1.7e-7 / 1.3e-7. Below K = 1,024 operands of wide range can lose to the FMA chains.
+// A result that is not finite in this form (infinite or NaN operands, whose parts are NaN; operands from 2^104, results from 2^80 on) is formed again as the
+// FMA kernels form it.
 //
-// One block: 128 features (the instruction's rows, so that few tokens waste nothing) by NT tokens. Per chunk, for the unit u:
+// One block: 128 features (the instruction's rows) by NT tokens. Per chunk, for the unit u:
 //   * the last warp asks TMA for the raw 128 x 64 weights, a ring of R chunks ahead;
-//   * eight or sixteen warps split them into tensor memory (operand A of the instruction) and the tokens' values, which they have fetched a
-//     unit ahead into registers, into shared memory in the 128-byte swizzle (operand B), both double-buffered; while unit u is
-//     multiplied they take the sums of unit u - 1 out of tensor memory (double-buffered too), add them in registers and split unit u + 1;
+//   * eight or sixteen warps take the two chains of unit u - 1 out of tensor memory (while the tensor core rests: beside its products, which read tensor
+//     memory too, a load from there takes several times as long: 1,500 x 4,096 x 1,024 178 us against 98), then, while unit u is multiplied, split the weights of
+//     unit u + 1 into tensor memory (operand A of the instruction) and its tokens' values, fetched a unit ahead into registers, into shared memory in the
+//     128-byte swizzle (operand B), both double-buffered; a tile's sums lie in shared memory where registers are short (128 tokens);
 //   * one more warp issues the 24 instructions.
-// Blocks of a cluster may share a tile's K (few tokens: the weights' stream wants all SMs): each sends its chunks' sums as they come to
-// the block that owns the feature, through distributed shared memory, and each adds up its features, all chunks in order. The first
-// chunk of weights is split before the wait for the kernel in front.
+// The first chunk of weights is split before the wait for the kernel in front. 1,500 x 4,096 x 1,024: 309 us by FMA, 88.7 with one chain a chunk, 97.5 now: what
+// bounds it is the splitting warps' chain a chunk; the tensor core works a third of the time.
 #include "gemm_f32_split.cuh"
 #include "tcgen05.cuh"
 

@@ -1,8 +1,9 @@
 """The matrix product y = h @ W^T that every projection uses, chosen by dtype and row count.
 
-* float32 run: small matrices on the package's own FMA kernels (``csrc/gemm_f32.cu``), larger ones on its tensor-core kernel
-  (``csrc/gemm_f32_tc.cu``), which forms each float32 product from bfloat16 parts that add up to the operands exactly; no
-  rounding below float32 either way, and every output element sums over k in one fixed order whatever the number of rows.
+* float32 run: matrices with an inner dimension below 1,024 on the package's own FMA kernels (``csrc/gemm_f32.cu``), others on its
+  tensor-core kernels (``csrc/gemm_f32_tc.cu`` and ``csrc/gemm_f32_rows.cu``), which form each product from bfloat16 parts that add up
+  to the operands (six of the nine partial products; what is left out is below 2^-24 of it) with an error that is no larger than the
+  FMA chains'; every output element sums over k in one fixed order whatever the number of rows.
 * bfloat16 run, up to 32 rows (decode steps): the package's weight-streaming tensor-core kernel
   (``csrc/gemm_skinny.cu``), with the residual add or the float32 store in its epilogue.
 * bfloat16 run, 9 to 64 rows and large matrices: the package's tcgen05 kernel with the weights as the instruction's rows
