@@ -35,6 +35,7 @@ struct FrShape {
   static constexpr int kSmem = WARPS * kStages * kStage + 2 * kSums * 4;
 };
 
+// (Not volatile: the two chains' instructions may be interleaved.)
 __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&w)[4], const uint32_t (&x)[2]) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
