@@ -42,7 +42,7 @@ class StepEntry:
 
 
 class Stepper:
-    STATUS_EVERY = 8
+    STATUS_EVERY = 16
 
     def __init__(self, model, cache, device, max_len: int | None = None, max_step_tokens: int = 8192,
                  use_graphs: bool = True, max_graph_batch: int = 256):
@@ -146,8 +146,8 @@ class Stepper:
     # ------------------------------------------------------------ the kernels' status word ----
     def _look_at_status(self, single_tokens: bool = False) -> None:
         """After every step: with ``check_kernels`` read the kernels' status word now, else start a copy of it. Single-token steps,
-        whose products wait on barriers too (float32 runs, 9 to 64 sequences of large models), take turns: a copy costs some 10 us of
-        the host's time, as much as a hundredth of a short step, and one in ``STATUS_EVERY`` tells of all that came before."""
+        whose products wait on barriers too (float32 runs, 9 to 64 sequences of large models), take turns: a copy costs some 20 us of
+        the host's time, several hundredths of a short step, and one in ``STATUS_EVERY`` tells of all that came before."""
         if self.check_kernels:
             ops.gemm_tc_check(self.device)
             return
