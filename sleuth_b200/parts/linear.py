@@ -62,7 +62,7 @@ def use_skinny(M: int, N: int, K: int, norm: bool = False) -> bool:
 # by the number of rows, so the line does too. us in a row of launches, other kernel / this one:
 #   17 to 32 rows (the weight-streaming kernel goes over the rows twice): from 8 M weights on. 24 rows x 2,048 x 4,096 7.9 / 6.7, 4,096 x 2,048 6.3 / 6.3.
 #   9 to 16 rows: the weight-streaming kernel keeps the smaller matrices. 4,096 x 2,560 5.9 / 6.3, 4,096 x 4,096 7.7 / 8.0, 2,048 x 8,192 8.6 / 9.1, but
-#     6,144 x 2,560 11.0 / 7.4, 16,384 x 1,024 10.2 / 8.1, 2,560 x 9,728 15.3 / 11.2; gated (rows of gate and up) 6,144 x 4,096 10.6 / 11.3,
+#     6,144 x 2,560 11.0 / 7.4, 16,384 x 1,024 10.2 / 8.1, 2,560 x 9,728 15.3 / 11.2, and where its blocks leave the SMs idle 2,560 x 4,096 7.0 / 6.3; gated (rows of gate and up) 6,144 x 4,096 10.6 / 11.3,
 #     8,192 x 2,048 7.7 / 8.0, 12,288 x 2,560 14.7 / 12.5, 19,456 x 2,560 22.0 / 19.1. Not output matrices (151,936 x 1,024 65.5 / 69.5).
 #   33 to 64 rows: cuBLAS is ahead where there are many features (64 rows x 6,144 x 2,560 8.1 / 9.6, 16,384 x 1,024 8.1 / 10.6, 19,456 x 2,560 18.7 / 21.7),
 #     behind where the sums are long (4,096 x 4,096 10.1 / 10.0, 2,560 x 9,728 14.9 / 13.3, 2,048 x 8,192 13.1 / 10.8). Gated it has the activation kernel
@@ -74,7 +74,11 @@ def use_stream(M: int, N: int, K: int, gated: bool = False) -> bool:
     if not USE_TC or not 8 < M <= 64 or weights < 8 << 20 or not ops.stream_supported(M, N, K):
         return False
     if M <= 16:
-        return (28 << 20 if gated else 10_000_000 if features > 4096 else 20 << 20) <= weights <= 128 << 20
+        if gated or weights >= 20 << 20:
+            return (28 if gated else 20) << 20 <= weights <= 128 << 20
+        # (the weight-streaming kernel's last round over the SMs, 16 features a block, is less than three quarters full on the whole)
+        blocks = -(-features // 16)
+        return features > 4096 and weights >= 10_000_000 or K >= 3584 and -(-blocks // 148) * 148 > 1.3 * blocks
     if M <= 32:
         return True
     if gated:

@@ -117,7 +117,7 @@ def test_large_matrices_of_some_rows_are_streamed_through_the_tensor_cores():
     """Where products and whole runs were timed with and without (4B, 8B and 0.6B sizes, and such between them)."""
     for M, N, K, gated, want in [(16, 2560, 9728, False, True), (16, 9728, 2560, True, True), (24, 6144, 2560, False, True), (64, 12288, 4096, True, True),
                                  (8, 9728, 2560, True, False), (65, 12288, 4096, True, False), (24, 1024, 3072, False, False), (24, 3072, 1024, True, False),
-                                 (16, 151936, 2560, False, False), (24, 151936, 2560, False, True), (16, 4096, 2560, False, False), (16, 4096, 4096, False, False),
+                                 (16, 151936, 2560, False, False), (24, 151936, 2560, False, True), (16, 4096, 2560, False, False), (16, 4096, 4096, False, False), (16, 2560, 4096, False, True), (16, 2048, 8192, False, False),
                               (16, 6144, 2560, False, True), (16, 3072, 4096, True, False), (16, 6144, 2560, True, True), (32, 4096, 2048, False, True), (33, 6144, 2560, False, False),
                               (64, 8192, 2048, False, False), (64, 4096, 12288, False, True), (64, 9728, 2560, True, False), (48, 9728, 2560, True, True), (64, 4608, 1024, True, True)]:
         assert linear.use_stream(M, N, K, gated) == want, (M, N, K)
